@@ -1,6 +1,7 @@
-// Flash attention forward on the 5th-generation tensor cores (tcgen05 + TMEM), fed by TMA.
+// Flash attention forward on the 5th-generation tensor cores (tcgen05 + TMEM), fed by TMA: a kernel of one query tile
+// per CTA (head size 256) and one of two tiles that take turns (64 and 128, further down).
 //
-// One CTA owns 128 query rows of one head.  Warp 8 is the copy/MMA warp: it streams K and V blocks
+// One tile: a CTA owns 128 query rows of one head.  Warp 8 is the copy/MMA warp: it streams K and V blocks
 // through a 2-stage shared-memory ring and issues  S = Q K^T  and  O += P V  as tcgen05.mma with the
 // accumulators in tensor memory (S double-buffered, O resident for the whole KV sweep).  Warps 0-7 are
 // the softmax warps, two per scheduler so that one hides the other's latencies: threads r and r + 128 share
@@ -382,6 +383,325 @@ __global__ void __launch_bounds__(THREADS, 1) flash_fwd_kernel(const __grid_cons
   }
 }
 
+// ------------------------------------------------------------------------------------------------ two query tiles
+// Head sizes 64 and 128.  One CTA owns 256 query rows of a head as two tiles of 128; while the softmax warps of one
+// tile turn its scores into probabilities, the tensor core runs the products of the other, so neither waits for the
+// other's chain.  Tensor memory: S of tile 0 and 1 in columns 0 and 128 (P, as bf16 pairs, overwrites the first half of
+// its own S and feeds the second product from there), O of the two tiles from column 256.
+//
+// Warps 0-3 / 4-7: softmax of tile 0 / 1, one thread per query row (no exchange between threads); warp 8 streams K
+// and V through two stages each; warp 9 issues, per key block and tile, O += P V and then S of the next key block: the
+// tensor core runs one thread's products in order, so S may overwrite the P that the product before it reads.
+// P is never staged in shared memory, which leaves its bandwidth to the operands (a 128 x 128 x 128 product with both
+// operands in shared memory reads 64 KB in the 512 cycles it computes: exactly the limit).
+//
+// Bound by the exponentials: a 128 x 128 block takes 1024 cycles of the special-function units beside 1024 (head size
+// 128) or 512 (64) of the tensor pipe.  Measured at one sequence of 8192, 16 heads of 128, causal: 1014 us with one
+// tile per CTA and P in shared memory (the kernel above, which head size 256 keeps: its O alone takes half of the tensor
+// memory), 277 us with this one (990 TFLOP/s); heads of 64: 238 us.
+constexpr int TT = 128;                               // rows of a tile
+constexpr int THREADS2 = 320;
+
+template <int HD>
+struct Cfg2 {
+  static constexpr int KC = HD / 64;
+  static constexpr int TILE = TT * HD * 2;            // Q tile, K block, V block
+  static constexpr int SMEM = 6 * TILE + 1024 + 256;
+  static constexpr int O_COL0 = 256;
+};
+
+// floor(a / b) for b > 0
+__device__ __forceinline__ int floor_div(int a, int b) {
+  const int q = a / b;
+  return q - ((a % b) < 0 ? 1 : 0);
+}
+
+template <int HD, bool DROP>
+__global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_constant__ Params p) {
+  using C = Cfg2<HD>;
+  constexpr int KC = C::KC;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t sQ = base, sK = sQ + 2 * C::TILE, sV = sK + 2 * C::TILE, bars = sV + 2 * C::TILE;
+  auto bar = [&](int i) { return bars + 8u * i; };
+  constexpr int Q_FULL = 0, K_FULL = 1, V_FULL = 3, K_EMPTY = 5, V_EMPTY = 7, S_FULL = 9, P_FULL = 11, O_DONE = 13, N_BARS = 15;
+  uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 6 * C::TILE + 8 * N_BARS);
+  volatile int* abort_smem = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the query blocks with the most visible keys start first (causal: the last ones), so the tail of the grid is short
+  const int qb = gridDim.y - 1 - blockIdx.y;
+  const int h = blockIdx.x % p.H, b = blockIdx.x / p.H;
+  const int hk = h / (p.H / p.Hkv);
+  const int q0 = qb * 2 * TT;
+
+  // key blocks visible to each tile (logical positions): [lo[t], hi[t])
+  int lo[2], hi[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int r0 = q0 + t * TT;
+    lo[t] = 0;
+    hi[t] = r0 < p.Tq ? (p.Tk + TT - 1) / TT : 0;
+    const int pos_lo = p.q_off + r0 * p.q_stride;
+    const int pos_hi = p.q_off + (min(r0 + TT, p.Tq) - 1) * p.q_stride;
+    if (p.causal) {
+      const int kmax = floor_div(pos_hi - p.k_off, p.k_stride);
+      hi[t] = kmax < 0 ? 0 : min(hi[t], kmax / TT + 1);
+    }
+    if (p.window > 0) {
+      const int kmin = floor_div(pos_lo - p.window - p.k_off, p.k_stride) + 1;
+      lo[t] = max(0, kmin) / TT;
+    }
+    if (lo[t] >= hi[t]) lo[t] = hi[t] = 0;
+  }
+  const bool any0 = hi[0] > lo[0], any1 = hi[1] > lo[1];
+  const int j_lo = any0 && any1 ? min(lo[0], lo[1]) : any0 ? lo[0] : lo[1];
+  const int j_hi = max(hi[0], hi[1]);
+
+  if (threadIdx.x == 0) {
+    mbar_init(bar(Q_FULL), 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(bar(K_FULL + s), 1);
+      mbar_init(bar(V_FULL + s), 1);
+      mbar_init(bar(K_EMPTY + s), 1);
+      mbar_init(bar(V_EMPTY + s), 1);
+      mbar_init(bar(S_FULL + s), 1);
+      mbar_init(bar(P_FULL + s), TT);
+      mbar_init(bar(O_DONE + s), 1);
+    }
+    *abort_smem = 0;
+    fence_mbar_init();
+  }
+  if (warp == 9) {
+    tmem_alloc<1>(smem_u32(tmem_slot), 512);
+    tmem_relinquish<1>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+  if (warp == 8) {
+    if (lane == 0 && j_hi > j_lo) {
+      // ------------------------------------------------------------------ copies
+      const int q_row = b * p.Tq + q0;
+      const int tiles = any1 ? 2 : 1;                  // the second tile may lie past the last query
+      mbar_expect_tx(bar(Q_FULL), tiles * C::TILE);
+      for (int t = 0; t < tiles; ++t)
+        for (int kc = 0; kc < KC; ++kc)
+          tma_load_2d(sQ + t * C::TILE + kc * (TT * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, q_row + t * TT);
+      bool ok = true;
+      for (int j = j_lo, n = 0; ok && j < j_hi; ++j, ++n) {
+        const int s = n & 1;
+        const int k_row = b * p.Tk + j * TT;
+        if (n >= 2) ok = mbar_wait(bar(K_EMPTY + s), ((n >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
+        if (!ok) break;
+        mbar_expect_tx(bar(K_FULL + s), C::TILE);
+        for (int kc = 0; kc < KC; ++kc)
+          tma_load_2d(sK + s * C::TILE + kc * (TT * 128), &p.tmK, bar(K_FULL + s), p.k_col0 + hk * HD + kc * 64, k_row);
+        if (n >= 2) ok = mbar_wait(bar(V_EMPTY + s), ((n >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
+        if (!ok) break;
+        mbar_expect_tx(bar(V_FULL + s), C::TILE);
+        for (int kc = 0; kc < KC; ++kc)
+          tma_load_2d(sV + s * C::TILE + kc * (TT * 128), &p.tmV, bar(V_FULL + s), p.v_col0 + hk * HD + kc * 64, k_row);
+      }
+    }
+  } else if (warp == 9) {
+    if (lane == 0 && j_hi > j_lo) {
+      // ------------------------------------------------------------------ products
+      constexpr uint32_t idesc_s = umma_idesc_bf16(TT, TT, 0, 0);
+      constexpr uint32_t idesc_o = umma_idesc_bf16(TT, HD, 0, 1);            // B = V is MN-major
+      auto issue_s = [&](int t, int s) {
+        const uint32_t qt = sQ + t * C::TILE, kb = sK + s * C::TILE;
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_f16<1>(tmem + t * 128, umma_smem_desc(qt + kc * (TT * 128) + k * 32, 16, 1024),
+                        umma_smem_desc(kb + kc * (TT * 128) + k * 32, 16, 1024), idesc_s, (kc | k) ? 1u : 0u);
+        umma_commit(bar(S_FULL + t));
+      };
+      bool ok = mbar_wait(bar(Q_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      if (ok) ok = mbar_wait(bar(K_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      if (ok) {
+        tc_fence_after();
+        for (int t = 0; t < 2; ++t)
+          if (j_lo >= lo[t] && j_lo < hi[t]) issue_s(t, 0);
+        umma_commit(bar(K_EMPTY));
+      }
+      int done[2] = {0, 0};                            // key blocks of each tile whose P V has been issued
+      for (int j = j_lo, n = 0; ok && j < j_hi; ++j, ++n) {
+        const int s = n & 1, sn = s ^ 1;
+        ok = mbar_wait(bar(V_FULL + s), (n >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+        if (!ok) break;
+        const bool more = j + 1 < j_hi;
+        bool k_ready = false;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (j >= lo[t] && j < hi[t]) {
+            ok = mbar_wait(bar(P_FULL + t), done[t] & 1, abort_smem, p.status, SITE_TMEM_FULL);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t v_base = sV + s * C::TILE;
+#pragma unroll
+            for (int k = 0; k < TT / 16; ++k)          // B = V: MN-major, groups of 64 head dims
+              umma_f16_ts(tmem + C::O_COL0 + t * 128, tmem + t * 128 + k * 8, umma_smem_desc(v_base + k * 2048, TT * 128, 1024),
+                          idesc_o, (done[t] | k) ? 1u : 0u);
+            umma_commit(bar(O_DONE + t));
+            ++done[t];
+          }
+          if (t == 1) umma_commit(bar(V_EMPTY + s));
+          if (more && j + 1 >= lo[t] && j + 1 < hi[t]) {
+            if (!k_ready) {
+              ok = mbar_wait(bar(K_FULL + sn), ((n + 1) >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+              if (!ok) break;
+              tc_fence_after();
+              k_ready = true;
+            }
+            issue_s(t, sn);
+          }
+        }
+        if (ok && more) umma_commit(bar(K_EMPTY + sn));
+      }
+    }
+  } else {
+    // -------------------------------------------------------------------- softmax warps: thread = query row
+    const int t = warp >> 2;
+    const int row = threadIdx.x & 127;                 // == TMEM lane
+    const int qi = q0 + t * TT + row;
+    const int qpos = p.q_off + qi * p.q_stride;
+    const uint32_t s_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + t * 128;
+    const uint32_t o_addr = s_addr + C::O_COL0;
+    const int n_blocks = hi[t] - lo[t], j0 = lo[t];
+    // keys this row sees: indices [k_first, k_end)
+    int k_first = 0, k_end = p.Tk;
+    if (p.causal) k_end = min(k_end, floor_div(qpos - p.k_off, p.k_stride) + 1);
+    if (p.window > 0) k_first = max(0, floor_div(qpos - p.window - p.k_off, p.k_stride) + 1);
+    // a block that every row of the tile sees whole needs no mask
+    const int r_lo = q0 + t * TT, r_hi = r_lo + TT - 1;
+    int full_lo = 0, full_hi = p.Tk;
+    if (p.causal) full_hi = min(full_hi, floor_div(p.q_off + r_lo * p.q_stride - p.k_off, p.k_stride) + 1);
+    if (p.window > 0) full_lo = max(0, floor_div(p.q_off + r_hi * p.q_stride - p.window - p.k_off, p.k_stride) + 1);
+    const float thr = 8.f / p.scale_log2;              // the reference point moves when the max grew by > 2^8
+    float m_ref = -CUDART_INF_F, l = 0.f;
+    DropoutRow dr;
+    bool ok = true;
+    for (int it = 0; it < n_blocks; ++it) {
+      ok = mbar_wait(bar(S_FULL + t), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t r[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_addr + c * 32, r[c]);
+      tmem_ld_wait();
+      const int kbase = (j0 + it) * TT;
+      if (kbase < full_lo || kbase + TT > full_hi) {
+        const int first = k_first - kbase, end = k_end - kbase;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i < first || c * 32 + i >= end) r[c][i] = 0xff800000u;     // -inf: exp2 gives an exact zero
+      }
+      float mxs[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mxs[c] = fmaxf(mxs[c], __uint_as_float(r[c][i]));
+      const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
+      float alpha = 1.f;
+      if (mx > m_ref + thr) {                          // also the first block with a visible key (m_ref = -inf)
+        alpha = ex2_approx((m_ref - mx) * p.scale_log2);          // ex2(-inf) = 0
+        m_ref = mx;
+      }
+      // tcgen05.ld / .st are warp-collective: the decision must be the same for all 32 rows of a warp.  Never for the
+      // first block: its product overwrites O.
+      if (it > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+        ok = mbar_wait(bar(O_DONE + t), (it - 1) & 1, abort_smem, p.status, SITE_TMEM_EMPTY);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < HD / 16; ++c) {
+          uint32_t o[16];
+          tmem_ld_32x16(o_addr + c * 16, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x16(o_addr + c * 16, o);
+        }
+      }
+      const float neg_ms = (m_ref == -CUDART_INF_F) ? 0.f : -m_ref * p.scale_log2;
+      if (DROP) dr.begin((uint32_t)(b * p.heads_total + p.head_off + h), (uint32_t)qpos);
+      float sums[2] = {0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float p0 = ex2_approx(fmaf(__uint_as_float(r[c][i]), p.scale_log2, neg_ms));
+          float p1 = ex2_approx(fmaf(__uint_as_float(r[c][i + 1]), p.scale_log2, neg_ms));
+          sums[0] += p0;                               // the row sum is that of the undropped probabilities
+          sums[1] += p1;
+          if (DROP) {
+            const uint32_t kpos = (uint32_t)(p.k_off + (kbase + c * 32 + i) * p.k_stride);
+            p0 = dr.keep(p.drop, kpos) ? p0 * p.drop.inv_keep : 0.f;
+            p1 = dr.keep(p.drop, kpos + (uint32_t)p.k_stride) ? p1 * p.drop.inv_keep : 0.f;
+          }
+          __nv_bfloat162 hb = __floats2bfloat162_rn(p0, p1);
+          w[i / 2] = *reinterpret_cast<uint32_t*>(&hb);
+        }
+        tmem_st_32x16(s_addr + c * 16, w);             // every score of the row is in registers by now
+      }
+      l = l * alpha + sums[0] + sums[1];
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(bar(P_FULL + t));
+    }
+    // ---- epilogue: O / l -> bf16 rows, log-sum-exp
+    if (ok && n_blocks > 0) {
+      ok = mbar_wait(bar(O_DONE + t), (n_blocks - 1) & 1, abort_smem, p.status, SITE_TMEM_FULL);
+      tc_fence_after();
+    }
+    ok = __all_sync(0xffffffffu, ok);                  // the TMEM loads below are warp-collective: every lane takes part,
+    if (ok) {                                          // only the global stores are predicated on the row being real
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      __nv_bfloat16* dst = p.out + ((long long)b * p.Tq + qi) * p.ldo + h * HD;
+#pragma unroll 1
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t o[32];
+        if (n_blocks > 0) {
+          tmem_ld_32x32(o_addr + c * 32, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 q4;
+          __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&q4);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            hb[i] = __floats2bfloat162_rn(__uint_as_float(o[8 * j + 2 * i]) * inv, __uint_as_float(o[8 * j + 2 * i + 1]) * inv);
+          if (qi < p.Tq) *reinterpret_cast<uint4*>(dst + c * 32 + j * 8) = q4;
+        }
+      }
+      if (p.lse && qi < p.Tq)
+        p.lse[((long long)b * p.H + h) * p.Tq + qi] =
+            l > 0.f ? (m_ref * p.scale_log2 + log2f(l)) * 0.6931471805599453f : -CUDART_INF_F;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc<1>(tmem, 512);
+  }
+}
+
 static bool map2d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_rows) {
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
@@ -412,13 +732,24 @@ static int launch(const MeshFlashArgs* a, cudaStream_t stream) {
   p.drop.k1 = (uint32_t)(a->seed >> 32);
   p.drop.site = a->site;
   p.head_off = a->head_off; p.heads_total = a->heads_total > 0 ? a->heads_total : a->H;
-  static bool configured = false;
-  if (!configured) {
-    MESH_CUDA_OK(cudaFuncSetAttribute(flash_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    configured = true;
+  if constexpr (HD <= 128) {
+    auto kern = p.drop.p > 0.f ? flash_fwd2_kernel<HD, true> : flash_fwd2_kernel<HD, false>;
+    static bool configured[2] = {false, false};
+    if (!configured[p.drop.p > 0.f]) {
+      MESH_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg2<HD>::SMEM));
+      configured[p.drop.p > 0.f] = true;
+    }
+    dim3 grid(a->H * a->B, (a->Tq + 2 * TT - 1) / (2 * TT));
+    kern<<<grid, THREADS2, Cfg2<HD>::SMEM, stream>>>(p);
+  } else {
+    static bool configured = false;
+    if (!configured) {
+      MESH_CUDA_OK(cudaFuncSetAttribute(flash_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+      configured = true;
+    }
+    dim3 grid((a->Tq + BQ - 1) / BQ, a->H, a->B);
+    flash_fwd_kernel<HD><<<grid, THREADS, C::SMEM, stream>>>(p);
   }
-  dim3 grid((a->Tq + BQ - 1) / BQ, a->H, a->B);
-  flash_fwd_kernel<HD><<<grid, THREADS, C::SMEM, stream>>>(p);
   MESH_CUDA_OK(cudaGetLastError());
   return 0;
 }
