@@ -1,4 +1,4 @@
-// Flash attention backward on tcgen05 / TMEM.
+// Flash attention backward on tcgen05 / TMEM: a serial kernel (dropout) and a pipelined one (everything else).
 //
 // One CTA owns one block of 128 keys of one KV head and walks the query blocks (of every query head of
 // the group) that can see it.  Per query block, five tensor-core products run from the same shared-memory
@@ -31,6 +31,7 @@ constexpr int THREADS = 288;          // + 1 copy/MMA warp
 
 struct Params {
   CUtensorMap tmQ, tmK, tmV, tmdO;           // boxes {64, 128}
+  CUtensorMap tmdQ;                          // fp32 [B][Tq][H*hd], box {32, 32, 1}
   const float* lse; const float* delta;      // [B, H, Tq]
   float* dq;                                 // fp32 [B*Tq, H*hd], zeroed by the caller
   __nv_bfloat16* dk; __nv_bfloat16* dv;      // [B*Tk, Hkv*hd] (bf16, written) ...
@@ -64,6 +65,55 @@ __device__ __forceinline__ void store_row32(uint32_t tile, int row, int c, const
     const uint32_t chunk = ((c & 1) * 4 + j) ^ (row & 7);
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + (chunk << 4)), "r"(w[4 * j]), "r"(w[4 * j + 1]),
                  "r"(w[4 * j + 2]), "r"(w[4 * j + 3]) : "memory");
+  }
+}
+
+// dV and dK of one key row (thread = row, half of the head dimension) from tensor memory: bf16 outputs, or added to the
+// fp32 accumulators.  The TMEM loads are warp-collective: only the stores are predicated on the row being real.
+template <int HD>
+__device__ __forceinline__ void write_dkv(const Params& p, uint32_t dv_addr, uint32_t dk_addr, int b, int hk, int kj, int half) {
+  const long long off = ((long long)b * p.Tk + kj) * p.ld_dkv + hk * HD + half * (HD / 2);
+#pragma unroll 1
+  for (int which = 0; which < 2; ++which) {
+    const uint32_t addr = (which ? dk_addr : dv_addr) + half * (HD / 2);
+#pragma unroll 1
+    for (int c = 0; c < HD / 64; ++c) {
+      uint32_t r[32];
+      tmem_ld32(addr + c * 32, r);
+      if (kj < p.Tk && p.dk_acc) {
+        float* dst = (which ? p.dk_acc : p.dv_acc) + off + c * 32;
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          float4 cur = *reinterpret_cast<float4*>(dst + e);
+          cur.x += __uint_as_float(r[e]); cur.y += __uint_as_float(r[e + 1]);
+          cur.z += __uint_as_float(r[e + 2]); cur.w += __uint_as_float(r[e + 3]);
+          *reinterpret_cast<float4*>(dst + e) = cur;
+        }
+      } else if (kj < p.Tk) {
+        __nv_bfloat16* dst = (which ? p.dk : p.dv) + off + c * 32;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 o;
+          __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            hb[e] = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1]));
+          *reinterpret_cast<uint4*>(dst + j * 8) = o;
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// nothing sees this key block: its gradients are zero
+template <int HD>
+__device__ __forceinline__ void zero_dkv(const Params& p, int b, int hk, int kj) {
+  if (kj >= p.Tk) return;
+  const long long off = ((long long)b * p.Tk + kj) * p.ld_dkv + hk * HD;
+  for (int e = 0; e < HD; e += 8) {
+    *reinterpret_cast<uint4*>(p.dk + off + e) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(p.dv + off + e) = make_uint4(0, 0, 0, 0);
   }
 }
 
@@ -280,51 +330,8 @@ __global__ void __launch_bounds__(THREADS, 1) flash_bwd_kernel(const __grid_cons
     }
     // ---- dK, dV of this key block (thread = key row, half of the head dimension)
     ok = __all_sync(0xffffffffu, ok);
-    if (ok && n_iter > 0) {
-      const int kj = k0 + row;
-      const long long off = ((long long)b * p.Tk + kj) * p.ld_dkv + hk * HD + half * (HD / 2);
-#pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-        const int col0 = (which ? C_DK : C_DV) + half * (HD / 2);
-#pragma unroll 1
-        for (int c = 0; c < HD / 64; ++c) {
-          uint32_t r[32];
-          tmem_ld32(lane_addr + col0 + c * 32, r);
-          if (kj >= p.Tk) continue;
-          if (p.dk_acc) {
-            float* dst = (which ? p.dk_acc : p.dv_acc) + off + c * 32;
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              float4 cur = *reinterpret_cast<float4*>(dst + e);
-              cur.x += __uint_as_float(r[e]); cur.y += __uint_as_float(r[e + 1]);
-              cur.z += __uint_as_float(r[e + 2]); cur.w += __uint_as_float(r[e + 3]);
-              *reinterpret_cast<float4*>(dst + e) = cur;
-            }
-          } else {
-            __nv_bfloat16* dst = (which ? p.dk : p.dv) + off + c * 32;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 o;
-              __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                hb[e] = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1]));
-              *reinterpret_cast<uint4*>(dst + j * 8) = o;
-            }
-          }
-        }
-      }
-    } else if (n_iter == 0 && !p.dk_acc && half == 0) {
-      // nothing sees this key block: its gradients are zero
-      const int kj = k0 + row;
-      if (kj < p.Tk) {
-        const long long off = ((long long)b * p.Tk + kj) * p.ld_dkv + hk * HD;
-        for (int e = 0; e < HD; e += 8) {
-          *reinterpret_cast<uint4*>(p.dk + off + e) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(p.dv + off + e) = make_uint4(0, 0, 0, 0);
-        }
-      }
-    }
+    if (ok && n_iter > 0) write_dkv<HD>(p, lane_addr + C_DV, lane_addr + C_DK, b, hk, k0 + row, half);
+    else if (n_iter == 0 && !p.dk_acc && half == 0) zero_dkv<HD>(p, b, hk, k0 + row);
   }
   tc_fence_before();
   __syncthreads();
@@ -334,12 +341,424 @@ __global__ void __launch_bounds__(THREADS, 1) flash_bwd_kernel(const __grid_cons
   }
 }
 
+// ------------------------------------------------------------------------------------------------ pipelined backward
+// Without dropout.  As above one CTA owns 128 keys of a KV head and walks the query blocks that see them, but the scores
+// are computed transposed (rows = keys) and the five products of consecutive query blocks overlap with the threads:
+//
+//     tensor core   ... dV += P^T dO | S' = K Q'^T | dQ = dS K | dK += dS^T Q | dP' = V dO'^T ...     (' = next block)
+//     warps 0-7     P from S, dS from P and dP: a thread holds one key row and half of the query columns
+//     warps 8-11    add dQ of the block to the float accumulator while dK runs: 32 x 32 pieces through shared memory
+//                   and one reducing bulk copy each.  (Reductions straight from registers, red.global.add.v2 with four
+//                   lanes on a 32-byte sector, held the whole pipeline up: 942 us instead of 706 us at one sequence of
+//                   8192, 16 heads of 128, causal.)
+//     warp 12       copies: K, V once; Q, L and Delta of the query blocks through two stages, dO through one (it is
+//                   free from dV of a block on and needed again three products later; the other 32 KB stage dQ)
+//     warp 13       issues the products in the order above
+//
+// P^T goes back to tensor memory as bf16 over the columns of S that its thread has read, and feeds dV from there; only
+// dS passes through shared memory, where dK reads it along the keys and dQ across them.  dQ takes the columns of dP,
+// which every thread has read by the time dS is complete.
+//
+// Bound by the chain dP -> dS -> dQ -> drain -> dP' beside a tensor pipe that needs 2560 cycles per pair of blocks at
+// head size 128.  Measured at one sequence of 8192, 16 heads of 128, causal: 1967 us with the serial kernel above,
+// 706 us with this one (973 TFLOP/s); heads of 64: 494 us.  Dropout stays with the kernel above: there a thread holds
+// a query row and pays one generator call for four keys, here it would pay one for every score.
+constexpr int THREADS2 = 448;
+
+struct Bars2 {
+  static constexpr int KV_FULL = 0, Q_FULL = 1, Q_EMPTY = 3, DO_FULL = 5, DO_EMPTY = 6, S_FULL = 7, P_FULL = 8, DP_FULL = 9,
+                       DS_FULL = 10, DQ_FULL = 11, DQ_READ = 12, ACC_DONE = 13, N = 14;
+};
+
+template <int HD>
+struct Cfg2 {
+  static constexpr int KC = HD / 64;
+  static constexpr int TILE = 128 * HD * 2;            // K, V, Q, dO tiles
+  static constexpr int PT = 128 * 128 * 2;             // dS tile
+  static constexpr int ROWS = 2 * 2 * 128 * 4;         // L and Delta of two query blocks
+  static constexpr int RED = 4 * 2 * 4096;             // two 32 x 32 fp32 pieces of dQ per warp
+  static constexpr int SMEM = 5 * TILE + PT + RED + ROWS + 8 * Bars2::N + 16;    // no room to align by hand at 128
+};
+
+template <int HD>
+__global__ void __launch_bounds__(THREADS2, 1) flash_bwd2_kernel(const __grid_constant__ Params p) {
+  using C = Cfg2<HD>;
+  using B_ = Bars2;
+  constexpr int KC = C::KC, TILE = C::TILE;
+  extern __shared__ __align__(1024) uint8_t smem_al[];
+  const uint32_t base = smem_u32(smem_al);
+  if (base & 1023u) {                                  // the swizzled tiles need it; nothing is placed before them
+    if (threadIdx.x == 0) status_record(p.status, MESH_ALIGN, SITE_NONE, 1024, base);
+    return;
+  }
+  const uint32_t sK = base, sV = sK + TILE, sQ = sV + TILE, sdO = sQ + 2 * TILE, sdS = sdO + TILE, sRed = sdS + C::PT;
+  uint8_t* gen = smem_al;
+  float* rows_s = reinterpret_cast<float*>(gen + 5 * TILE + C::PT + C::RED);   // [stage][-L * log2(e), -Delta * scale][128]
+  const uint32_t bars = sRed + C::RED + C::ROWS;
+  auto bar = [&](int i) { return bars + 8u * i; };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 5 * TILE + C::PT + C::RED + C::ROWS + 8 * B_::N);
+  volatile int* abort_smem = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  // tensor memory columns: S (P^T), dP (dQ), dV, dK
+  constexpr int C_S = 0, C_DP = 128, C_DQ = 128, C_DV = 256, C_DK = 256 + HD;
+  static_assert(C_DK + HD <= 512, "head_dim up to 128 fits tensor memory");
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // key blocks in the slow grid dimension: the first ones, which the causal mask hides from nobody, start first
+  const int jb = blockIdx.y, hk = blockIdx.x % p.Hkv, b = blockIdx.x / p.Hkv;
+  const int group = p.H / p.Hkv;
+  const int k0 = jb * BKV;
+
+  // query blocks that can see this key block
+  const int kpos_lo = p.k_off + k0 * p.k_stride;
+  const int kpos_hi = p.k_off + (min(k0 + BKV, p.Tk) - 1) * p.k_stride;
+  int i_lo = 0, i_hi = (p.Tq + BQ - 1) / BQ;
+  if (p.causal) {
+    const int qmin = kpos_lo - p.q_off <= 0 ? 0 : (kpos_lo - p.q_off + p.q_stride - 1) / p.q_stride;
+    i_lo = max(i_lo, qmin / BQ);
+  }
+  if (p.window > 0) {
+    const int qmax_pos = kpos_hi + p.window - 1;
+    const int qmax = qmax_pos - p.q_off < 0 ? -1 : (qmax_pos - p.q_off) / p.q_stride;
+    i_hi = min(i_hi, qmax / BQ + 1);
+    if (qmax < 0) i_hi = 0;
+  }
+  const int n_q = max(0, i_hi - i_lo);
+  const int n_iter = n_q * group;
+
+  if (threadIdx.x == 0) {
+    mbar_init(bar(B_::KV_FULL), 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(bar(B_::Q_FULL + s), 1);
+      mbar_init(bar(B_::Q_EMPTY + s), 1);
+    }
+    mbar_init(bar(B_::DO_FULL), 33);                   // the copy and 32 lanes that stored L and Delta
+    mbar_init(bar(B_::DO_EMPTY), 1);
+    mbar_init(bar(B_::S_FULL), 1);
+    mbar_init(bar(B_::P_FULL), SM_THREADS);
+    mbar_init(bar(B_::DP_FULL), 1);
+    mbar_init(bar(B_::DS_FULL), SM_THREADS);
+    mbar_init(bar(B_::DQ_FULL), 1);
+    mbar_init(bar(B_::DQ_READ), 128);
+    mbar_init(bar(B_::ACC_DONE), 1);
+    *abort_smem = 0;
+    fence_mbar_init();
+  }
+  if (warp == 13) {
+    tmem_alloc<1>(smem_u32(tmem_slot), 512);
+    tmem_relinquish<1>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+  if (warp == 12) {
+    // -------------------------------------------------------------------- copies
+    if (n_iter > 0) {
+      if (lane == 0) {
+        const int k_row = b * p.Tk + k0;
+        mbar_expect_tx(bar(B_::KV_FULL), 2 * TILE);
+        for (int kc = 0; kc < KC; ++kc) {
+          tma_load_2d(sK + kc * (128 * 128), &p.tmK, bar(B_::KV_FULL), p.k_col0 + hk * HD + kc * 64, k_row);
+          tma_load_2d(sV + kc * (128 * 128), &p.tmV, bar(B_::KV_FULL), p.v_col0 + hk * HD + kc * 64, k_row);
+        }
+      }
+      bool ok = true;
+      for (int it = 0; ok && it < n_iter; ++it) {
+        const int s = it & 1;
+        const int g = it / n_q, i = i_lo + it % n_q;
+        const int h = hk * group + g;
+        const int q_row = b * p.Tq + i * BQ;
+        if (it >= 2) ok = mbar_wait(bar(B_::Q_EMPTY + s), ((it >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_expect_tx(bar(B_::Q_FULL + s), TILE);
+          for (int kc = 0; kc < KC; ++kc)
+            tma_load_2d(sQ + s * TILE + kc * (128 * 128), &p.tmQ, bar(B_::Q_FULL + s), p.q_col0 + h * HD + kc * 64, q_row);
+        }
+        if (it >= 1) ok = mbar_wait(bar(B_::DO_EMPTY), (it - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_expect_tx(bar(B_::DO_FULL), TILE);
+          for (int kc = 0; kc < KC; ++kc)
+            tma_load_2d(sdO + kc * (128 * 128), &p.tmdO, bar(B_::DO_FULL), p.do_col0 + h * HD + kc * 64, q_row);
+        }
+        // rows with no visible key at all (L = -inf) and rows past the end get P = 0 through an infinite offset
+        const long long row0 = ((long long)b * p.H + h) * p.Tq + i * BQ;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int r = u * 32 + lane;
+          const bool real = i * BQ + r < p.Tq;
+          const float L = real ? __ldg(p.lse + row0 + r) : -CUDART_INF_F;
+          const float dl = real ? __ldg(p.delta + row0 + r) : 0.f;
+          rows_s[s * 256 + r] = (L == -CUDART_INF_F) ? -CUDART_INF_F : -L * 1.4426950408889634f;
+          rows_s[s * 256 + 128 + r] = -dl * p.scale;
+        }
+        mbar_arrive(bar(B_::DO_FULL));
+      }
+    }
+  } else if (warp == 13) {
+    if (lane == 0 && n_iter > 0) {
+      // ------------------------------------------------------------------ products
+      constexpr uint32_t id_s = umma_idesc_bf16(128, 128, 0, 0);        // K Q^T and V dO^T: both K-major over head_dim
+      constexpr uint32_t id_t = umma_idesc_bf16(128, HD, 0, 1);         // P^T dO and dS^T Q: A along the queries, B MN-major
+      constexpr uint32_t id_q = umma_idesc_bf16(128, HD, 1, 1);         // dS K: A read across the keys
+      auto issue_nt = [&](uint32_t d, uint32_t a, uint32_t bm) {
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t off = kc * (128 * 128) + k * 32;
+            umma_f16<1>(d, umma_smem_desc(a + off, 16, 1024), umma_smem_desc(bm + off, 16, 1024), id_s, (kc | k) ? 1u : 0u);
+          }
+      };
+      bool ok = mbar_wait(bar(B_::KV_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      if (ok) ok = mbar_wait(bar(B_::Q_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      if (ok) {
+        tc_fence_after();
+        issue_nt(tmem + C_S, sK, sQ);
+        umma_commit(bar(B_::S_FULL));
+        ok = mbar_wait(bar(B_::DO_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      }
+      if (ok) {
+        tc_fence_after();
+        issue_nt(tmem + C_DP, sV, sdO);
+        umma_commit(bar(B_::DP_FULL));
+      }
+      for (int it = 0; ok && it < n_iter; ++it) {
+        const int s = it & 1, sn = s ^ 1;
+        const uint32_t qt = sQ + s * TILE;
+        ok = mbar_wait(bar(B_::P_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < 8; ++k)                    // P^T: 64 queries in columns 0.., the others in columns 64..
+          umma_f16_ts(tmem + C_DV, tmem + C_S + (k < 4 ? k * 8 : 64 + (k - 4) * 8), umma_smem_desc(sdO + k * 2048, 128 * 128, 1024),
+                      id_t, (it | k) ? 1u : 0u);
+        umma_commit(bar(B_::DO_EMPTY));
+        if (it + 1 < n_iter) {
+          ok = mbar_wait(bar(B_::Q_FULL + sn), ((it + 1) >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+          if (!ok) break;
+          tc_fence_after();
+          issue_nt(tmem + C_S, sK, sQ + sn * TILE);
+          umma_commit(bar(B_::S_FULL));
+        }
+        ok = mbar_wait(bar(B_::DS_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          umma_f16<1>(tmem + C_DQ, umma_smem_desc(sdS + k * 2048, 128 * 128, 1024), umma_smem_desc(sK + k * 2048, 128 * 128, 1024),
+                      id_q, k ? 1u : 0u);
+        umma_commit(bar(B_::DQ_FULL));
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          umma_f16<1>(tmem + C_DK, umma_smem_desc(sdS + (k / 4) * (128 * 128) + (k % 4) * 32, 16, 1024),
+                      umma_smem_desc(qt + k * 2048, 128 * 128, 1024), id_t, (it | k) ? 1u : 0u);
+        umma_commit(bar(B_::Q_EMPTY + s));
+        if (it + 1 < n_iter) {
+          ok = mbar_wait(bar(B_::DO_FULL), (it + 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+          if (ok) ok = mbar_wait(bar(B_::DQ_READ), it & 1, abort_smem, p.status, SITE_TMEM_EMPTY);
+          if (!ok) break;
+          tc_fence_after();
+          issue_nt(tmem + C_DP, sV, sdO);
+          umma_commit(bar(B_::DP_FULL));               // also: dK and dQ of this block are done with dS
+        }
+      }
+      if (ok) umma_commit(bar(B_::ACC_DONE));
+    }
+  } else if (warp >= 8) {
+    // -------------------------------------------------------------------- dQ into the float accumulator
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C_DQ;
+    const uint32_t stage = sRed + (warp & 3) * 8192;
+    bool ok = true;
+    for (int it = 0; it < n_iter; ++it) {
+      const int g = it / n_q, i = i_lo + it % n_q;
+      const int h = hk * group + g;
+      ok = mbar_wait(bar(B_::DQ_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32(lane_addr + c * 32, r);
+        tmem_ld_wait();
+        if (c == HD / 32 - 1) {
+          tc_fence_before();
+          mbar_arrive(bar(B_::DQ_READ));
+        }
+        if (lane == 0) tma_store_wait_read<1>();       // the piece before the last one has left its buffer
+        __syncwarp();
+        const uint32_t buf = stage + (c & 1) * 4096 + lane * 128;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + ((j ^ (lane & 7)) << 4)), "r"(r[4 * j]),
+                       "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3]) : "memory");
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_reduce_add_3d(&p.tmdQ, stage + (c & 1) * 4096, h * HD + c * 32, i * BQ + (warp & 3) * 32, b);
+          tma_store_commit();
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait_all<0>();
+  } else {
+    // -------------------------------------------------------------------- P^T and dS^T: thread = key row, half of the queries
+    const int row = threadIdx.x & 127;                 // == TMEM lane
+    const int half = threadIdx.x >> 7;
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int kj = k0 + row;
+    const int kpos = p.k_off + kj * p.k_stride;
+    // visible queries of this key: indices [q_first, q_end)
+    int q_first = 0, q_end = 0x7fffffff;
+    if (p.causal) q_first = kpos - p.q_off <= 0 ? 0 : (kpos - p.q_off + p.q_stride - 1) / p.q_stride;
+    if (p.window > 0) {                                // q_pos <= kpos + window - 1
+      const int last = kpos + p.window - 1 - p.q_off;
+      q_end = last < 0 ? 0 : last / p.q_stride + 1;
+    }
+    if (kj >= p.Tk) q_end = 0;
+    bool ok = true;
+    for (int it = 0; it < n_iter; ++it) {
+      const int i = i_lo + it % n_q;
+      const float4* nl = reinterpret_cast<const float4*>(rows_s + (it & 1) * 256 + half * 64);
+      const float4* nd = nl + 32;
+      // does a mask or the end of the keys cut into this (query block, key block) pair?
+      const int qpos_lo = p.q_off + i * BQ * p.q_stride, qpos_hi = p.q_off + (i * BQ + BQ - 1) * p.q_stride;
+      const bool masked = (k0 + BKV > p.Tk) || (p.causal && kpos_hi > qpos_lo) ||
+                          (p.window > 0 && kpos_lo <= qpos_hi - p.window);
+      ok = mbar_wait(bar(B_::DO_FULL), it & 1, abort_smem, p.status, SITE_SMEM_FULL);   // L and Delta
+      if (ok) ok = mbar_wait(bar(B_::S_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      float pv[64];
+      const int first = q_first - i * BQ - half * 64, end = q_end - i * BQ - half * 64;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {                    // P of 32 queries takes 16 columns that have been read
+        uint32_t rs[32], w[16];
+        tmem_ld_32x32(lane_addr + C_S + half * 64 + c * 32, rs);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float4 L4 = nl[c * 8 + e];
+          const float L[4] = {L4.x, L4.y, L4.z, L4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            pv[c * 32 + e * 4 + u] = ex2_approx(fmaf(__uint_as_float(rs[e * 4 + u]), p.scale_log2, L[u]));
+        }
+        if (masked) {
+#pragma unroll
+          for (int e = c * 32; e < c * 32 + 32; ++e)
+            if (e < first || e >= end) pv[e] = 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          __nv_bfloat162 hb = __floats2bfloat162_rn(pv[c * 32 + 2 * e], pv[c * 32 + 2 * e + 1]);
+          w[e] = *reinterpret_cast<uint32_t*>(&hb);
+        }
+        tmem_st_32x16(lane_addr + C_S + half * 64 + c * 16, w);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(bar(B_::P_FULL));
+      ok = mbar_wait(bar(B_::DP_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t rp[32], w[16];
+        tmem_ld_32x32(lane_addr + C_DP + half * 64 + c * 32, rp);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float4 d4 = nd[c * 8 + e];
+          const int o = 4 * e;
+          __nv_bfloat162 a = __floats2bfloat162_rn(pv[c * 32 + o] * fmaf(__uint_as_float(rp[o]), p.scale, d4.x),
+                                                   pv[c * 32 + o + 1] * fmaf(__uint_as_float(rp[o + 1]), p.scale, d4.y));
+          __nv_bfloat162 bb = __floats2bfloat162_rn(pv[c * 32 + o + 2] * fmaf(__uint_as_float(rp[o + 2]), p.scale, d4.z),
+                                                    pv[c * 32 + o + 3] * fmaf(__uint_as_float(rp[o + 3]), p.scale, d4.w));
+          w[2 * e] = *reinterpret_cast<uint32_t*>(&a);
+          w[2 * e + 1] = *reinterpret_cast<uint32_t*>(&bb);
+        }
+        store_row32(sdS, row, half * 2 + c, w);
+      }
+      fence_proxy_async_smem();
+      tc_fence_before();
+      mbar_arrive(bar(B_::DS_FULL));
+    }
+    // ---- dK, dV of this key block (thread = key row, half of the head dimension)
+    if (ok && n_iter > 0) {
+      ok = mbar_wait(bar(B_::ACC_DONE), 0, abort_smem, p.status, SITE_TMEM_FULL);
+      tc_fence_after();
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok && n_iter > 0) write_dkv<HD>(p, lane_addr + C_DV, lane_addr + C_DK, b, hk, kj, half);
+    else if (n_iter == 0 && !p.dk_acc && half == 0) zero_dkv<HD>(p, b, hk, kj);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 13) {
+    tc_fence_after();
+    tmem_dealloc<1>(tmem, 512);
+  }
+}
+
+// Delta = rowsum(dO o O) of the [rows, H, HD] matrices, stored as [B, H, T]; `zero` (fp32 [rows, H, HD], may be null) is
+// cleared on the way: the accumulator of dQ.  HD / 8 lanes share a row of a head.
+template <int HD>
+__global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ dout, long long ld_do,
+                                                    const __nv_bfloat16* __restrict__ out, long long ld_o, float* __restrict__ delta,
+                                                    float* __restrict__ zero, int B, int T, int H) {
+  constexpr int L = HD / 8;
+  const long long total = (long long)B * T * H * L;
+  for (long long idx = blockIdx.x * 256ll + threadIdx.x; idx < total; idx += gridDim.x * 256ll) {   // total is a multiple of L
+    const int v = (int)(idx % L);
+    const long long rh = idx / L;
+    const int h = (int)(rh % H);
+    const long long row = rh / H;
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(dout + row * ld_do + (long long)h * HD) + v);
+    const uint4 o = __ldg(reinterpret_cast<const uint4*>(out + row * ld_o + (long long)h * HD) + v);
+    const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&o);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(o2[i]);
+      s += x.x * y.x + x.y * y.y;
+    }
+    const unsigned lanes = __activemask();             // whole groups of L lanes are in or out of the last pass together
+#pragma unroll
+    for (int m = L / 2; m > 0; m >>= 1) s += __shfl_xor_sync(lanes, s, m);
+    if (v == 0) {
+      const long long b = row / T, t = row % T;
+      delta[(b * H + h) * T + t] = s;
+    }
+    if (zero) {
+      float4* z = reinterpret_cast<float4*>(zero + rh * HD) + 2 * v;
+      z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+}
+
 static bool map2d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t ld) {
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
   cuuint32_t box[2] = {64, 128};
   cuuint32_t es[2] = {1, 1};
   return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+static bool map_dq(CUtensorMap* tm, const float* dq, const MeshFlashArgs& f, long long ld, int hd) {
+  cuuint64_t dims[3] = {(cuuint64_t)f.H * hd, (cuuint64_t)f.Tq, (cuuint64_t)f.B};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)f.Tq * ld * 4};
+  cuuint32_t box[3] = {32, 32, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dq, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int HD>
@@ -352,6 +771,7 @@ static int launch(const MeshFlashBwdArgs* a, cudaStream_t stream) {
   if (!map2d(&p.tmK, f.k, (uint64_t)f.k_cols, (uint64_t)f.B * f.Tk, (uint64_t)f.ldk)) return last_error_code();
   if (!map2d(&p.tmV, f.v, (uint64_t)f.v_cols, (uint64_t)f.B * f.Tk, (uint64_t)f.ldv)) return last_error_code();
   if (!map2d(&p.tmdO, a->dout, (uint64_t)a->do_cols, (uint64_t)f.B * f.Tq, (uint64_t)a->ld_do)) return last_error_code();
+  if (!map_dq(&p.tmdQ, a->dq, f, a->ld_dq, HD)) return last_error_code();
   p.lse = f.lse; p.delta = a->delta; p.dq = a->dq; p.dk = (__nv_bfloat16*)a->dk; p.dv = (__nv_bfloat16*)a->dv;
   p.dk_acc = a->dk_acc; p.dv_acc = a->dv_acc;
   p.ld_dq = a->ld_dq; p.ld_dkv = a->ld_dkv;
@@ -367,13 +787,23 @@ static int launch(const MeshFlashBwdArgs* a, cudaStream_t stream) {
   p.drop.k1 = (uint32_t)(f.seed >> 32);
   p.drop.site = f.site;
   p.head_off = f.head_off; p.heads_total = f.heads_total > 0 ? f.heads_total : f.H;
-  static bool configured = false;
-  if (!configured) {
-    MESH_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    configured = true;
+  if (p.drop.p > 0.f) {
+    static bool configured = false;
+    if (!configured) {
+      MESH_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+      configured = true;
+    }
+    dim3 grid((f.Tk + BKV - 1) / BKV, f.Hkv, f.B);
+    flash_bwd_kernel<HD><<<grid, THREADS, SMEM, stream>>>(p);
+  } else {
+    static bool configured = false;
+    if (!configured) {
+      MESH_CUDA_OK(cudaFuncSetAttribute(flash_bwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg2<HD>::SMEM));
+      configured = true;
+    }
+    dim3 grid(f.Hkv * f.B, (f.Tk + BKV - 1) / BKV);
+    flash_bwd2_kernel<HD><<<grid, THREADS2, Cfg2<HD>::SMEM, stream>>>(p);
   }
-  dim3 grid((f.Tk + BKV - 1) / BKV, f.Hkv, f.B);
-  flash_bwd_kernel<HD><<<grid, THREADS, SMEM, stream>>>(p);
   MESH_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -392,4 +822,26 @@ extern "C" int mesh_flash_attention_bwd(const MeshFlashBwdArgs* a, void* stream)
     case 128: return fab::launch<128>(a, (cudaStream_t)stream);
     default: return set_error(-2, "flash_attention_bwd: head_dim must be 64 or 128 (dK and dV live in tensor memory)");
   }
+}
+
+extern "C" int mesh_attention_delta(const void* dout, long long ld_do, const void* out, long long ld_o, float* delta, float* zero,
+                                    int B, int T, int H, int head_dim, void* stream) {
+  using namespace mesh;
+  if (ld_do % 8 || ld_o % 8 || (uintptr_t)dout % 16 || (uintptr_t)out % 16 || (uintptr_t)zero % 16)
+    return set_error(-2, "attention_delta: rows must be 16-byte aligned");
+  const long long groups = (long long)B * T * H * (head_dim / 8);
+  if (groups <= 0) return 0;
+  const unsigned grid = (unsigned)((groups + 255) / 256 < 148 * 16 ? (groups + 255) / 256 : 148 * 16);
+#define MESH_DELTA(HD)                                                                                                       \
+  fab::delta_kernel<HD><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dout, ld_do, (const __nv_bfloat16*)out, \
+                                                                ld_o, delta, zero, B, T, H)
+  switch (head_dim) {
+    case 64: MESH_DELTA(64); break;
+    case 128: MESH_DELTA(128); break;
+    case 256: MESH_DELTA(256); break;
+    default: return set_error(-2, "attention_delta: head_dim must be 64, 128 or 256");
+  }
+#undef MESH_DELTA
+  MESH_CUDA_OK(cudaGetLastError());
+  return 0;
 }

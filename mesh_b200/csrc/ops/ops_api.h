@@ -78,6 +78,11 @@ typedef struct MeshFlashBwdArgs {
 } MeshFlashBwdArgs;
 int mesh_flash_attention_bwd(const MeshFlashBwdArgs* a, void* stream);
 
+// delta[b, h, t] = sum over the head of dout * out (bf16, [B*T, H*head_dim] with leading dimensions ld_do, ld_o); when
+// `zero` is given the dense fp32 matrix [B*T, H*head_dim] behind it is cleared in the same pass (the dq accumulator).
+int mesh_attention_delta(const void* dout, long long ld_do, const void* out, long long ld_o, float* delta, float* zero,
+                         int B, int T, int H, int head_dim, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -152,6 +152,25 @@ class _FlashBwd(ctypes.Structure):
                 ("dv_acc", c_void_p), ("ld_dq", c_longlong), ("ld_dkv", c_longlong)]
 
 
+def _delta(dout, out, clear=None):
+    """``rowsum(dout * out)`` as ``[B, H, T]``; ``clear``: a dense fp32 ``[B, T, H, hd]`` set to zero in the same pass."""
+    B, T, H, hd = dout.shape
+    dense = all(t.dtype == torch.bfloat16 and t.is_cuda and t.shape == dout.shape and t.stride(3) == 1 and t.stride(2) == hd
+                and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 and (B == 1 or t.stride(0) == T * t.stride(1)) for t in (dout, out))
+    if not dense or hd not in (64, 128, 256):
+        if clear is not None:
+            clear.zero_()
+        return (dout.float() * out.float()).sum(-1).transpose(1, 2).contiguous()
+    delta = torch.empty((B, H, T), dtype=torch.float32, device=dout.device)
+    rc = _native.lib().mesh_attention_delta(c_void_p(dout.data_ptr()), c_longlong(dout.stride(1)), c_void_p(out.data_ptr()),
+                                            c_longlong(out.stride(1)), c_void_p(delta.data_ptr()),
+                                            c_void_p(0 if clear is None else clear.data_ptr()), c_int(B), c_int(T), c_int(H),
+                                            c_int(hd), c_void_p(torch.cuda.current_stream().cuda_stream))
+    _native.check(rc, "mesh_attention_delta")
+    _native.count_launch()
+    return delta
+
+
 def flash_attention_backward(q, k, v, out, lse, dout, *, causal=True, window=0, scale=None, q_off=0, q_stride=1,
                              k_off=0, k_stride=1, delta=None, dq=None, dkv_acc=None, dropout=None):
     """Gradients of :func:`flash_attention`.  Returns ``(dq fp32 [B,Tq,H,hd], dk, dv)``.
@@ -165,7 +184,9 @@ def flash_attention_backward(q, k, v, out, lse, dout, *, causal=True, window=0, 
     scale = hd ** -0.5 if scale is None else scale
     dout = dout.contiguous()
     if delta is None:
-        delta = (dout.float() * out.float()).sum(-1).transpose(1, 2).contiguous()       # [B, H, Tq]
+        clear = torch.empty((B, Tq, H, hd), dtype=torch.float32, device=q.device) if dq is None and hd in (64, 128) else None
+        delta = _delta(dout, out, clear)
+        dq = clear if clear is not None else dq
     if dq is None:
         dq = torch.zeros((B, Tq, H, hd), dtype=torch.float32, device=q.device)
     if hd not in (64, 128):
@@ -284,8 +305,8 @@ class _RingAttention(torch.autograd.Function):
         P, r = comm.world, comm.rank
         B, T, H, hd = q.shape
         dout = dout.contiguous()
-        delta = (dout.float() * out.float()).sum(-1).transpose(1, 2).contiguous()
-        dq = torch.zeros((B, T, H, hd), dtype=torch.float32, device=q.device)
+        dq = torch.empty((B, T, H, hd), dtype=torch.float32, device=q.device)
+        delta = _delta(dout, out, dq)
         kv = torch.stack([k, v]).contiguous()
         dkv = torch.zeros(kv.shape, dtype=torch.float32, device=q.device)
         ring = [(j, (j + 1) % P) for j in range(P)]

@@ -240,3 +240,47 @@ def test_flash_backward_with_dropout(hd, H, Hkv):
     _close(q.grad, qf.grad, 3e-2)
     _close(k.grad, kf.grad, 3e-2)
     _close(v.grad, vf.grad, 3e-2)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,Tq,Tk,H,Hkv,causal,window,off,stride", [
+    (1, 1, 1, 1, 1, True, 0, (0, 0), 1),             # a single key: its output is v, its score gradients vanish
+    (2, 129, 129, 2, 1, True, 0, (0, 0), 1),         # one row past a tile
+    (1, 257, 257, 4, 2, True, 1, (0, 0), 1),         # a window of one key
+    (2, 383, 640, 2, 2, False, 0, (0, 0), 1),        # ragged ends, several key blocks
+    (1, 700, 700, 4, 1, True, 130, (0, 0), 1),       # the window moves the first key block of the two query tiles apart
+    (1, 512, 512, 2, 2, True, 0, (1, 0), 2),         # striped positions
+    (1, 300, 512, 2, 2, True, 0, (0, 150), 1),       # queries that see no key
+])
+def test_flash_tiles(hd, B, Tq, Tk, H, Hkv, causal, window, off, stride):
+    """Both directions at the edges of the query tiles and key blocks.  Probabilities, score gradients and results are
+    rounded to bf16 (2^-9 each): three of them in quadrature stay below 4e-3; twice that is allowed."""
+    from mesh_b200.ops.attention import attention_ref, flash_attention, flash_attention_backward
+    from mesh_b200.utils.status import check_status
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, do = (torch.randn(B, Tq, H, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Tk, Hkv, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    kw = dict(causal=causal, window=window, q_off=off[0], q_stride=stride, k_off=off[1], k_stride=stride)
+    out, lse = flash_attention(q, k, v, need_lse=True, **kw)
+    dq, dk, dv = flash_attention_backward(q, k, v, out, lse, do, **kw)
+    check_status()
+    qf, kf, vf = (t.double().requires_grad_(True) for t in (q, k, v))
+    s = torch.einsum("bthd,bshd->bhts", qf, kf.repeat_interleave(H // Hkv, 2)) * hd ** -0.5
+    qp, kp = off[0] + torch.arange(Tq, device="cuda") * stride, off[1] + torch.arange(Tk, device="cuda") * stride
+    hide = torch.zeros(Tq, Tk, dtype=torch.bool, device="cuda")
+    if causal:
+        hide |= kp[None] > qp[:, None]
+    if window:
+        hide |= kp[None] <= qp[:, None] - window
+    s = s.masked_fill(hide, float("-inf"))
+    blind = hide.all(-1)
+    pr = torch.softmax(s.masked_fill(blind[:, None], 0.0), -1).masked_fill(blind[:, None], 0.0)
+    ref = torch.einsum("bhts,bshd->bthd", pr, vf.repeat_interleave(H // Hkv, 2))
+    grads = torch.autograd.grad(ref, (qf, kf, vf), do.double())
+    for got, want in zip((out, dq, dk, dv), (ref, *grads)):
+        err = float((got.double() - want).detach().norm())
+        # where the exact value vanishes (one visible key per query) what is left is the rounding of dP - Delta
+        assert err <= 8e-3 * max(float(want.detach().norm()), float(do.double().norm()) * 0.5), (err, float(want.detach().norm()))
+    seen = ~blind
+    torch.testing.assert_close(lse[:, :, seen].double(), torch.logsumexp(s, -1)[:, :, seen].detach(), atol=1e-4, rtol=1e-4)
+    assert bool(torch.isinf(lse[:, :, blind]).all())
