@@ -21,8 +21,6 @@ constexpr int ATT_WARPS = 8;
 constexpr int MAX_GROUPS = 8;    // query heads per KV head, at most
 constexpr int MAX_HD = 256;
 
-// Each warp takes keys j = warp, warp+8, ... of the CTA's slice.  A lane owns head_dim/32 = up to 8
-// consecutive dims (16 bytes of K and of V per key).
 struct AttArgs {
   const __nv_bfloat16* q; const __nv_bfloat16* kc; const __nv_bfloat16* vc; const int* pos;
   __nv_bfloat16* out; float* scratch; int* counters;
@@ -30,102 +28,163 @@ struct AttArgs {
   int B, head_dim;                                   // used by callers that loop over the work items themselves
 };
 
-// One work item (split, kv head, sequence-token b) of the attention; `sm_acc_raw`: ATT_WARPS * group * HD floats of
-// shared memory.  The ATT_THREADS computing threads call it together (`sync` is their barrier).
 struct AttBlockSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
 
+// PER consecutive bf16 of a cache row, as stored
+template <int PER> struct Raw;
+template <> struct Raw<8> { uint4 v; };
+template <> struct Raw<4> { uint2 v; };
+template <> struct Raw<2> { uint32_t v; };
+template <int PER>
+__device__ __forceinline__ void widen(const Raw<PER>& r, float (&f)[PER]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+  for (int i = 0; i < PER / 2; ++i) {
+    const float2 t = __bfloat1622float2(h[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
+// Running softmax of one warp over its keys.  A lane owns HD / 32 consecutive dims of K, V and the accumulators; m and l
+// are those of head `lane / 2 % MAXG`, the head whose scores the lane holds after the reduction below.
+template <int HD, int MAXG>
+struct WarpState {
+  static constexpr int PER = HD / 32;
+  static constexpr int KEYS = 16 / MAXG;              // keys a warp takes at a time: 16 scores, two lanes each
+  float m, l, acc[MAXG][PER];
+};
+
+// Keys of this warp: KEYS consecutive ones starting at lo + gw * KEYS, then every `warps` * KEYS further, up to hi.  All
+// loads of a step are issued together (a key costs a trip to L2 or HBM, not two); the 16 partial dot products are
+// reduced with 16 shuffles instead of 5 each, and every lane then works on one score: one exponential, not 16.
+template <int HD, int MAXG>
+__device__ __forceinline__ void scan_keys(const AttArgs& A, int kvh, int b, int lo, int hi, int gw, int warps,
+                                          WarpState<HD, MAXG>& st) {
+  constexpr int PER = HD / 32, KEYS = WarpState<HD, MAXG>::KEYS;
+  const int lane = threadIdx.x & 31;
+  const int group = A.q_heads / A.kv_heads;
+  const int seq_idx = b / A.T;
+  // no __restrict__ here: inside a step kernel q and the newest cache row were written by an earlier phase of the
+  // same kernel, and a read-only (non-coherent) load could return what the line held before
+  const __nv_bfloat16* kbase = A.kc + ((long long)seq_idx * A.kv_heads + kvh) * A.max_seq * HD + lane * PER;
+  const __nv_bfloat16* vbase = A.vc + ((long long)seq_idx * A.kv_heads + kvh) * A.max_seq * HD + lane * PER;
+  float qv[MAXG][PER];                                // query vectors of the group, scaled
+#pragma unroll
+  for (int g = 0; g < MAXG; ++g) {
+    Raw<PER> r = {};
+    if (g < group) r = *reinterpret_cast<const Raw<PER>*>(A.q + ((long long)b * A.q_heads + kvh * group + g) * HD + lane * PER);
+    widen<PER>(r, qv[g]);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) qv[g][i] *= A.scale;
+  }
+  st.m = -CUDART_INF_F;
+  st.l = 0.f;
+#pragma unroll
+  for (int g = 0; g < MAXG; ++g)
+#pragma unroll
+    for (int i = 0; i < PER; ++i) st.acc[g][i] = 0.f;
+  const int my = lane >> 1;                           // the (key, head) whose score this lane holds
+  const int my_key = my / MAXG;
+  for (int j = lo + gw * KEYS; j < hi; j += warps * KEYS) {
+    Raw<PER> kr[KEYS], vr[KEYS];
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) {
+      const long long at = (long long)min(j + k, hi - 1) * HD;
+      kr[k] = *reinterpret_cast<const Raw<PER>*>(kbase + at);
+      vr[k] = *reinterpret_cast<const Raw<PER>*>(vbase + at);
+    }
+    float s[16];
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) {
+      float kf[PER];
+      widen<PER>(kr[k], kf);
+#pragma unroll
+      for (int g = 0; g < MAXG; ++g) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) t += qv[g][i] * kf[i];
+        s[k * MAXG + g] = t;
+      }
+    }
+    // after the step with offset o a lane keeps the half of its values that its bit o names
+#pragma unroll
+    for (int o = 16, n = 8; o > 1; o >>= 1, n >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float send = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    float sc = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+    if (j + my_key >= hi) sc = -CUDART_INF_F;
+    float mx = sc;                                    // over the keys of this head
+#pragma unroll
+    for (int o = 16; o >= 2 * MAXG; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float mn = fmaxf(st.m, mx);                 // finite: key j exists
+    const float corr = __expf(st.m - mn), w = __expf(sc - mn);
+    float ws = w;
+#pragma unroll
+    for (int o = 16; o >= 2 * MAXG; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    st.l = st.l * corr + ws;
+    st.m = mn;
+#pragma unroll
+    for (int g = 0; g < MAXG; ++g) {
+      const float cg = __shfl_sync(0xffffffffu, corr, 2 * g);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) st.acc[g][i] *= cg;
+    }
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) {
+      float vf[PER];
+      widen<PER>(vr[k], vf);
+#pragma unroll
+      for (int g = 0; g < MAXG; ++g) {
+        const float wg = __shfl_sync(0xffffffffu, w, 2 * (k * MAXG + g));
+#pragma unroll
+        for (int i = 0; i < PER; ++i) st.acc[g][i] += wg * vf[i];
+      }
+    }
+  }
+}
+
+// The keys query token b sees: [lo, hi).
+__device__ __forceinline__ void visible(const AttArgs& A, int b, int& lo, int& hi) {
+  const int seq_idx = b / A.T;
+  const int p = A.pos[seq_idx] + (b - seq_idx * A.T);
+  lo = (A.window > 0) ? max(0, p - A.window + 1) : 0;
+  hi = p + 1;
+}
+
+// One work item (split, kv head, sequence-token b) of the attention; `sm_acc_raw`: ATT_WARPS * group * HD floats of
+// shared memory.  The ATT_THREADS computing threads call it together (`sync` is their barrier).
 template <int HD, int MAXG, class Sync = AttBlockSync>
 __device__ __forceinline__ void attention_item(const AttArgs& A, int split, int kvh, int b, float* sm_acc_raw,
                                                Sync sync = Sync{}) {
-  constexpr int PER = HD / 32;                       // dims per lane
+  constexpr int PER = HD / 32;
   constexpr int MAX_GROUP = MAXG;
-  // no __restrict__ here: inside a step kernel q and the newest cache row were written by an earlier phase of the
-  // same kernel, and a read-only (non-coherent) load could return what the line held before
-  const __nv_bfloat16* q = A.q;
-  const __nv_bfloat16* kc = A.kc;
-  const __nv_bfloat16* vc = A.vc;
-  const int* pos = A.pos;
   __nv_bfloat16* out = A.out;
   float* scratch = A.scratch;
   int* counters = A.counters;
-  const int q_heads = A.q_heads, kv_heads = A.kv_heads, max_seq = A.max_seq, window = A.window, splits = A.splits, T = A.T;
-  const float scale = A.scale;
-  // b indexes (sequence, query token); the cache belongs to the sequence
-  const int seq_idx = b / T;
+  const int q_heads = A.q_heads, kv_heads = A.kv_heads, splits = A.splits;
   const int group = q_heads / kv_heads;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = pos[seq_idx] + (b - seq_idx * T);
-  const int lo_all = (window > 0) ? max(0, p - window + 1) : 0;
-  const int n_keys = p + 1 - lo_all;
-  const int per_split = (n_keys + splits - 1) / splits;
+  int lo_all, hi_all;
+  visible(A, b, lo_all, hi_all);
+  const int per_split = (hi_all - lo_all + splits - 1) / splits;
   const int lo = lo_all + split * per_split;
-  const int hi = min(p + 1, lo + per_split);
-
-  // query vectors of the group, scaled, in registers
-  float qv[MAX_GROUP][PER];
-#pragma unroll
-  for (int g = 0; g < MAX_GROUP; ++g) {
-    if (g < group) {
-      const __nv_bfloat16* qp = q + ((long long)b * q_heads + kvh * group + g) * HD + lane * PER;
-#pragma unroll
-      for (int i = 0; i < PER; ++i) qv[g][i] = __bfloat162float(qp[i]) * scale;
-    }
-  }
-  float m[MAX_GROUP], l[MAX_GROUP], acc[MAX_GROUP][PER];
-#pragma unroll
-  for (int g = 0; g < MAX_GROUP; ++g) {
-    m[g] = -CUDART_INF_F;
-    l[g] = 0.f;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) acc[g][i] = 0.f;
-  }
-  const __nv_bfloat16* kbase = kc + ((long long)seq_idx * kv_heads + kvh) * max_seq * HD + lane * PER;
-  const __nv_bfloat16* vbase = vc + ((long long)seq_idx * kv_heads + kvh) * max_seq * HD + lane * PER;
-  for (int j = lo + warp; j < hi; j += ATT_WARPS) {
-    float kf[PER], vf[PER];
-    if constexpr (PER == 8) {
-      const uint4 kq = *reinterpret_cast<const uint4*>(kbase + (long long)j * HD);
-      const uint4 vq = *reinterpret_cast<const uint4*>(vbase + (long long)j * HD);
-      const __nv_bfloat162* kh = reinterpret_cast<const __nv_bfloat162*>(&kq);
-      const __nv_bfloat162* vh = reinterpret_cast<const __nv_bfloat162*>(&vq);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 a = __bfloat1622float2(kh[i]), c = __bfloat1622float2(vh[i]);
-        kf[2 * i] = a.x; kf[2 * i + 1] = a.y; vf[2 * i] = c.x; vf[2 * i + 1] = c.y;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        kf[i] = __bfloat162float(kbase[(long long)j * HD + i]);
-        vf[i] = __bfloat162float(vbase[(long long)j * HD + i]);
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < MAX_GROUP; ++g) {
-      if (g < group) {
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) s += qv[g][i] * kf[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        const float mn = fmaxf(m[g], s);
-        const float corr = __expf(m[g] - mn), w = __expf(s - mn);
-        l[g] = l[g] * corr + w;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) acc[g][i] = acc[g][i] * corr + w * vf[i];
-        m[g] = mn;
-      }
-    }
-  }
+  WarpState<HD, MAXG> st;
+  scan_keys<HD, MAXG>(A, kvh, b, lo, min(hi_all, lo + per_split), warp, ATT_WARPS, st);
   // ---- merge the 8 warps of the CTA through shared memory
   __shared__ float sm_m[ATT_WARPS][MAX_GROUP], sm_l[ATT_WARPS][MAX_GROUP];
   auto sm_acc = [&](int w, int g, int d) -> float& { return sm_acc_raw[((long long)w * group + g) * HD + d]; };
 #pragma unroll
   for (int g = 0; g < MAX_GROUP; ++g) {
     if (g < group) {
-      if (lane == 0) { sm_m[warp][g] = m[g]; sm_l[warp][g] = l[g]; }
+      if (lane == 2 * g) { sm_m[warp][g] = st.m; sm_l[warp][g] = st.l; }
 #pragma unroll
-      for (int i = 0; i < PER; ++i) sm_acc(warp, g, lane * PER + i) = acc[g][i];
+      for (int i = 0; i < PER; ++i) sm_acc(warp, g, lane * PER + i) = st.acc[g][i];
     }
   }
   sync();

@@ -53,14 +53,13 @@ struct LinArgs {
   const uint32_t* step_ptr; uint32_t calls_per_step, call_index;   // sequence number = step * calls + index + 1
   const __nv_bfloat16* residual; long long ldr;       // [B, N]
   Status* status;
-  int l2_prefetch;
   const uint8_t* next_w; unsigned long long next_bytes;   // weights of the linear layer that follows in the stream
   int xpad;                                           // bytes of padding per x row in shared memory (bank spread)
 };
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(                                                   // not volatile: loads of the next products may pass it
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -253,44 +252,48 @@ __device__ __forceinline__ void mma_chunk(const Chunk<W4, U>& c, const uint8_t* 
 // Barrier among the threads that compute a layer: the whole CTA of a stand-alone launch.
 struct BlockSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
 
-// The B rows of x -> shared memory, optionally RMS-normalised.  Called by the THREADS computing threads together.
+// The B rows of x -> shared memory, optionally RMS-normalised.  Called by the THREADS computing threads together.  The
+// warps share the rows out (all eight work on the row of a batch of one), so that the loads of a short batch are all in
+// flight at once; a thread normalises what it loaded itself.
 template <class Sync>
 __device__ __forceinline__ void stage_x(const LinArgs& a, uint8_t* xs, int xstride, Sync sync) {
-  __shared__ float rstd_s[NB];
-  const int K = a.K;
+  __shared__ float part_s[WARPS];
+  const int nvec = a.K >> 3;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  {
-    const int nvec = K >> 3;
-    for (int b = warp; b < a.B; b += WARPS) {
-      float ss = 0.f;
-      for (int v = lane; v < nvec; v += 32) {
-        const uint4 q = *reinterpret_cast<const uint4*>(a.x + (long long)b * a.ldx + v * 8);
-        *reinterpret_cast<uint4*>(xs + b * xstride + v * 16) = q;
-        if (a.norm_w) {
-          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+  const int wpr = a.B > 4 ? 1 : a.B > 2 ? 2 : a.B > 1 ? 4 : 8;      // warps per row
+  const int b = warp / wpr, first = (warp % wpr) * 32 + lane, stride = wpr * 32;
+  float ss = 0.f;
+  if (b < a.B) {
+#pragma unroll 4
+    for (int v = first; v < nvec; v += stride) {
+      const uint4 q = *reinterpret_cast<const uint4*>(a.x + (long long)b * a.ldx + v * 8);
+      *reinterpret_cast<uint4*>(xs + b * xstride + v * 16) = q;
+      if (a.norm_w) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float2 f = __bfloat1622float2(h[i]);
-            ss += f.x * f.x + f.y * f.y;
-          }
+        for (int i = 0; i < 4; ++i) {
+          float2 f = __bfloat1622float2(h[i]);
+          ss += f.x * f.x + f.y * f.y;
         }
       }
-      if (a.norm_w) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) rstd_s[b] = rsqrtf(ss / (float)K + a.eps);
-      }
     }
+  }
+  if (a.norm_w) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) part_s[warp] = ss;
     sync();
-    if (a.norm_w) {
-      for (int idx = threadIdx.x; idx < a.B * nvec; idx += THREADS) {
-        const int b = idx / nvec, v = idx % nvec;
+    if (b < a.B) {
+      float t = 0.f;
+      for (int w = 0; w < wpr; ++w) t += part_s[b * wpr + w];
+      const float r = rsqrtf(t / (float)a.K + a.eps);
+#pragma unroll 4
+      for (int v = first; v < nvec; v += stride) {
         uint4* p = reinterpret_cast<uint4*>(xs + b * xstride + v * 16);
         uint4 q = *p;
         const uint4 wq = *reinterpret_cast<const uint4*>(a.norm_w + v * 8);
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
         const __nv_bfloat162* wh = reinterpret_cast<const __nv_bfloat162*>(&wq);
-        const float r = rstd_s[b];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           float2 f = __bfloat1622float2(h[i]);
@@ -299,60 +302,59 @@ __device__ __forceinline__ void stage_x(const LinArgs& a, uint8_t* xs, int xstri
         }
         *p = q;
       }
-      sync();
     }
   }
-
+  sync();
 }
 
 // K-split reduction of one 16-row group through shared memory, then the layer's epilogue.  c: this thread's partial
-// sums (c0,c1 = row g8, batch 2t,2t+1; c2,c3 = row g8+8).  Ends with the computing threads in step.
+// sums (c0,c1 = row g8, batch 2t,2t+1; c2,c3 = row g8+8).  `red`: [WARPS][16][NB], two of them used in turn: a thread
+// writes the partials of group g + 2 only after the barrier of group g + 1, which everybody reaches after reading those
+// of group g, so one barrier per group is enough.
 template <class Sync>
-__device__ __forceinline__ void finish_group(const LinArgs& a, int grp, float (&c)[4], float* red, float* fin, Sync sync) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g8 = lane >> 2, t4 = lane & 3;
+__device__ __forceinline__ void finish_group(const LinArgs& a, int grp, const float (&c)[4], int g8, float* red, Sync sync) {
+  const int warp = threadIdx.x >> 5, t4 = threadIdx.x & 3;
     int rA, rB;
     group_rows(a, grp, rA, rB);
-    // ---- K-split reduction through shared memory: c0,c1 = (row g8, batch 2t,2t+1); c2,c3 = row g8+8
     float* my = red + warp * 16 * NB;
-    my[g8 * NB + 2 * t4] = c[0];
-    my[g8 * NB + 2 * t4 + 1] = c[1];
-    my[(g8 + 8) * NB + 2 * t4] = c[2];
-    my[(g8 + 8) * NB + 2 * t4 + 1] = c[3];
+    *reinterpret_cast<float2*>(my + g8 * NB + 2 * t4) = make_float2(c[0], c[1]);
+    *reinterpret_cast<float2*>(my + (g8 + 8) * NB + 2 * t4) = make_float2(c[2], c[3]);
     sync();
-    if (threadIdx.x < 16 * NB) {
+    auto sum = [&](int e) {
       float s = 0.f;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) s += red[w * 16 * NB + threadIdx.x];
-      fin[threadIdx.x] = s;
-    }
-    sync();
+      for (int w = 0; w < WARPS; ++w) s += red[w * 16 * NB + e];
+      return s;
+    };
     // ---- epilogue: thread e = (row r of 16, batch n)
     if (threadIdx.x < 16 * NB) {
       const int r = threadIdx.x / NB, n = threadIdx.x % NB;
-      const float val = fin[threadIdx.x];
       const int row = (r < 8) ? rA + r : rB + (r - 8);
       if (a.mode == MESH_DEC_STORE) {
         if (n < a.B) {
-          float val = fin[threadIdx.x];
+          float val = sum(threadIdx.x);
           if (a.residual) val += __bfloat162float(a.residual[(long long)n * a.ldr + row]);
           if (a.out_f32) reinterpret_cast<float*>(a.out)[(long long)n * a.ldo + row] = val;
           else reinterpret_cast<__nv_bfloat16*>(a.out)[(long long)n * a.ldo + row] = __float2bfloat16_rn(val);
         }
       } else if (a.mode == MESH_DEC_GLU) {
         if (r < 8 && n < a.B) {
-          const float u = fin[(r + 8) * NB + n];
+          const float val = sum(threadIdx.x), u = sum(threadIdx.x + 8 * NB);
           reinterpret_cast<__nv_bfloat16*>(a.out)[(long long)n * a.ldo + row] = __float2bfloat16_rn(dec_act(val, a.act) * u);
         }
       } else if (a.mode == MESH_DEC_QKV) {
         if (r < 8 && n < a.B) {
           const int hd = a.head_dim, half = hd / 2;
           const int h = row / hd, i = row % hd;            // i < half
-          const float lo = val, hi = fin[(r + 8) * NB + n];
           const int p = a.pos[n];
-          float o_lo = lo, o_hi = hi;
+          float cs = 1.f, sn = 0.f;
           if (h < a.q_heads + a.kv_heads) {                  // q and k heads are rotated
-            const float cs = a.cos_t[(long long)p * half + i], sn = a.sin_t[(long long)p * half + i];
+            cs = a.cos_t[(long long)p * half + i];
+            sn = a.sin_t[(long long)p * half + i];
+          }
+          const float lo = sum(threadIdx.x), hi = sum(threadIdx.x + 8 * NB);
+          float o_lo = lo, o_hi = hi;
+          if (h < a.q_heads + a.kv_heads) {
             o_lo = lo * cs - hi * sn;
             o_hi = hi * cs + lo * sn;
           }
@@ -369,6 +371,7 @@ __device__ __forceinline__ void finish_group(const LinArgs& a, int grp, float (&
         }
       } else {   // MESH_DEC_ALLREDUCE: one-shot sum over ranks of this row group, plus the residual
         if (n < a.B) {
+          const float val = sum(threadIdx.x);
           // the two halves of the slot array alternate call by call, so a fast peer's next
           // reduction never lands on words a slow rank has not read yet
           const uint32_t ar_seq = (a.step_ptr ? *a.step_ptr : 0u) * a.calls_per_step + a.call_index + 1u;
@@ -407,12 +410,28 @@ __device__ __forceinline__ void finish_group(const LinArgs& a, int grp, float (&
         }
       }
     }
-  sync();
 }
 
-// Shared memory a launch needs for a layer of width K and batch B: the staged rows of x plus the K-split partials.
+// Shared memory a layer of width K and batch B needs: the staged rows of x plus the K-split partials.
+constexpr int RED_FLOATS = WARPS * 16 * NB;
+__host__ __device__ inline size_t xsum_bytes(int K, bool coded) { return coded ? (size_t)(K / 64) * NB * sizeof(float) : 0; }
 __host__ __device__ inline size_t lin_smem_bytes(int K, int B) {
-  return (size_t)B * ((size_t)K * 2 + XPAD) + (size_t)(WARPS + 1) * 16 * NB * sizeof(float);
+  return (size_t)B * ((size_t)K * 2 + XPAD) + (size_t)2 * RED_FLOATS * sizeof(float);
+}
+
+// The layer that follows streams weights that depend on nothing computed here: ask for them to be brought into L2
+// now, behind this kernel's own loads, so that HBM keeps streaming through this kernel's reduction and epilogue,
+// the kernel boundary and the next kernel's prologue.  Every CTA requests its slice in 16 KiB pieces.
+__device__ __forceinline__ void prefetch_next(const LinArgs& a, int threads) {
+  if (a.next_w == nullptr) return;
+  constexpr unsigned long long PIECE = 16384;
+  const unsigned long long pieces = (a.next_bytes + PIECE - 1) / PIECE;
+  for (unsigned long long i = (unsigned long long)blockIdx.x * threads + threadIdx.x; i < pieces;
+       i += (unsigned long long)gridDim.x * threads) {
+    const unsigned long long off = i * PIECE;
+    const uint32_t n = (uint32_t)((a.next_bytes - off < PIECE ? a.next_bytes - off : PIECE) & ~15ull);
+    if (n) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.next_w + off), "r"(n) : "memory");
+  }
 }
 
 // The whole layer for one CTA of a grid of `gridDim.x` (groups blockIdx.x, blockIdx.x + gridDim.x, ...).
@@ -424,8 +443,7 @@ __device__ __forceinline__ void linear_body(const LinArgs& a, uint8_t* smem, Wai
   const int K = a.K;
   const int xstride = K * 2 + a.xpad;                             // bytes per x row
   uint8_t* xs = smem;                                             // [B][xstride]
-  float* red = reinterpret_cast<float*>(smem + (size_t)a.B * (K * 2 + XPAD));   // [WARPS][16][NB]
-  float* fin = red + WARPS * 16 * NB;                             // [16][NB]
+  float* red = reinterpret_cast<float*>(smem + (size_t)a.B * (K * 2 + XPAD));   // 2 x [WARPS][16][NB]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g8 = lane >> 2, t4 = lane & 3;
   constexpr int CH = ChunkK<W4, U>::value;
@@ -439,19 +457,6 @@ __device__ __forceinline__ void linear_body(const LinArgs& a, uint8_t* smem, Wai
   const LinHot hot{a.w, a.scales, a.K, a.mode, a.up_off, a.head_dim};
   Chunk<W4, U> c0, c1;
   if (steps > 0) load_chunk<W4, U>(hot, blockIdx.x, 0, k_lo, g8, t4, c0);
-  if (a.l2_prefetch) {
-    // Every row this CTA will read is requested into L2 now, while the kernel before this one in the stream is
-    // still running (this kernel's CTAs are resident beside it): HBM keeps streaming across the kernel boundary and
-    // the loads below find their bytes in L2.  One bulk prefetch per row (16 rows per group).
-    const long long row_bytes = W4 == 0 ? (long long)K * 2 : (W4 == 3 ? (long long)K : (long long)K / 2);
-    for (int i = threadIdx.x; i < my_groups * 16; i += THREADS) {
-      int rA, rB;
-      group_rows(a, blockIdx.x + (i >> 4) * gridDim.x, rA, rB);
-      const int row = ((i & 15) < 8) ? rA + (i & 15) : rB + (i & 15) - 8;
-      const uint8_t* src = reinterpret_cast<const uint8_t*>(a.w) + (long long)row * row_bytes;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"((uint32_t)row_bytes) : "memory");
-    }
-  }
   wait_inputs();
 
   stage_x(a, xs, xstride, BlockSync{});
@@ -459,19 +464,7 @@ __device__ __forceinline__ void linear_body(const LinArgs& a, uint8_t* smem, Wai
   const uint8_t* xbase = xs + (g8 < a.B ? g8 : a.B - 1) * xstride + (k_lo + lane_k<W4>(t4)) * 2;
   float c[4] = {0.f, 0.f, 0.f, 0.f};
 
-  // The layer that follows streams weights that depend on nothing computed here: ask for them to be brought into L2
-  // now, behind this kernel's own loads, so that HBM keeps streaming through this kernel's reduction and epilogue,
-  // the kernel boundary and the next kernel's prologue.  Every CTA requests its slice in 16 KiB pieces.
-  if (a.next_w != nullptr) {
-    constexpr unsigned long long PIECE = 16384;
-    const unsigned long long pieces = (a.next_bytes + PIECE - 1) / PIECE;
-    for (unsigned long long i = (unsigned long long)blockIdx.x * THREADS + threadIdx.x; i < pieces;
-         i += (unsigned long long)gridDim.x * THREADS) {
-      const unsigned long long off = i * PIECE;
-      const uint32_t n = (uint32_t)((a.next_bytes - off < PIECE ? a.next_bytes - off : PIECE) & ~15ull);
-      if (n) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.next_w + off), "r"(n) : "memory");
-    }
-  }
+  prefetch_next(a, THREADS);
 
   // Two register sets alternate: while one chunk feeds the tensor cores the next one is in flight,
   // across group boundaries too, so the stream of weight loads never drains.
@@ -486,9 +479,82 @@ __device__ __forceinline__ void linear_body(const LinArgs& a, uint8_t* smem, Wai
     if (step & 1) mma_chunk<W4, U>(c1, xbase + ci * CH * 2, c);
     else          mma_chunk<W4, U>(c0, xbase + ci * CH * 2, c);
     if (ci != chunks - 1) continue;
-    finish_group(a, grp, c, red, fin, BlockSync{});
+    finish_group(a, grp, c, g8, red + (gi & 1) * RED_FLOATS, BlockSync{});
     c[0] = c[1] = c[2] = c[3] = 0.f;
   }
+}
+
+// ---- codes in shared memory (the streaming kernels)
+template <class T>
+__device__ __forceinline__ T at(const uint8_t* p) { return *reinterpret_cast<const T*>(p); }
+// the eight nibbles of a word, i-th of each half in o[i], as the bf16 numbers 128 + nibble
+__device__ __forceinline__ void nibbles(uint32_t p, uint32_t (&o)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = ((p >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
+}
+
+// Sums of the staged x over every 64 k, times what the offset of a code adds to a product (-136 = -(128 + 8) for 4-bit,
+// -2304 = -(17 * 128 + 128) for 8-bit codes): xsum [K / 64][NB].  The computing threads call it together after stage_x.
+template <int W4, class Sync>
+__device__ __forceinline__ void sum_x(const LinArgs& a, const uint8_t* xs, int xstride, float* xsum, Sync sync) {
+  for (int i = threadIdx.x; i < a.K / 64 * NB; i += THREADS) {
+    const int n = i % NB;
+    if (n >= a.B) continue;
+    const uint4* xv = reinterpret_cast<const uint4*>(xs + n * xstride + (i / NB) * 128);
+    float s = 0.f;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const uint4 q = xv[v];
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(h[e]);
+        s += f.x + f.y;
+      }
+    }
+    xsum[i] = s * (W4 == 2 ? -136.f : -2304.f);
+  }
+  sync();
+}
+
+// 64 k of 16 rows: c += scale * (codes . x).  Codes enter the products as the bf16 numbers 128 + nibble, which are exact;
+// the scale, and what the offsets add (`off`: xsum of this group, batch columns 2 t4 and 2 t4 + 1), are applied to the sum
+// in fp32: half the instructions of scaling every weight, and no weight is rounded.  pA / pB: this
+// lane's 8 (4-bit) or 16 (8-bit) bytes of rows A and B, k = 16 t4 ..; xp: the lane's 16 x.
+template <int W4>
+__device__ __forceinline__ void mma_codes(const uint8_t* pA, const uint8_t* pB, float sa, float sb, float2 off, const uint8_t* xp, float (&c)[4]) {
+  const uint4 x0 = *reinterpret_cast<const uint4*>(xp), x1 = *reinterpret_cast<const uint4*>(xp + 16);
+  float lo[4] = {off.x, off.y, off.x, off.y};
+  uint32_t wa[4], wb[4];
+  if constexpr (W4 == 2) {
+    const uint2 pa = at<uint2>(pA), pb = at<uint2>(pB);
+    nibbles(pa.x, wa);
+    nibbles(pb.x, wb);
+    mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], x0.x, x0.y);
+    mma_bf16(lo, wa[2], wb[2], wa[3], wb[3], x0.z, x0.w);
+    nibbles(pa.y, wa);
+    nibbles(pb.y, wb);
+    mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], x1.x, x1.y);
+    mma_bf16(lo, wa[2], wb[2], wa[3], wb[3], x1.z, x1.w);
+  } else {
+    const uint4 pa = at<uint4>(pA), pb = at<uint4>(pB);
+    const uint32_t wpa[4] = {pa.x, pa.y, pa.z, pa.w}, wpb[4] = {pb.x, pb.y, pb.z, pb.w};
+    const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    float hi[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                          // four codes = low and high nibbles of two pairs
+      nibbles(__byte_perm(wpa[j], 0, 0x3120), wa);
+      nibbles(__byte_perm(wpb[j], 0, 0x3120), wb);
+      mma_bf16(lo, wa[0], wb[0], wa[2], wb[2], xw[2 * j], xw[2 * j + 1]);
+      mma_bf16(hi, wa[1], wb[1], wa[3], wb[3], xw[2 * j], xw[2 * j + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lo[i] = fmaf(16.f, hi[i], lo[i]);
+  }
+  c[0] = fmaf(sa, lo[0], c[0]);
+  c[1] = fmaf(sa, lo[1], c[1]);
+  c[2] = fmaf(sb, lo[2], c[2]);
+  c[3] = fmaf(sb, lo[3], c[3]);
 }
 
 // Kernel variants (weight format, chunk width), chosen from the layer's shape by `lin_prepare`.
@@ -547,22 +613,6 @@ inline int lin_prepare(const MeshDecodeLinear* d, LinArgs& a, int& variant) {
     variant = wide ? LIN_BF16_U4 : LIN_BF16_U1;
   }
   return 0;
-}
-
-// Runs the layer with the body that `variant` names.
-template <class Wait>
-__device__ __forceinline__ void linear_dispatch(int variant, const LinArgs& a, uint8_t* smem, Wait wait_inputs) {
-  switch (variant) {
-    case LIN_W4N_U2: linear_body<1, 2>(a, smem, wait_inputs); break;
-    case LIN_W4N_U1: linear_body<1, 1>(a, smem, wait_inputs); break;
-    case LIN_BF16_U4: linear_body<0, 4>(a, smem, wait_inputs); break;
-    case LIN_BF16_U1: linear_body<0, 1>(a, smem, wait_inputs); break;
-    case LIN_W8_U4: linear_body<3, 4>(a, smem, wait_inputs); break;
-    case LIN_W8_U2: linear_body<3, 2>(a, smem, wait_inputs); break;
-    case LIN_W8_U1: linear_body<3, 1>(a, smem, wait_inputs); break;
-    case LIN_W4W_U2: linear_body<2, 2>(a, smem, wait_inputs); break;
-    default: linear_body<2, 1>(a, smem, wait_inputs); break;
-  }
 }
 
 }  // namespace decode

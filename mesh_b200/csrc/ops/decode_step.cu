@@ -277,38 +277,29 @@ __host__ __device__ inline void variant_geom(int variant, int& kt, int& rowb, in
   }
 }
 
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ float lds_half(uint32_t addr) {
-  unsigned short h;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(addr));
-  return __half2float(__ushort_as_half(h));
-}
-
-// This warp's chunk of a stage -> registers, in the layout `mma_chunk` multiplies.
+// This warp's chunk of a stage: c += W x.
 template <int W4, int U>
-__device__ __forceinline__ void load_chunk_stage(uint32_t slot, int warp, int g8, int t4, Chunk<W4, U>& c) {
+__device__ __forceinline__ void mma_stage(const uint8_t* slot, int warp, int g8, int t4, int k0, const float* xsum,
+                                          const uint8_t* xp, float (&c)[4]) {
   using G = StageGeom<W4, U>;
   constexpr int WB = W4 == 0 ? G::CH * 2 : (W4 == 3 ? G::CH : G::CH / 2);     // bytes of a warp's k range in a row
-  const uint32_t ra = slot + (uint32_t)g8 * G::RS + (uint32_t)warp * WB + (uint32_t)t4 * 16;
-  const uint32_t rb = ra + 8u * G::RS;
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    c.a[u] = lds128(ra + 64u * u);
-    c.b[u] = lds128(rb + 64u * u);
-  }
-  if constexpr (W4 != 0) {
-    constexpr int BLK = W4 == 2 ? 128 : 64;
-    const uint32_t sc = slot + 16u * G::RS;
-    const int k_lane = warp * G::CH + lane_k<W4>(t4);
+  const uint8_t* ra = slot + g8 * G::RS + warp * WB;
+  if constexpr (W4 == 0) {
+    Chunk<W4, U> ch;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint32_t idx = (uint32_t)((k_lane + u * BLK) >> 6) * 2u;
-      c.sa[u] = lds_half(sc + (uint32_t)g8 * G::SROWB + idx);
-      c.sb[u] = lds_half(sc + (uint32_t)(g8 + 8) * G::SROWB + idx);
+      ch.a[u] = at<uint4>(ra + t4 * 16 + 64 * u);
+      ch.b[u] = at<uint4>(ra + t4 * 16 + 64 * u + 8 * G::RS);
+    }
+    mma_chunk<W4, U>(ch, xp, c);
+  } else {
+    const uint8_t* sc = slot + 16 * G::RS + g8 * G::SROWB + warp * G::CH / 64 * 2;
+    constexpr int GB = W4 == 2 ? 32 : 64;                                       // bytes of 64 codes
+#pragma unroll
+    for (int g = 0; g < G::CH / 64; ++g) {
+      const uint8_t* w = ra + g * GB + t4 * (GB / 4);
+      mma_codes<W4>(w, w + 8 * G::RS, __half2float(at<__half>(sc + 2 * g)), __half2float(at<__half>(sc + 8 * G::SROWB + 2 * g)),
+                    *reinterpret_cast<const float2*>(xsum + (k0 / 64 + g) * NB + 2 * t4), xp + g * 128, c);
     }
   }
 }
@@ -324,27 +315,30 @@ __device__ __forceinline__ void linear_stream(const LinArgs& a, uint8_t* work, R
   const int xstride = K * 2 + a.xpad;
   uint8_t* xs = work;
   float* red = reinterpret_cast<float*>(work + (size_t)a.B * (K * 2 + XPAD));
-  float* fin = red + WARPS * 16 * NB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g8 = lane >> 2, t4 = lane & 3;
   const int kstages = K / G::KT;
   if (wait) gb.wait();
-  if ((int)blockIdx.x < a.n_groups) stage_x(a, xs, xstride, ComputeSync{});      // a CTA with no group of this layer stages nothing
-  const uint8_t* xrow = xs + (g8 < a.B ? g8 : a.B - 1) * xstride + (warp * G::CH + lane_k<W4>(t4)) * 2;
+  float* xsum = red + 2 * RED_FLOATS;
+  if ((int)blockIdx.x < a.n_groups) {                                    // a CTA with no group of this layer stages nothing
+    stage_x(a, xs, xstride, ComputeSync{});
+    if constexpr (W4 != 0) sum_x<W4>(a, xs, xstride, xsum, ComputeSync{});
+  }
+  const uint8_t* xrow = xs + (g8 < a.B ? g8 : a.B - 1) * xstride + (warp * G::CH + t4 * (W4 == 0 ? 8 : 16)) * 2;
   float c[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
+  int turn = 0;
+  for (int grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x, turn ^= 1) {
     for (int ks = 0; ks < kstages; ++ks) {
       if (!*dead) mbar_wait(ring.full(), ring.phase, dead, a.status, SITE_SMEM_FULL);
-      Chunk<W4, U> ch;
-      load_chunk_stage<W4, U>(ring.slot(), warp, g8, t4, ch);
-      mma_chunk<W4, U>(ch, xrow + (size_t)ks * G::KT * 2, c);
+      mma_stage<W4, U>(reinterpret_cast<const uint8_t*>(__cvta_shared_to_generic(ring.slot())), warp, g8, t4, ks * G::KT + warp * G::CH, xsum, xrow + (size_t)ks * G::KT * 2, c);
       __syncwarp();
       if (lane == 0) mbar_arrive(ring.empty());
       ring.advance();
     }
-    finish_group(a, grp, c, red, fin, ComputeSync{});
+    finish_group(a, grp, c, g8, red + turn * RED_FLOATS, ComputeSync{});
     c[0] = c[1] = c[2] = c[3] = 0.f;
   }
+  ComputeSync{}();                       // the next operation reuses the shared memory
 }
 
 __device__ __forceinline__ void linear_stream_dispatch(int variant, const LinArgs& a, uint8_t* work, Ring& ring,
@@ -511,7 +505,6 @@ extern "C" int mesh_decode_step_prepare(const MeshDecodeOp* ops, int n_ops, void
       s.kind = DOP_LINEAR;
       const int rc = lin_prepare(&o.lin, s.lin, s.variant);
       if (rc) return rc;
-      s.lin.l2_prefetch = 0;
       s.lin.next_w = nullptr;
       s.lin.next_bytes = 0;
       int kt, rowb, srowb;
@@ -519,7 +512,7 @@ extern "C" int mesh_decode_step_prepare(const MeshDecodeOp* ops, int n_ops, void
       if (kt == 0) return set_error(-2, "decode_step: a layer of this width has no streamed form (K must be a multiple of 1024 for 4-bit weights)");
       if (((uintptr_t)o.lin.w & 15) || ((uintptr_t)o.lin.scales & 15))
         return set_error(-2, "decode_step: weights and scales must be 16-byte aligned");
-      work = std::max(work, lin_smem_bytes(o.lin.K, o.lin.B));
+      work = std::max(work, lin_smem_bytes(o.lin.K, o.lin.B) + xsum_bytes(o.lin.K, o.lin.w4 != 0));
       slot = std::max(slot, (size_t)16 * (rowb + ROW_PAD) + (size_t)16 * srowb);
     } else if (o.kind == MESH_DEC_OP_ATTENTION) {
       if (o.B < 1 || o.q_heads % o.kv_heads || o.q_heads / o.kv_heads > 4)

@@ -140,3 +140,70 @@ def test_decode_argmax():
     decode_argmax(logits, tok, pos, vocab_offset=1000, step=step)
     assert tok.tolist() == (logits.argmax(-1) + 1000).tolist() and tok[2].item() == 1777
     assert pos.tolist() == [1, 1, 1, 1] and step.tolist() == [1, 0]
+
+
+@pytest.mark.parametrize("bits,B,K,N", [(16, 1, 256, 16), (16, 2, 768, 2384), (16, 8, 8192, 2400), (16, 5, 2560, 32), (4, 1, 1024, 48),
+                                        (4, 8, 3072, 2384), (4, 3, 6144, 16), (4, 2, 1536, 64), (8, 1, 512, 16), (8, 8, 1536, 2400), (8, 3, 3072, 48)])
+def test_decode_linear_streams(bits, B, K, N):
+    """Short and long rings, one and several groups per CTA, odd numbers of stages.  Codes are exact inside the kernel and
+    sums are fp32, so what is left is the rounding of the result: half a step of 2^-7, 2^-8 of the value at most."""
+    from mesh_b200.ops.decode import decode_linear, quantize_w4, quantize_w8
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    x = torch.randn(B, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).bfloat16()
+    if bits == 16:
+        y, wd = decode_linear(x, w), w.double()
+    else:
+        codes, scales = (quantize_w4 if bits == 4 else quantize_w8)(w)
+        if bits == 4:
+            word = codes.view(torch.int32).to(torch.int64) & 0xFFFFFFFF
+            c = torch.stack([(word >> (4 * n)) & 15 for n in (0, 4, 1, 5, 2, 6, 3, 7)], -1).view(N, K).double() - 8
+        else:
+            c = codes.double() - 128
+        wd = (c.view(N, K // 64, 64) * scales.double()[..., None]).view(N, K)
+        y = decode_linear(x, codes, scales=scales)
+        odd = torch.empty(scales.numel() + 1, dtype=torch.float16, device="cuda")[1:].view_as(scales).copy_(scales)
+        _close(decode_linear(x, codes, scales=odd), y)                    # scales off the 16-byte grid: the other reader
+    want = x.double() @ wd.T
+    if bits == 4 and K % 1024:
+        wd = wd.bfloat16().double()                                       # that reader rounds the weights
+        want = x.double() @ wd.T
+    assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+
+
+@pytest.mark.parametrize("hd,qh,kvh,splits,S,window", [(256, 8, 1, 16, 300, 0), (128, 6, 2, 3, 300, 40), (64, 4, 4, 1, 64, 0),
+                                                       (256, 8, 2, 64, 5000, 0), (64, 8, 1, 8, 5000, 4500)])
+def test_decode_attention_clusters_and_splits(hd, qh, kvh, splits, S, window):
+    """Both kernels: a cluster per KV head (few splits or a short context) and many splits merged through memory."""
+    from mesh_b200.ops.decode import DecodeAttention
+    B = 3
+    g = torch.Generator(device="cuda").manual_seed(hd + S)
+    kc, vc = (torch.randn(B, kvh, S, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(B, qh * hd, device="cuda", generator=g).bfloat16()
+    pos = torch.tensor([0, S // 2, S - 1], dtype=torch.int32, device="cuda")
+    att = DecodeAttention(B, qh, kvh, hd, splits=splits)
+    out = torch.empty(B, qh * hd, device="cuda", dtype=torch.bfloat16)
+    for _ in range(2):
+        att(q, kc, vc, pos, out, window=window)
+    for b in range(B):
+        p = int(pos[b])
+        lo = max(0, p - window + 1) if window else 0
+        k, v = (t[b, :, lo:p + 1].double().repeat_interleave(qh // kvh, 0) for t in (kc, vc))
+        s = torch.einsum("hd,hkd->hk", q[b].view(qh, hd).double(), k) / math.sqrt(hd)
+        want = torch.einsum("hk,hkd->hd", torch.softmax(s, -1), v).reshape(-1)
+        # fp32 inside, one rounding to bf16 at the end: 2^-8 of the value at most
+        assert float((out[b].double() - want).norm() / want.norm()) < 2 ** -8
+
+
+@pytest.mark.parametrize("V,ld", [(1, 1), (5, 8), (16385, 16385), (262144, 262144)])
+def test_decode_argmax_slices(V, ld):
+    from mesh_b200.ops.decode import decode_argmax
+    B = 3
+    logits = torch.randn(B, ld, device="cuda")[:, :V]
+    logits[0, 0] = logits[0, V - 1] = 9.0                                 # tie between the first and the last slice
+    logits[1, V - 1] = 9.0
+    logits[2] = float("-inf")
+    logits[2, V // 2] = -1e30
+    tok = torch.zeros(B, dtype=torch.int32, device="cuda")
+    decode_argmax(logits, tok, None)
+    assert tok.tolist() == [0, V - 1, V // 2]
