@@ -5,6 +5,11 @@
 // columns here (online max / sum, the reference's statistics of compiler/mesh_compiler/operations.py:6281-6330), two
 // tiny all-reduces combine them, and the gradient (softmax - onehot) * g is formed from the logits again, so no fp32
 // copy of the logits or of their exponentials is ever stored.
+//
+// Bound by HBM: 8192 rows of 50304 logits (824 MB) are read in 160 us for the statistics (5.2 TB/s; 290 us before the
+// exponentials were batched) and read and written in 269 us for the gradient (6.1 TB/s).  Where the whole vocabulary is
+// here, losses, their mean and the gradient are these launches and one small one: 640 -> 434 us forward and backward,
+// some twenty tensor operations on the rows among what went.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -15,10 +20,12 @@ namespace mesh {
 namespace {
 
 constexpr int CE_THREADS = 256;
+constexpr float LOG2E = 1.4426950408889634f;
 
-__device__ __forceinline__ void online(float& m, float& s, float x) {
-  if (x > m) { s = s * __expf(m - x) + 1.f; m = x; }
-  else s += __expf(x - m);
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 __device__ __forceinline__ void merge(float& m, float& s, float m2, float s2) {
   const float mm = fmaxf(m, m2);
@@ -26,33 +33,65 @@ __device__ __forceinline__ void merge(float& m, float& s, float m2, float s2) {
   s = s * __expf(m - mm) + s2 * __expf(m2 - mm);
   m = mm;
 }
+__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(h[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+// Eight values at a time: one comparison with the running maximum, and the exponentials relative to it in one fma and one
+// ex2 each (value by value, with a branch and two exponentials in it, the pass ran at 2.8 TB/s).
+__device__ __forceinline__ void online8(float& m, float& s, const uint4& q) {
+  float f[8];
+  unpack8(q, f);
+  const float mx = fmaxf(fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])), fmaxf(fmaxf(f[4], f[5]), fmaxf(f[6], f[7])));
+  if (mx > m) { s *= __expf(m - mx); m = mx; }
+  const float off = (m == -CUDART_INF_F) ? 0.f : -m * LOG2E;
+  float a = 0.f, b = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    a += ex2_approx(fmaf(f[i], LOG2E, off));
+    b += ex2_approx(fmaf(f[i + 1], LOG2E, off));
+  }
+  s += a + b;
+}
+__device__ __forceinline__ void online(float& m, float& s, float x) {
+  if (x > m) { s = s * __expf(m - x) + 1.f; m = x; }
+  else s += m == -CUDART_INF_F ? 0.f : __expf(x - m);
+}
 
-// row_max[r], row_sum[r] (relative to row_max[r]) and target_logit[r] (0 when the target is not in this shard or ignored)
+// Elements of a row before its first 16-byte boundary (rows of an odd width start anywhere).
+__device__ __forceinline__ int head_of(const __nv_bfloat16* x, int cols) {
+  return min(cols, (int)(((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) >> 1));
+}
+
+// row_max[r], row_sum[r] (relative to row_max[r]) and target_logit[r] (0 when the target is not in this shard or ignored).
+// `loss` (may be null, the whole vocabulary is here then): the token's loss, 0 when ignored.
 __global__ void __launch_bounds__(CE_THREADS)
 ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int rows, int cols, const long long* __restrict__ targets,
                 long long vocab_start, long long ignore_index, float* __restrict__ row_max, float* __restrict__ row_sum,
-                float* __restrict__ target_logit) {
+                float* __restrict__ target_logit, float* __restrict__ loss) {
   __shared__ float sm[CE_THREADS / 32], ss[CE_THREADS / 32];
-  const bool vec = (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const __nv_bfloat16* x = logits + (long long)r * ld;
     float m = -CUDART_INF_F, s = 0.f;
-    int done = 0;
-    if (vec) {
-      const int nv = cols >> 3;
-      for (int v = threadIdx.x; v < nv; v += CE_THREADS) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(x) + v);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+    const int head = head_of(x, cols);
+    const int nv = (cols - head) >> 3;
+    const uint4* xv = reinterpret_cast<const uint4*>(x + head);
+    int v = threadIdx.x;
+    for (; v + 3 * CE_THREADS < nv; v += 4 * CE_THREADS) {             // four loads in flight
+      uint4 q[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(h[i]);
-          online(m, s, f.x);
-          online(m, s, f.y);
-        }
-      }
-      done = nv << 3;
+      for (int u = 0; u < 4; ++u) q[u] = __ldg(xv + v + u * CE_THREADS);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) online8(m, s, q[u]);
     }
-    for (int c = done + threadIdx.x; c < cols; c += CE_THREADS) online(m, s, __bfloat162float(x[c]));
+    for (; v < nv; v += CE_THREADS) online8(m, s, __ldg(xv + v));
+    for (int c = threadIdx.x; c < head; c += CE_THREADS) online(m, s, __bfloat162float(x[c]));
+    for (int c = head + nv * 8 + threadIdx.x; c < cols; c += CE_THREADS) online(m, s, __bfloat162float(x[c]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
@@ -66,63 +105,142 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int rows
       row_max[r] = M;
       row_sum[r] = S;
       const long long t = targets[r], local = t - vocab_start;
-      target_logit[r] = (t != ignore_index && local >= 0 && local < cols) ? __bfloat162float(x[local]) : 0.f;
+      const float tl = (t != ignore_index && local >= 0 && local < cols) ? __bfloat162float(x[local]) : 0.f;
+      target_logit[r] = tl;
+      if (loss) loss[r] = t != ignore_index ? logf(S) + M - tl : 0.f;
     }
     __syncthreads();
   }
 }
 
-// d[r, c] = (exp(x - gmax[r]) / gsum[r] - [c == target]) * gscale[r]; gscale = upstream gradient, 0 for ignored rows
+// out = sum(loss), or that over the number of tokens that are not ignored (at least 1); divisor: what it was divided by.
+__global__ void __launch_bounds__(1024)
+ce_reduce_kernel(const float* __restrict__ loss, const long long* __restrict__ targets, int rows, long long ignore_index, int mean,
+                 float* __restrict__ out, float* __restrict__ divisor) {
+  __shared__ float sl[32];
+  __shared__ int sn[32];
+  float l = 0.f;
+  int n = 0;
+  for (int i = threadIdx.x; i < rows; i += 1024) {
+    l += loss[i];
+    n += targets[i] != ignore_index;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  if ((threadIdx.x & 31) == 0) { sl[threadIdx.x >> 5] = l; sn[threadIdx.x >> 5] = n; }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    l = sl[threadIdx.x];
+    n = sn[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      l += __shfl_xor_sync(0xffffffffu, l, o);
+      n += __shfl_xor_sync(0xffffffffu, n, o);
+    }
+    if (threadIdx.x == 0) {
+      const float div = mean ? (float)max(n, 1) : 1.f;
+      *out = l / div;
+      *divisor = div;
+    }
+  }
+}
+
+__device__ __forceinline__ uint4 grad8(const uint4& q, float off, float inv) {
+  float f[8];
+  unpack8(q, f);
+  uint4 o;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    h[i] = __floats2bfloat162_rn(ex2_approx(fmaf(f[2 * i], LOG2E, off)) * inv, ex2_approx(fmaf(f[2 * i + 1], LOG2E, off)) * inv);
+  return o;
+}
+
+// d[r, c] = (exp(x - gmax[r]) / gsum[r] - [c == target]) * g / divisor, 0 in ignored rows.  g: one value per row, or one for
+// all of them (g_stride 0); divisor: may be null.  The target's element is written once more after the row: no comparison
+// per element.
 __global__ void __launch_bounds__(CE_THREADS)
-ce_grad_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, __nv_bfloat16* __restrict__ d, long long ldd, int rows, int cols,
-               const long long* __restrict__ targets, long long vocab_start, const float* __restrict__ gmax,
-               const float* __restrict__ gsum, const float* __restrict__ gscale) {
-  const bool vec = (ld % 8 == 0) && (ldd % 8 == 0) && (((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(d)) & 15) == 0);
+ce_grad_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, __nv_bfloat16* d, long long ldd, int rows, int cols,
+               const long long* __restrict__ targets, long long vocab_start, long long ignore_index,
+               const float* __restrict__ gmax, const float* __restrict__ gsum, const float* __restrict__ gscale, int g_stride,
+               const float* __restrict__ divisor) {
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const __nv_bfloat16* x = logits + (long long)r * ld;
     __nv_bfloat16* o = d + (long long)r * ldd;
-    const float mx = gmax[r], g = gscale[r];
-    const float inv = g / gsum[r];
-    const long long local = targets[r] - vocab_start;
-    int done = 0;
-    if (vec) {
-      const int nv = cols >> 3;
-      for (int v = threadIdx.x; v < nv; v += CE_THREADS) {
-        uint4 q = __ldg(reinterpret_cast<const uint4*>(x) + v);
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+    const long long t = targets[r], local = t - vocab_start;
+    float g = gscale[(long long)r * g_stride];
+    if (divisor) g /= divisor[0];
+    if (t == ignore_index) g = 0.f;
+    const float off = -gmax[r] * LOG2E, inv = g / gsum[r];
+    const bool mine = local >= 0 && local < cols;
+    // d may be the logits themselves: the target's logit is read before its element is written
+    const float tx = (threadIdx.x == 0 && mine) ? __bfloat162float(x[local]) : 0.f;
+    __syncthreads();
+    const bool vec = ((reinterpret_cast<uintptr_t>(x) ^ reinterpret_cast<uintptr_t>(o)) & 15) == 0;
+    const int head = vec ? head_of(x, cols) : cols;
+    const int nv = (cols - head) >> 3;
+    const uint4* xv = reinterpret_cast<const uint4*>(x + head);
+    uint4* ov = reinterpret_cast<uint4*>(o + head);
+    int v = threadIdx.x;
+    for (; v + 3 * CE_THREADS < nv; v += 4 * CE_THREADS) {
+      uint4 q[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(h[i]);
-          float a = __expf(f.x - mx) * inv, b = __expf(f.y - mx) * inv;
-          const int c = v * 8 + 2 * i;
-          if (c == local) a -= g;
-          if (c + 1 == local) b -= g;
-          h[i] = __floats2bfloat162_rn(a, b);
-        }
-        reinterpret_cast<uint4*>(o)[v] = q;
-      }
-      done = nv << 3;
+      for (int u = 0; u < 4; ++u) q[u] = xv[v + u * CE_THREADS];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) __stcs(ov + v + u * CE_THREADS, grad8(q[u], off, inv));
     }
-    for (int c = done + threadIdx.x; c < cols; c += CE_THREADS) {
-      float a = __expf(__bfloat162float(x[c]) - mx) * inv;
-      if (c == local) a -= g;
-      o[c] = __float2bfloat16_rn(a);
-    }
+    for (; v < nv; v += CE_THREADS) ov[v] = grad8(xv[v], off, inv);
+    for (int c = threadIdx.x; c < head; c += CE_THREADS) o[c] = __float2bfloat16_rn(ex2_approx(fmaf(__bfloat162float(x[c]), LOG2E, off)) * inv);
+    for (int c = head + nv * 8 + threadIdx.x; c < cols; c += CE_THREADS)
+      o[c] = __float2bfloat16_rn(ex2_approx(fmaf(__bfloat162float(x[c]), LOG2E, off)) * inv);
+    __syncthreads();
+    if (threadIdx.x == 0 && mine) o[local] = __float2bfloat16_rn(ex2_approx(fmaf(tx, LOG2E, off)) * inv - g);
   }
 }
 
 }  // namespace
 }  // namespace mesh
 
-extern "C" int mesh_ce_stats_bf16(const void* logits, long long ld, int rows, int cols, const long long* targets,
-                                  long long vocab_start, long long ignore_index, float* row_max, float* row_sum,
-                                  float* target_logit, void* stream) {
+extern "C" int mesh_ce_loss_bf16(const void* logits, long long ld, int rows, int cols, const long long* targets,
+                                 long long vocab_start, long long ignore_index, float* row_max, float* row_sum,
+                                 float* target_logit, float* loss, void* stream) {
   using namespace mesh;
   if (rows <= 0 || cols <= 0) return 0;
   if (!logits || !targets || !row_max || !row_sum || !target_logit) return set_error(-2, "ce_stats: null argument");
   int grid = rows < 148 * 8 ? rows : 148 * 8;
   ce_stats_kernel<<<grid, CE_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, ld, rows, cols, targets, vocab_start,
-                                                                ignore_index, row_max, row_sum, target_logit);
+                                                                ignore_index, row_max, row_sum, target_logit, loss);
+  MESH_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+extern "C" int mesh_ce_stats_bf16(const void* logits, long long ld, int rows, int cols, const long long* targets,
+                                  long long vocab_start, long long ignore_index, float* row_max, float* row_sum,
+                                  float* target_logit, void* stream) {
+  return mesh_ce_loss_bf16(logits, ld, rows, cols, targets, vocab_start, ignore_index, row_max, row_sum, target_logit, nullptr, stream);
+}
+
+extern "C" int mesh_ce_reduce(const float* loss, const long long* targets, int rows, long long ignore_index, int mean, float* out,
+                              float* divisor, void* stream) {
+  using namespace mesh;
+  if (!out || !divisor || (rows > 0 && (!loss || !targets))) return set_error(-2, "ce_reduce: null argument");
+  ce_reduce_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(loss, targets, rows, ignore_index, mean, out, divisor);
+  MESH_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+extern "C" int mesh_ce_grad_of_bf16(const void* logits, long long ld, void* dlogits, long long ldd, int rows, int cols,
+                                    const long long* targets, long long vocab_start, long long ignore_index, const float* gmax,
+                                    const float* gsum, const float* g, int g_stride, const float* divisor, void* stream) {
+  using namespace mesh;
+  if (rows <= 0 || cols <= 0) return 0;
+  if (!logits || !dlogits || !targets || !gmax || !gsum || !g) return set_error(-2, "ce_grad: null argument");
+  int grid = rows < 148 * 8 ? rows : 148 * 8;
+  ce_grad_kernel<<<grid, CE_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, ld, (__nv_bfloat16*)dlogits, ldd, rows, cols,
+                                                               targets, vocab_start, ignore_index, gmax, gsum, g, g_stride, divisor);
   MESH_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -130,12 +248,6 @@ extern "C" int mesh_ce_stats_bf16(const void* logits, long long ld, int rows, in
 extern "C" int mesh_ce_grad_bf16(const void* logits, long long ld, void* dlogits, long long ldd, int rows, int cols,
                                  const long long* targets, long long vocab_start, const float* gmax, const float* gsum,
                                  const float* gscale, void* stream) {
-  using namespace mesh;
-  if (rows <= 0 || cols <= 0) return 0;
-  if (!logits || !dlogits || !targets || !gmax || !gsum || !gscale) return set_error(-2, "ce_grad: null argument");
-  int grid = rows < 148 * 8 ? rows : 148 * 8;
-  ce_grad_kernel<<<grid, CE_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, ld, (__nv_bfloat16*)dlogits, ldd, rows, cols,
-                                                               targets, vocab_start, gmax, gsum, gscale);
-  MESH_CUDA_OK(cudaGetLastError());
-  return 0;
+  constexpr long long none = (long long)(1ull << 63);        // gscale is zero in ignored rows already
+  return mesh_ce_grad_of_bf16(logits, ld, dlogits, ldd, rows, cols, targets, vocab_start, none, gmax, gsum, gscale, 1, nullptr, stream);
 }

@@ -39,6 +39,18 @@ int mesh_ce_grad_bf16(const void* logits, long long ld, void* dlogits, long long
                       const long long* targets, long long vocab_start, const float* gmax, const float* gsum,
                       const float* gscale, void* stream);
 
+// The same statistics with the token's loss, log(row_sum) + row_max - target_logit, 0 when ignored: for logits that hold
+// the whole vocabulary.  mesh_ce_reduce: *out = sum of the losses, or their mean over the tokens that are not ignored
+// (mean = 1); *divisor = what the sum was divided by.  mesh_ce_grad_of_bf16: the gradient for upstream g[r * g_stride] (0: one
+// value for all rows), divided by *divisor when given, zero in ignored rows.
+int mesh_ce_loss_bf16(const void* logits, long long ld, int rows, int cols, const long long* targets, long long vocab_start,
+                      long long ignore_index, float* row_max, float* row_sum, float* target_logit, float* loss, void* stream);
+int mesh_ce_reduce(const float* loss, const long long* targets, int rows, long long ignore_index, int mean, float* out,
+                   float* divisor, void* stream);
+int mesh_ce_grad_of_bf16(const void* logits, long long ld, void* dlogits, long long ldd, int rows, int cols, const long long* targets,
+                         long long vocab_start, long long ignore_index, const float* gmax, const float* gsum, const float* g,
+                         int g_stride, const float* divisor, void* stream);
+
 // softmax over experts then top-k (k <= 8, experts <= 256).  bias (fp32[experts], may be NULL) is added
 // to the logits before the softmax.  weights fp32[tokens,k] (renormalised over the k when renorm),
 // indices int32[tokens,k]; ties go to the lower expert index.

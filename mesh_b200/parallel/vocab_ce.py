@@ -75,6 +75,56 @@ class _VocabParallelCEKernel(torch.autograd.Function):
         return d, None, None, None, None
 
 
+class _WholeVocabCEKernel(torch.autograd.Function):
+    """bf16 CUDA logits of the whole vocabulary (a group of one): statistics and losses in one kernel, their sum or mean in
+    another, the gradient in a third."""
+
+    @staticmethod
+    def forward(ctx, logits, targets, start, ignore_index, reduction):
+        from ctypes import c_int, c_longlong, c_void_p
+        from .. import _native
+        L = _native.lib()
+        n, v = logits.shape
+        t64 = targets.to(torch.int64).contiguous()
+        stats = torch.empty((3, n), dtype=torch.float32, device=logits.device)      # max, sum, target logit
+        loss = torch.empty(n, dtype=torch.float32, device=logits.device)
+        at = stats.data_ptr()
+        rc = L.mesh_ce_loss_bf16(c_void_p(logits.data_ptr()), c_longlong(logits.stride(0)), c_int(n), c_int(v), c_void_p(t64.data_ptr()),
+                                 c_longlong(start), c_longlong(ignore_index), c_void_p(at), c_void_p(at + 4 * n), c_void_p(at + 8 * n),
+                                 c_void_p(loss.data_ptr()), _s())
+        _native.check(rc, "mesh_ce_loss_bf16")
+        _native.count_launch()
+        divisor = None
+        if reduction != "none":
+            per_token, divisor = loss, torch.empty(1, dtype=torch.float32, device=logits.device)
+            loss = torch.empty((), dtype=torch.float32, device=logits.device)
+            rc = L.mesh_ce_reduce(c_void_p(per_token.data_ptr()), c_void_p(t64.data_ptr()), c_int(n), c_longlong(ignore_index),
+                                  c_int(int(reduction == "mean")), c_void_p(loss.data_ptr()), c_void_p(divisor.data_ptr()), _s())
+            _native.check(rc, "mesh_ce_reduce")
+            _native.count_launch()
+        ctx.save_for_backward(logits, t64, stats, divisor)
+        ctx.cfg = (start, ignore_index)
+        return loss
+
+    @staticmethod
+    def backward(ctx, g):
+        from ctypes import c_int, c_longlong, c_void_p
+        from .. import _native
+        logits, t64, stats, divisor = ctx.saved_tensors
+        start, ignore_index = ctx.cfg
+        n, v = logits.shape
+        g = g.float().contiguous()
+        d = torch.empty((n, v), dtype=torch.bfloat16, device=logits.device)
+        at = stats.data_ptr()
+        rc = _native.lib().mesh_ce_grad_of_bf16(c_void_p(logits.data_ptr()), c_longlong(logits.stride(0)), c_void_p(d.data_ptr()),
+                                                c_longlong(v), c_int(n), c_int(v), c_void_p(t64.data_ptr()), c_longlong(start),
+                                                c_longlong(ignore_index), c_void_p(at), c_void_p(at + 4 * n), c_void_p(g.data_ptr()),
+                                                c_int(int(divisor is None)), c_void_p(0 if divisor is None else divisor.data_ptr()), _s())
+        _native.check(rc, "mesh_ce_grad_of_bf16")
+        _native.count_launch()
+        return d, None, None, None, None
+
+
 class _VocabParallelCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, targets, start, group, ignore_index):
@@ -111,6 +161,11 @@ def vocab_parallel_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, vo
     context).  Returns the per-token losses (``reduction="none"``), their sum, or their mean over the tokens that are
     not ``ignore_index``."""
     if logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.stride(1) == 1:
+        # one launch each for losses, reduction and gradient where there is nobody to exchange statistics with; a target is
+        # a column of these logits there, or ignored (elsewhere a class of another rank has no column here)
+        if _world(group) == 1 and targets.is_cuda and targets.shape == logits.shape[:1]:
+            return _WholeVocabCEKernel.apply(logits, targets, int(vocab_start), int(ignore_index),
+                                             reduction if reduction in ("none", "sum") else "mean")
         loss = _VocabParallelCEKernel.apply(logits, targets, int(vocab_start), group, int(ignore_index))
     else:
         loss = _VocabParallelCE.apply(logits, targets, int(vocab_start), group, int(ignore_index))

@@ -86,3 +86,30 @@ def test_cross_entropy_kernels_match_fp32(n, v, start):
     want.backward()
     assert abs(float(loss) - float(want)) <= 2e-3 * abs(float(want)) + 1e-3
     assert float((logits.grad.float() - ref.grad).abs().max()) < 8e-3
+
+
+@pytest.mark.parametrize("n,v,ld,reduction", [(1, 1, 1, "mean"), (5, 7, 9, "none"), (3, 16384 + 9, 16384 + 9, "mean"), (1300, 2049, 2056, "sum"),
+                                              (4, 4096, 8192, "mean")])
+def test_cross_entropy_rows_of_any_alignment(n, v, ld, reduction):
+    """Rows that start off the 16-byte grid, a row stride that differs from the width, masked logits (-inf), all rows
+    ignored but one, targets in the first, the last and no column's vector body; losses in fp32 (relative 1e-5), gradients
+    rounded to bf16 (2^-8)."""
+    from mesh_b200.parallel.vocab_ce import vocab_parallel_cross_entropy
+    g = torch.Generator(device="cuda").manual_seed(v)
+    buf = (torch.randn(n, ld, device="cuda", generator=g) * 3).bfloat16()
+    logits = buf[:, :v].detach()
+    if v > 8:
+        logits[:, 2:5] = float("-inf")
+    logits.requires_grad_(True)
+    t = torch.tensor([0, v - 1, v // 2 if v > 16 else 0], device="cuda").repeat(-(-n // 3))[:n].contiguous()
+    if n > 3:
+        t[1:] = torch.where(torch.arange(1, n, device="cuda") % 4 == 0, -100, t[1:])
+    loss = vocab_parallel_cross_entropy(logits, t, 0, None, reduction=reduction)
+    up = torch.rand(loss.shape, device="cuda", generator=g) + 0.5
+    (d,) = torch.autograd.grad(loss, logits, up)
+    ref = logits.detach().double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(ref, t, ignore_index=-100, reduction=reduction)
+    (dw,) = torch.autograd.grad(want, ref, up.double())
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=1e-5, atol=1e-5)
+    # p - 1 cancels in the target's column: its error is fp32's of p (1e-6 of the upstream value)
+    assert bool(((d.double() - dw).abs() <= 2 ** -8 * dw.abs() + 2e-6 * float(up.max())).all())
