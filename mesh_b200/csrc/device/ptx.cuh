@@ -95,6 +95,19 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
   return ok;
 }
 
+// One look, without the suspension of a try_wait (several microseconds when the phase does not complete).
+__device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
+}
+
 // Bounded wait.  `abort_smem` is a CTA-wide word: the first role that gives up sets
 // it so the other roles leave their own waits within ~1k polls instead of each
 // running out its own limit.  Returns false when the caller must unwind.
@@ -114,6 +127,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
   return true;
+}
+
+// The same for a converged warp: every lane waits, and all of them get the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_smem, Status* st, int site) {
+  const bool ok = mbar_wait(bar, parity, abort_smem, st, site);
+  return __all_sync(0xffffffffu, ok);
 }
 
 // ----------------------------------------------------------------------------- fences

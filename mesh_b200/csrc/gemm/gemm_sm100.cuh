@@ -353,7 +353,9 @@ gemm_kernel(const __grid_constant__ Params p) {
 
   if (warp == 0) {
     // ===================================================================== TMA producer
-    if (lane == 0) {
+    // as below: the whole warp runs the loop, one elected lane waits for other kernels' rows and issues the copies
+    {
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -378,104 +380,127 @@ gemm_kernel(const __grid_constant__ Params p) {
         const int own_lo = AG ? p.rank * p.ag_rows_per_rank : 0;
         const bool own = AG && m0 >= own_lo && m0 < own_lo + p.ag_rows_per_rank;
         if (p.a_ready != nullptr && !own && (p.tiles != nullptr || m0 < p.M)) {
-          ok = wait_flag_ge(p.a_ready + m0 / p.a_ready_rows, p.a_ready_value, p.status, SITE_LOCAL_FLAG);
+          if (leader) {
+            ok = wait_flag_ge(p.a_ready + m0 / p.a_ready_rows, p.a_ready_value, p.status, SITE_LOCAL_FLAG);
+            fence_proxy_async_all();   // data was written through the generic proxy, TMA reads it
+          }
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) { *abort_smem = 1; break; }
-          fence_proxy_async_all();   // data was written through the generic proxy, TMA reads it
         }
         for (int kb = 0; kb < wk.k_blocks; ++kb) {
           const int ka = wk.ka0 + kb * BK, kbb = wk.kb0 + kb * BK;      // K coordinates in A and in B
           if (p.k_ready != nullptr) {
             const int need = (ka + BK - 1) / p.k_ready_rows + 1;
-            while (ok && k_checked < need) {
-              ok = wait_flag_ge(p.k_ready + k_checked, p.k_ready_value, p.status, SITE_LOCAL_FLAG);
-              ++k_checked;
-              if (ok && k_checked == need) fence_proxy_async_all();
+            if (k_checked < need) {
+              if (leader) {
+                while (ok && k_checked < need) ok = wait_flag_ge(p.k_ready + k_checked++, p.k_ready_value, p.status, SITE_LOCAL_FLAG);
+                if (ok) fence_proxy_async_all();
+              }
+              k_checked = need;
+              ok = __all_sync(0xffffffffu, ok);
+              if (!ok) { *abort_smem = 1; break; }
             }
-            if (!ok) { *abort_smem = 1; break; }
           }
-          ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_smem, p.status, SITE_SMEM_EMPTY);
+          ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_smem, p.status, SITE_SMEM_EMPTY);
           if (!ok) break;
-          const uint32_t sA = sA0 + stage * A_STAGE_BYTES;
-          const uint32_t sB = sB0 + stage * B_STAGE_BYTES;
-          if constexpr (!PAIR) {
-            const uint32_t fb = full_bar(stage);
-            mbar_expect_tx(fb, BQ != 0 ? A_STAGE_BYTES : STAGE_BYTES);
-            if (A_MN) tma_load_3d(sA, &p.tmA, fb, 0, ka, m0 / 64);
-            else if (own) tma_load_2d(sA, &p.tmA2, fb, ka, m0 - own_lo);
-            else      tma_load_2d(sA, &p.tmA, fb, ka, m0);
-            if (BQ != 0) {
-              // B is written by the dequantising warps
-            } else if (EPI == EPI_GLU_FWD) {
-              tma_load_2d(sB, &p.tmB, fb, kbb, n0);
-              tma_load_2d(sB + B_STAGE_BYTES / 2, &p.tmB, fb, kbb, p.b_up_rows + n0);
-            } else if (B_MN) {
-              tma_load_3d(sB, &p.tmB, fb, 0, kbb, n0 / 64);
+          if (leader) {
+            const uint32_t sA = sA0 + stage * A_STAGE_BYTES;
+            const uint32_t sB = sB0 + stage * B_STAGE_BYTES;
+            if constexpr (!PAIR) {
+              const uint32_t fb = full_bar(stage);
+              mbar_expect_tx(fb, BQ != 0 ? A_STAGE_BYTES : STAGE_BYTES);
+              if (A_MN) tma_load_3d(sA, &p.tmA, fb, 0, ka, m0 / 64);
+              else if (own) tma_load_2d(sA, &p.tmA2, fb, ka, m0 - own_lo);
+              else      tma_load_2d(sA, &p.tmA, fb, ka, m0);
+              if (BQ != 0) {
+                // B is written by the dequantising warps
+              } else if (EPI == EPI_GLU_FWD) {
+                tma_load_2d(sB, &p.tmB, fb, kbb, n0);
+                tma_load_2d(sB + B_STAGE_BYTES / 2, &p.tmB, fb, kbb, p.b_up_rows + n0);
+              } else if (B_MN) {
+                tma_load_3d(sB, &p.tmB, fb, 0, kbb, n0 / 64);
+              } else {
+                tma_load_2d(sB, &p.tmB, fb, kbb, n0);
+              }
             } else {
-              tma_load_2d(sB, &p.tmB, fb, kbb, n0);
-            }
-          } else {
-            // Both CTAs' bytes are counted on the leader's barrier; only the leader arms it.
-            if (cta_rank == 0) mbar_expect_tx(full_bar(stage), 2 * (BQ != 0 ? A_STAGE_BYTES : STAGE_BYTES));
-            const uint32_t fb = mapa_u32(full_bar(stage), 0);
-            if (A_MN) tma_load_3d_pair(sA, &p.tmA, fb, 0, ka, m0 / 64);
-            else if (own) tma_load_2d_pair(sA, &p.tmA2, fb, ka, m0 - own_lo);
-            else      tma_load_2d_pair(sA, &p.tmA, fb, ka, m0);
-            if (BQ != 0) {
-              // B is written by the dequantising warps
-            } else if (EPI == EPI_GLU_FWD) {
-              // leader stages the gate rows, its peer the up rows: accumulator columns [0,128) | [128,256)
-              tma_load_2d_pair(sB, &p.tmB, fb, kbb, (cta_rank ? p.b_up_rows : 0) + n0);
-            } else if (B_MN) {
-              tma_load_3d_pair(sB, &p.tmB, fb, 0, kbb, (n0 + (int)cta_rank * BN_CTA) / 64);
-            } else {
-              tma_load_2d_pair(sB, &p.tmB, fb, kbb, n0 + (int)cta_rank * BN_CTA);
+              // Both CTAs' bytes are counted on the leader's barrier; only the leader arms it.
+              if (cta_rank == 0) mbar_expect_tx(full_bar(stage), 2 * (BQ != 0 ? A_STAGE_BYTES : STAGE_BYTES));
+              const uint32_t fb = mapa_u32(full_bar(stage), 0);
+              if (A_MN) tma_load_3d_pair(sA, &p.tmA, fb, 0, ka, m0 / 64);
+              else if (own) tma_load_2d_pair(sA, &p.tmA2, fb, ka, m0 - own_lo);
+              else      tma_load_2d_pair(sA, &p.tmA, fb, ka, m0);
+              if (BQ != 0) {
+                // B is written by the dequantising warps
+              } else if (EPI == EPI_GLU_FWD) {
+                // leader stages the gate rows, its peer the up rows: accumulator columns [0,128) | [128,256)
+                tma_load_2d_pair(sB, &p.tmB, fb, kbb, (cta_rank ? p.b_up_rows : 0) + n0);
+              } else if (B_MN) {
+                tma_load_3d_pair(sB, &p.tmB, fb, 0, kbb, (n0 + (int)cta_rank * BN_CTA) / 64);
+              } else {
+                tma_load_2d_pair(sB, &p.tmB, fb, kbb, n0 + (int)cta_rank * BN_CTA);
+              }
             }
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
     // ===================================================================== MMA issuer
-    if (lane == 0 && cta_rank == 0) {
+    // The tensor core takes in little more than the products it is working on, so whatever the issuing warp does between
+    // two stages leaves it idle.  The loop is warp-uniform and one elected lane issues (in a lane's own branch every
+    // operand of a product is moved to a uniform register first), descriptors are counted up from the stage's, and the next
+    // stage's barrier is looked at while products are queued: a wait is some 75 cycles even when its barrier is complete,
+    // and a stage of a 128-wide tile computes for 256.
+    if (cta_rank == 0) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM * CTAS, BN, A_MN, B_MN);
+      // K-major: 16 k-elements = 32 B inside the 128 B swizzle row; 8-row groups 1 KiB apart.
+      // MN-major: 16 k-rows = 2 KiB; 64-element MN groups one TMA box (64 rows * 128 B) apart.
+      const uint64_t da0 = A_MN ? umma_smem_desc(sA0, 8192, 1024) : umma_smem_desc(sA0, 16, 1024);
+      const uint64_t db0 = B_MN ? umma_smem_desc(sB0, 8192, 1024) : umma_smem_desc(sB0, 16, 1024);
+      constexpr uint32_t a_step = (A_MN ? 2048 : 32) >> 4, b_step = (B_MN ? 2048 : 32) >> 4;
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      uint32_t ready = 0;                    // the next stage's barrier was seen complete
       int t = 0;
       for (int tile = tile_first; ok && tile < total_tiles; tile += tile_step, ++t) {
         const int acc = t & 1;
         const uint32_t acc_phase = (t >> 1) & 1;
-        ok = mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_smem, p.status, SITE_TMEM_EMPTY);
+        ok = mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_smem, p.status, SITE_TMEM_EMPTY);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         const int tile_k_blocks = p.tiles != nullptr ? p.tiles[tile].k_blocks : p.k_blocks;
         for (int kb = 0; kb < tile_k_blocks; ++kb) {
-          ok = mbar_wait(full_bar(stage), phase, abort_smem, p.status, SITE_SMEM_FULL);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t sA = sA0 + stage * A_STAGE_BYTES;
-          const uint32_t sB = sB0 + stage * B_STAGE_BYTES;
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            // K-major: 16 k-elements = 32 B inside the 128 B swizzle row; 8-row groups 1 KiB apart.
-            // MN-major: 16 k-rows = 2 KiB; 64-element MN groups one TMA box (64 rows * 128 B) apart.
-            const uint64_t da = A_MN ? umma_smem_desc(sA + k * 2048, 8192, 1024)
-                                     : umma_smem_desc(sA + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? umma_smem_desc(sB + k * 2048, 8192, 1024)
-                                     : umma_smem_desc(sB + k * 32, 16, 1024);
-            umma_f16<CTAS>(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+          if (!__all_sync(0xffffffffu, ready)) {
+            ok = mbar_wait_warp(full_bar(stage), phase, abort_smem, p.status, SITE_SMEM_FULL);
+            if (!ok) break;
           }
-          // stage is free (in both CTAs of a pair) once these MMAs have read it
-          if constexpr (PAIR) umma_commit_pair(empty_bar(stage), 3);
-          else umma_commit(empty_bar(stage));
+          tc_fence_after();
+          const uint64_t da = da0 + (uint32_t)(stage * (A_STAGE_BYTES >> 4)), db = db0 + (uint32_t)(stage * (B_STAGE_BYTES >> 4));
+          if (leader) {
+            umma_f16<CTAS>(d_tmem, da, db, idesc, kb != 0 ? 1u : 0u);
+            umma_f16<CTAS>(d_tmem, da + a_step, db + b_step, idesc, 1u);
+          }
+          const uint32_t bar_done = empty_bar(stage);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          ready = mbar_test_wait(full_bar(stage), phase);
+          if (leader) {
+#pragma unroll
+            for (int k = 2; k < BK / UMMA_K; ++k) umma_f16<CTAS>(d_tmem, da + k * a_step, db + k * b_step, idesc, 1u);
+            // stage is free (in both CTAs of a pair) once these MMAs have read it
+            if constexpr (PAIR) umma_commit_pair(bar_done, 3);
+            else umma_commit(bar_done);
+          }
         }
-        if (ok) {
+        if (ok && leader) {
           if constexpr (PAIR) umma_commit_pair(tfull_bar(acc), 3);
           else umma_commit(tfull_bar(acc));
         }
+        __syncwarp();
       }
     }
   } else if (warp < 2 + EPI_WARPS) {
