@@ -56,6 +56,25 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// two fp32 at a time
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
 template <int HD>
 struct Cfg {
   static constexpr int BKV = HD <= 128 ? 128 : 64;
@@ -424,7 +443,7 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = base, sK = sQ + 2 * C::TILE, sV = sK + 2 * C::TILE, bars = sV + 2 * C::TILE;
   auto bar = [&](int i) { return bars + 8u * i; };
-  constexpr int Q_FULL = 0, K_FULL = 1, V_FULL = 3, K_EMPTY = 5, V_EMPTY = 7, S_FULL = 9, P_FULL = 11, O_DONE = 13, N_BARS = 15;
+  constexpr int Q_FULL = 0, K_FULL = 1, V_FULL = 3, K_EMPTY = 5, V_EMPTY = 7, S_FULL = 9, P_FULL = 11, O_DONE = 13, P_HALF = 15, N_BARS = 17;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 6 * C::TILE + 8 * N_BARS);
   volatile int* abort_smem = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -467,6 +486,7 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
       mbar_init(bar(K_EMPTY + s), 1);
       mbar_init(bar(V_EMPTY + s), 1);
       mbar_init(bar(S_FULL + s), 1);
+      mbar_init(bar(P_HALF + s), TT);
       mbar_init(bar(P_FULL + s), TT);
       mbar_init(bar(O_DONE + s), 1);
     }
@@ -508,61 +528,71 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
       }
     }
   } else if (warp == 9) {
-    if (lane == 0 && j_hi > j_lo) {
-      // ------------------------------------------------------------------ products
+    if (j_hi > j_lo) {
+      // ------------------------------------------------------------------ products: the whole warp runs the loop and one
+      // elected lane issues, so that descriptors and addresses stay in uniform registers
       constexpr uint32_t idesc_s = umma_idesc_bf16(TT, TT, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(TT, HD, 0, 1);            // B = V is MN-major
+      const bool leader = elect_one();
+      const uint64_t dq0 = umma_smem_desc(sQ, 16, 1024), dk0 = umma_smem_desc(sK, 16, 1024);
+      const uint64_t dv0 = umma_smem_desc(sV, TT * 128, 1024);               // groups of 64 head dims
       auto issue_s = [&](int t, int s) {
-        const uint32_t qt = sQ + t * C::TILE, kb = sK + s * C::TILE;
+        const uint64_t da = dq0 + (uint32_t)(t * (C::TILE >> 4)), db = dk0 + (uint32_t)(s * (C::TILE >> 4));
+        if (leader) {
 #pragma unroll
-        for (int kc = 0; kc < KC; ++kc)
+          for (int kc = 0; kc < KC; ++kc)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16<1>(tmem + t * 128, umma_smem_desc(qt + kc * (TT * 128) + k * 32, 16, 1024),
-                        umma_smem_desc(kb + kc * (TT * 128) + k * 32, 16, 1024), idesc_s, (kc | k) ? 1u : 0u);
-        umma_commit(bar(S_FULL + t));
+            for (int k = 0; k < 4; ++k)
+              umma_f16<1>(tmem + t * 128, da + (kc * (TT * 128) + k * 32) / 16, db + (kc * (TT * 128) + k * 32) / 16, idesc_s, (kc | k) ? 1u : 0u);
+          umma_commit(bar(S_FULL + t));
+        }
       };
-      bool ok = mbar_wait(bar(Q_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
-      if (ok) ok = mbar_wait(bar(K_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      if (ok) ok = mbar_wait_warp(bar(K_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
       if (ok) {
         tc_fence_after();
         for (int t = 0; t < 2; ++t)
           if (j_lo >= lo[t] && j_lo < hi[t]) issue_s(t, 0);
-        umma_commit(bar(K_EMPTY));
+        if (leader) umma_commit(bar(K_EMPTY));
       }
       int done[2] = {0, 0};                            // key blocks of each tile whose P V has been issued
       for (int j = j_lo, n = 0; ok && j < j_hi; ++j, ++n) {
         const int s = n & 1, sn = s ^ 1;
-        ok = mbar_wait(bar(V_FULL + s), (n >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
-        if (!ok) break;
+        ok = mbar_wait_warp(bar(V_FULL + s), (n >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
         const bool more = j + 1 < j_hi;
-        bool k_ready = false;
+        if (ok && more) ok = mbar_wait_warp(bar(K_FULL + sn), ((n + 1) >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+        if (!ok) break;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (j >= lo[t] && j < hi[t]) {
-            ok = mbar_wait(bar(P_FULL + t), done[t] & 1, abort_smem, p.status, SITE_TMEM_FULL);
+            // the first half of the keys while the threads work on the second
+            ok = mbar_wait_warp(bar(P_HALF + t), done[t] & 1, abort_smem, p.status, SITE_TMEM_FULL);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t v_base = sV + s * C::TILE;
+            const uint64_t db = dv0 + (uint32_t)(s * (C::TILE >> 4));
+            const uint32_t first = done[t] ? 1u : 0u;
+            if (leader) {
 #pragma unroll
-            for (int k = 0; k < TT / 16; ++k)          // B = V: MN-major, groups of 64 head dims
-              umma_f16_ts(tmem + C::O_COL0 + t * 128, tmem + t * 128 + k * 8, umma_smem_desc(v_base + k * 2048, TT * 128, 1024),
-                          idesc_o, (done[t] | k) ? 1u : 0u);
-            umma_commit(bar(O_DONE + t));
+              for (int k = 0; k < TT / 32; ++k)
+                umma_f16_ts(tmem + C::O_COL0 + t * 128, tmem + t * 128 + k * 8, db + k * 128, idesc_o, k ? 1u : first);
+            }
+            __syncwarp();
+            ok = mbar_wait_warp(bar(P_FULL + t), done[t] & 1, abort_smem, p.status, SITE_TMEM_FULL);
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) {
+#pragma unroll
+              for (int k = TT / 32; k < TT / 16; ++k)
+                umma_f16_ts(tmem + C::O_COL0 + t * 128, tmem + t * 128 + k * 8, db + k * 128, idesc_o, 1u);
+              umma_commit(bar(O_DONE + t));
+            }
             ++done[t];
           }
-          if (t == 1) umma_commit(bar(V_EMPTY + s));
-          if (more && j + 1 >= lo[t] && j + 1 < hi[t]) {
-            if (!k_ready) {
-              ok = mbar_wait(bar(K_FULL + sn), ((n + 1) >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
-              if (!ok) break;
-              tc_fence_after();
-              k_ready = true;
-            }
-            issue_s(t, sn);
-          }
+          if (t == 1 && leader) umma_commit(bar(V_EMPTY + s));
+          if (more && j + 1 >= lo[t] && j + 1 < hi[t]) issue_s(t, sn);
         }
-        if (ok && more) umma_commit(bar(K_EMPTY + sn));
+        if (ok && more && leader) umma_commit(bar(K_EMPTY + sn));
+        __syncwarp();
       }
     }
   } else {
@@ -635,16 +665,17 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
       }
       const float neg_ms = (m_ref == -CUDART_INF_F) ? 0.f : -m_ref * p.scale_log2;
       if (DROP) dr.begin((uint32_t)(b * p.heads_total + p.head_off + h), (uint32_t)qpos);
-      float sums[2] = {0.f, 0.f};
+      const F2 scale2 = f2(p.scale_log2, p.scale_log2), off2 = f2(neg_ms, neg_ms);
+      F2 sum2[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0 = ex2_approx(fmaf(__uint_as_float(r[c][i]), p.scale_log2, neg_ms));
-          float p1 = ex2_approx(fmaf(__uint_as_float(r[c][i + 1]), p.scale_log2, neg_ms));
-          sums[0] += p0;                               // the row sum is that of the undropped probabilities
-          sums[1] += p1;
+          float x0, x1;
+          unpack(fma2(f2(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), scale2, off2), x0, x1);
+          float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
+          sum2[(i / 2) & 1] = add2(sum2[(i / 2) & 1], f2(p0, p1));      // the row sum is that of the undropped probabilities
           if (DROP) {
             const uint32_t kpos = (uint32_t)(p.k_off + (kbase + c * 32 + i) * p.k_stride);
             p0 = dr.keep(p.drop, kpos) ? p0 * p.drop.inv_keep : 0.f;
@@ -654,11 +685,15 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
           w[i / 2] = *reinterpret_cast<uint32_t*>(&hb);
         }
         tmem_st_32x16(s_addr + c * 16, w);             // every score of the row is in registers by now
+        if (c == 1 || c == 3) {
+          tmem_st_wait();
+          tc_fence_before();
+          mbar_arrive(bar((c == 1 ? P_HALF : P_FULL) + t));
+        }
       }
-      l = l * alpha + sums[0] + sums[1];
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(bar(P_FULL + t));
+      float s0, s1;
+      unpack(add2(sum2[0], sum2[1]), s0, s1);
+      l = l * alpha + s0 + s1;
     }
     // ---- epilogue: O / l -> bf16 rows, log-sum-exp
     if (ok && n_blocks > 0) {

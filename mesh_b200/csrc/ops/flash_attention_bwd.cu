@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(THREADS, 1) flash_bwd_kernel(const __grid_cons
 //     warps 0-7     P from S, dS from P and dP: a thread holds one key row and half of the query columns
 //     warps 8-11    add dQ of the block to the float accumulator while dK runs: 32 x 32 pieces through shared memory
 //                   and one reducing bulk copy each.  (Reductions straight from registers, red.global.add.v2 with four
-//                   lanes on a 32-byte sector, held the whole pipeline up: 942 us instead of 706 us at one sequence of
+//                   lanes on a 32-byte sector, held the whole pipeline up: 942 us instead of 706 us then, at one sequence of
 //                   8192, 16 heads of 128, causal.)
 //     warp 12       copies: K, V once; Q, L and Delta of the query blocks through two stages, dO through one (it is
 //                   free from dV of a block on and needed again three products later; the other 32 KB stage dQ)
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(THREADS, 1) flash_bwd_kernel(const __grid_cons
 //
 // Bound by the chain dP -> dS -> dQ -> drain -> dP' beside a tensor pipe that needs 2560 cycles per pair of blocks at
 // head size 128.  Measured at one sequence of 8192, 16 heads of 128, causal: 1967 us with the serial kernel above,
-// 706 us with this one (973 TFLOP/s); heads of 64: 494 us.  Dropout stays with the kernel above: there a thread holds
+// 694 us with this one (990 TFLOP/s); heads of 64: 477 us.  Dropout stays with the kernel above: there a thread holds
 // a query row and pays one generator call for four keys, here it would pay one for every score.
 constexpr int THREADS2 = 448;
 
@@ -500,74 +500,88 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_bwd2_kernel(const __grid_co
       }
     }
   } else if (warp == 13) {
-    if (lane == 0 && n_iter > 0) {
-      // ------------------------------------------------------------------ products
+    if (n_iter > 0) {
+      // ------------------------------------------------------------------ products: the whole warp runs the loop and one
+      // elected lane issues, so that descriptors and addresses stay in uniform registers
       constexpr uint32_t id_s = umma_idesc_bf16(128, 128, 0, 0);        // K Q^T and V dO^T: both K-major over head_dim
       constexpr uint32_t id_t = umma_idesc_bf16(128, HD, 0, 1);         // P^T dO and dS^T Q: A along the queries, B MN-major
       constexpr uint32_t id_q = umma_idesc_bf16(128, HD, 1, 1);         // dS K: A read across the keys
-      auto issue_nt = [&](uint32_t d, uint32_t a, uint32_t bm) {
+      const bool leader = elect_one();
+      // K-major and MN-major descriptors of the tiles; 16 deeper in k is 32 bytes in the one and 2 KiB in the other
+      const uint64_t kK = umma_smem_desc(sK, 16, 1024), kV = umma_smem_desc(sV, 16, 1024), kQ = umma_smem_desc(sQ, 16, 1024);
+      const uint64_t kdO = umma_smem_desc(sdO, 16, 1024), kdS = umma_smem_desc(sdS, 16, 1024);
+      const uint64_t mK = umma_smem_desc(sK, 128 * 128, 1024), mQ = umma_smem_desc(sQ, 128 * 128, 1024);
+      const uint64_t mdO = umma_smem_desc(sdO, 128 * 128, 1024), mdS = umma_smem_desc(sdS, 128 * 128, 1024);
+      auto issue_nt = [&](uint32_t d, uint64_t a, uint64_t bm) {
 #pragma unroll
         for (int kc = 0; kc < KC; ++kc)
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t off = kc * (128 * 128) + k * 32;
-            umma_f16<1>(d, umma_smem_desc(a + off, 16, 1024), umma_smem_desc(bm + off, 16, 1024), id_s, (kc | k) ? 1u : 0u);
-          }
+          for (int k = 0; k < 4; ++k)
+            umma_f16<1>(d, a + (kc * (128 * 128) + k * 32) / 16, bm + (kc * (128 * 128) + k * 32) / 16, id_s, (kc | k) ? 1u : 0u);
       };
-      bool ok = mbar_wait(bar(B_::KV_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
-      if (ok) ok = mbar_wait(bar(B_::Q_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      bool ok = mbar_wait_warp(bar(B_::KV_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+      if (ok) ok = mbar_wait_warp(bar(B_::Q_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
       if (ok) {
         tc_fence_after();
-        issue_nt(tmem + C_S, sK, sQ);
-        umma_commit(bar(B_::S_FULL));
-        ok = mbar_wait(bar(B_::DO_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
+        if (leader) {
+          issue_nt(tmem + C_S, kK, kQ);
+          umma_commit(bar(B_::S_FULL));
+        }
+        ok = mbar_wait_warp(bar(B_::DO_FULL), 0, abort_smem, p.status, SITE_SMEM_FULL);
       }
       if (ok) {
         tc_fence_after();
-        issue_nt(tmem + C_DP, sV, sdO);
-        umma_commit(bar(B_::DP_FULL));
+        if (leader) {
+          issue_nt(tmem + C_DP, kV, kdO);
+          umma_commit(bar(B_::DP_FULL));
+        }
       }
       for (int it = 0; ok && it < n_iter; ++it) {
         const int s = it & 1, sn = s ^ 1;
-        const uint32_t qt = sQ + s * TILE;
-        ok = mbar_wait(bar(B_::P_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+        const bool more = it + 1 < n_iter;
+        const uint32_t first = it ? 1u : 0u;
+        if (more) ok = mbar_wait_warp(bar(B_::Q_FULL + sn), ((it + 1) >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+        if (ok) ok = mbar_wait_warp(bar(B_::P_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k)                    // P^T: 64 queries in columns 0.., the others in columns 64..
-          umma_f16_ts(tmem + C_DV, tmem + C_S + (k < 4 ? k * 8 : 64 + (k - 4) * 8), umma_smem_desc(sdO + k * 2048, 128 * 128, 1024),
-                      id_t, (it | k) ? 1u : 0u);
-        umma_commit(bar(B_::DO_EMPTY));
-        if (it + 1 < n_iter) {
-          ok = mbar_wait(bar(B_::Q_FULL + sn), ((it + 1) >> 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
-          if (!ok) break;
-          tc_fence_after();
-          issue_nt(tmem + C_S, sK, sQ + sn * TILE);
-          umma_commit(bar(B_::S_FULL));
+          for (int k = 0; k < 8; ++k)                  // P^T: 64 queries in columns 0.., the others in columns 64..
+            umma_f16_ts(tmem + C_DV, tmem + C_S + (k < 4 ? k * 8 : 64 + (k - 4) * 8), mdO + k * 128, id_t, k ? 1u : first);
+          umma_commit(bar(B_::DO_EMPTY));
+          if (more) {
+            issue_nt(tmem + C_S, kK, kQ + (uint32_t)(sn * (TILE >> 4)));
+            umma_commit(bar(B_::S_FULL));
+          }
         }
-        ok = mbar_wait(bar(B_::DS_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
+        __syncwarp();
+        ok = mbar_wait_warp(bar(B_::DS_FULL), it & 1, abort_smem, p.status, SITE_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_f16<1>(tmem + C_DQ, umma_smem_desc(sdS + k * 2048, 128 * 128, 1024), umma_smem_desc(sK + k * 2048, 128 * 128, 1024),
-                      id_q, k ? 1u : 0u);
-        umma_commit(bar(B_::DQ_FULL));
+          for (int k = 0; k < 8; ++k) umma_f16<1>(tmem + C_DQ, mdS + k * 128, mK + k * 128, id_q, k ? 1u : 0u);
+          umma_commit(bar(B_::DQ_FULL));
+          const uint64_t q = mQ + (uint32_t)(s * (TILE >> 4));
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_f16<1>(tmem + C_DK, umma_smem_desc(sdS + (k / 4) * (128 * 128) + (k % 4) * 32, 16, 1024),
-                      umma_smem_desc(qt + k * 2048, 128 * 128, 1024), id_t, (it | k) ? 1u : 0u);
-        umma_commit(bar(B_::Q_EMPTY + s));
-        if (it + 1 < n_iter) {
-          ok = mbar_wait(bar(B_::DO_FULL), (it + 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
-          if (ok) ok = mbar_wait(bar(B_::DQ_READ), it & 1, abort_smem, p.status, SITE_TMEM_EMPTY);
+          for (int k = 0; k < 8; ++k)
+            umma_f16<1>(tmem + C_DK, kdS + ((k / 4) * (128 * 128) + (k % 4) * 32) / 16, q + k * 128, id_t, k ? 1u : first);
+          umma_commit(bar(B_::Q_EMPTY + s));
+        }
+        __syncwarp();
+        if (more) {
+          ok = mbar_wait_warp(bar(B_::DO_FULL), (it + 1) & 1, abort_smem, p.status, SITE_SMEM_FULL);
+          if (ok) ok = mbar_wait_warp(bar(B_::DQ_READ), it & 1, abort_smem, p.status, SITE_TMEM_EMPTY);
           if (!ok) break;
           tc_fence_after();
-          issue_nt(tmem + C_DP, sV, sdO);
-          umma_commit(bar(B_::DP_FULL));               // also: dK and dQ of this block are done with dS
+          if (leader) {
+            issue_nt(tmem + C_DP, kV, kdO);
+            umma_commit(bar(B_::DP_FULL));             // also: dK and dQ of this block are done with dS
+          }
+          __syncwarp();
         }
       }
-      if (ok) umma_commit(bar(B_::ACC_DONE));
+      if (ok && leader) umma_commit(bar(B_::ACC_DONE));
     }
   } else if (warp >= 8) {
     // -------------------------------------------------------------------- dQ into the float accumulator
