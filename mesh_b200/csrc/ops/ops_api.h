@@ -13,6 +13,9 @@ int mesh_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y
 // kernel.  `blocks` rows of scratch are used (<= 1024).
 int mesh_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw,
                      float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream);
+// The same with dw in bf16, rounded once from the fp32 sums.
+int mesh_rmsnorm_bwd_bf16(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw,
+                          float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream);
 int mesh_rmsnorm_bwd_blocks(int rows);
 
 // Rotate-half rotary embedding, in place, on x[tokens, heads, head_dim] (row stride `ld` elements

@@ -198,7 +198,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // over all rows was a chain of up to 592 loads: 24 us for 512 partials of 2048 columns; now 3).
 constexpr int DW_COLS = 32, DW_ROWS = 32;
 __global__ void __launch_bounds__(DW_COLS * DW_ROWS)
-rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int blocks, int cols) {
+rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, __nv_bfloat16* __restrict__ dw16, int blocks,
+                         int cols) {
   __shared__ float sh[DW_ROWS][DW_COLS + 1];
   const int x = threadIdx.x % DW_COLS, y = threadIdx.x / DW_COLS;
   const int c = blockIdx.x * DW_COLS + x;
@@ -210,7 +211,10 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
   sh[y][x] = s;
   __syncthreads();
   s = warp_sum(sh[x][y]);                    // warp y sums column y
-  if (x == 0 && blockIdx.x * DW_COLS + y < cols) dw[blockIdx.x * DW_COLS + y] = s;
+  if (x == 0 && blockIdx.x * DW_COLS + y < cols) {
+    if (dw) dw[blockIdx.x * DW_COLS + y] = s;
+    else dw16[blockIdx.x * DW_COLS + y] = __float2bfloat16_rn(s);
+  }
 }
 
 }  // namespace
@@ -244,8 +248,8 @@ extern "C" int mesh_rmsnorm_fwd(const void* x, const void* residual, const void*
 
 extern "C" int mesh_rmsnorm_bwd_blocks(int rows) { return rows < 592 ? rows : 592; }
 
-extern "C" int mesh_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw,
-                                float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream) {
+static int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw, __nv_bfloat16* dw16,
+                       float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream) {
   if (rows <= 0) return 0;
   if (cols % 8 || cols > NORM_THREADS * MAX_VEC_PER_THREAD * 8)
     return set_error(-2, "rmsnorm: cols must be a multiple of 8 and <= %d", NORM_THREADS * MAX_VEC_PER_THREAD * 8);
@@ -261,9 +265,19 @@ extern "C" int mesh_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
   else BWD(8);
 #undef BWD
   MESH_CUDA_OK(cudaGetLastError());
-  if (dw && dw_partial) {
-    rmsnorm_dw_reduce_kernel<<<(cols + DW_COLS - 1) / DW_COLS, DW_COLS * DW_ROWS, 0, (cudaStream_t)stream>>>(dw_partial, dw, blocks, cols);
+  if ((dw || dw16) && dw_partial) {
+    rmsnorm_dw_reduce_kernel<<<(cols + DW_COLS - 1) / DW_COLS, DW_COLS * DW_ROWS, 0, (cudaStream_t)stream>>>(dw_partial, dw, dw16, blocks, cols);
     MESH_CUDA_OK(cudaGetLastError());
   }
   return 0;
+}
+
+extern "C" int mesh_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw,
+                                float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream) {
+  return rmsnorm_bwd(dy, x, w, rstd, dx, dw, nullptr, dw_partial, blocks, rows, cols, w_offset, stream);
+}
+
+extern "C" int mesh_rmsnorm_bwd_bf16(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw,
+                                     float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream) {
+  return rmsnorm_bwd(dy, x, w, rstd, dx, nullptr, (__nv_bfloat16*)dw, dw_partial, blocks, rows, cols, w_offset, stream);
 }

@@ -63,7 +63,7 @@ def _op_code(op) -> int:
 
 
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_native.stream())
 
 
 class Communicator:

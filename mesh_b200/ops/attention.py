@@ -69,7 +69,7 @@ def flash_attention(q, k, v, *, causal=True, window=0, scale=None, q_off=0, q_st
     a.scale = scale
     a.status = status_block(q.device).data_ptr()
     _set_dropout(a, dropout)
-    rc = _native.lib().mesh_flash_attention_fwd(ctypes.byref(a), c_void_p(torch.cuda.current_stream().cuda_stream))
+    rc = _native.lib().mesh_flash_attention_fwd(ctypes.byref(a), c_void_p(_native.stream()))
     _native.check(rc, "mesh_flash_attention_fwd")
     _native.count_launch()
     return (out, lse) if need_lse else out
@@ -165,7 +165,7 @@ def _delta(dout, out, clear=None):
     rc = _native.lib().mesh_attention_delta(c_void_p(dout.data_ptr()), c_longlong(dout.stride(1)), c_void_p(out.data_ptr()),
                                             c_longlong(out.stride(1)), c_void_p(delta.data_ptr()),
                                             c_void_p(0 if clear is None else clear.data_ptr()), c_int(B), c_int(T), c_int(H),
-                                            c_int(hd), c_void_p(torch.cuda.current_stream().cuda_stream))
+                                            c_int(hd), c_void_p(_native.stream()))
     _native.check(rc, "mesh_attention_delta")
     _native.count_launch()
     return delta
@@ -216,7 +216,7 @@ def flash_attention_backward(q, k, v, out, lse, dout, *, causal=True, window=0, 
         assert dkv_acc.dtype == torch.float32 and dkv_acc.is_contiguous()
         dk, dv = dkv_acc[0], dkv_acc[1]
         a.dk_acc, a.dv_acc, a.ld_dkv = dk.data_ptr(), dv.data_ptr(), dk.stride(1)
-    rc = _native.lib().mesh_flash_attention_bwd(ctypes.byref(a), c_void_p(torch.cuda.current_stream().cuda_stream))
+    rc = _native.lib().mesh_flash_attention_bwd(ctypes.byref(a), c_void_p(_native.stream()))
     _native.check(rc, "mesh_flash_attention_bwd")
     _native.count_launch()
     return dq, dk, dv

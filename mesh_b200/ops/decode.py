@@ -220,7 +220,7 @@ def dequantize_w8(codes: torch.Tensor, scales: torch.Tensor) -> torch.Tensor:
 
 
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_native.stream())
 
 
 def _p(t) -> int:

@@ -27,7 +27,7 @@ def _check2d(t: torch.Tensor, name: str) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _native.stream()
 
 
 _trace: list | None = None
@@ -156,11 +156,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     """
     g, M, N, K = _base_args(a, b, a_mn, b_mn)
     if out is None:
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    _check2d(out, "out")
+        out = a.new_empty((M, N))
+    else:
+        _check2d(out, "out")
     g.D, g.ldd, g.d_cols = out.data_ptr(), out.stride(0), out.shape[1]
-    g.epi = EPI_STORE
-    g.num_ctas, g.tile_n, g.pair = num_ctas, tile_n, pair
+    g.num_ctas, g.tile_n, g.pair = num_ctas, tile_n, pair      # epi: EPI_STORE is 0
     if flow:
         chain(g, **flow)
     _launch(g)
@@ -278,18 +278,20 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
         ctx.save_for_backward(x, w)
-        x2 = x.reshape(-1, x.shape[-1])
-        y = gemm(x2, w)
-        return y.reshape(*x.shape[:-1], w.shape[0])
+        if x.dim() == 2:                                            # views cost host time that short calls are bound by
+            return gemm(x, w)
+        return gemm(x.reshape(-1, x.shape[-1]), w).reshape(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
-        x2 = x.reshape(-1, x.shape[-1])
+        flat = x.dim() == 2
+        dy2 = (dy if flat else dy.reshape(-1, dy.shape[-1])).contiguous()
+        x2 = x if flat else x.reshape(-1, x.shape[-1])
         dx = dw = None
         if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, w, b_mn=True).reshape(x.shape)          # [M,N] x [N,K] stored [K=N, cols=K]
+            dx = gemm(dy2, w, b_mn=True)                            # [M,N] x [N,K] stored [K=N, cols=K]
+            dx = dx if flat else dx.reshape(x.shape)
         if ctx.needs_input_grad[1]:
             dw = gemm(dy2, x2, a_mn=True, b_mn=True)               # dy^T x : [N, K]
         return dx, dw

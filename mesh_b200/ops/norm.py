@@ -15,7 +15,7 @@ from .. import _native
 
 
 def _s() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_native.stream())
 
 
 def _p(t) -> c_void_p:
@@ -31,7 +31,7 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, residual: t
     rows = x.numel() // cols
     y = torch.empty_like(x) if out is None else out
     res_out = torch.empty_like(x) if residual is not None else None
-    rstd = torch.empty(rows, dtype=torch.float32, device=x.device) if need_rstd else None
+    rstd = x.new_empty(rows, dtype=torch.float32) if need_rstd else None
     L = _native.lib()
     rc = L.mesh_rmsnorm_fwd(_p(x), _p(residual), _p(w), _p(y), _p(res_out), _p(rstd), c_int(rows), c_int(cols),
                             c_float(eps), c_float(weight_offset), _s())
@@ -40,16 +40,19 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, residual: t
     return y, res_out, rstd
 
 
-def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor, weight_offset: float = 0.0):
+def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor, weight_offset: float = 0.0,
+                dw_dtype: torch.dtype = torch.float32):
+    """``dw_dtype``: fp32, or bf16 (rounded once from the fp32 sums)."""
     cols = x.shape[-1]
     rows = x.numel() // cols
     L = _native.lib()
     blocks = L.mesh_rmsnorm_bwd_blocks(c_int(rows))
     dx = torch.empty_like(x)
-    dw = torch.empty(cols, dtype=torch.float32, device=x.device)
-    partial = torch.empty((blocks, cols), dtype=torch.float32, device=x.device)
-    rc = L.mesh_rmsnorm_bwd(_p(dy.contiguous()), _p(x), _p(w), _p(rstd), _p(dx), _p(dw), _p(partial), c_int(blocks),
-                            c_int(rows), c_int(cols), c_float(weight_offset), _s())
+    dw = x.new_empty(cols, dtype=dw_dtype)
+    partial = x.new_empty((blocks, cols), dtype=torch.float32)
+    fn = L.mesh_rmsnorm_bwd_bf16 if dw_dtype == torch.bfloat16 else L.mesh_rmsnorm_bwd
+    rc = fn(_p(dy.contiguous()), _p(x), _p(w), _p(rstd), _p(dx), _p(dw), _p(partial), c_int(blocks),
+            c_int(rows), c_int(cols), c_float(weight_offset), _s())
     _native.check(rc, "mesh_rmsnorm_bwd")
     _native.count_launch(2)
     return dx, dw
@@ -67,6 +70,9 @@ class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
+        if w.dtype == torch.bfloat16:
+            dx, dw = rmsnorm_bwd(dy, x, w, rstd, ctx.weight_offset, torch.bfloat16)
+            return dx, dw, None, None
         dx, dw = rmsnorm_bwd(dy, x, w, rstd, ctx.weight_offset)
         return dx, dw.to(w.dtype), None, None
 

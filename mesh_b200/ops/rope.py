@@ -28,7 +28,7 @@ def rope_(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torc
     rc = _native.lib().mesh_rope(c_void_p(x.data_ptr()), c_void_p(positions.data_ptr()), c_void_p(cos.data_ptr()),
                                  c_void_p(sin.data_ptr()), c_int(tokens), c_int(heads), c_int(hd),
                                  c_longlong(x.stride(0)), c_int(int(inverse)),
-                                 c_void_p(torch.cuda.current_stream().cuda_stream))
+                                 c_void_p(_native.stream()))
     _native.check(rc, "mesh_rope")
     _native.count_launch(1)
     return x

@@ -21,7 +21,7 @@ def router_topk(logits: torch.Tensor, k: int, bias: torch.Tensor | None = None, 
     rc = _native.lib().mesh_router_topk(c_void_p(logits.data_ptr()), c_int(int(logits.dtype == torch.float32)),
                                         c_void_p(0 if bias is None else bias.data_ptr()), c_void_p(w.data_ptr()),
                                         c_void_p(idx.data_ptr()), c_int(T), c_int(E), c_int(k), c_int(int(renorm)),
-                                        c_void_p(torch.cuda.current_stream().cuda_stream))
+                                        c_void_p(_native.stream()))
     _native.check(rc, "mesh_router_topk")
     _native.count_launch(1)
     return w, idx

@@ -47,7 +47,7 @@ class _Combine(ctypes.Structure):
 
 
 def _s():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_native.stream())
 
 
 class EPMoE:

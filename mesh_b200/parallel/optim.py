@@ -40,7 +40,7 @@ class ShardedAdamW:
                                                c_void_p(out_bf16.data_ptr() if out_bf16 is not None else 0),
                                                c_longlong(st["master"].numel()), c_float(self.lr), c_float(b1), c_float(b2),
                                                c_float(self.eps), c_float(self.wd), c_int(self_step), c_float(1.0),
-                                               c_void_p(torch.cuda.current_stream().cuda_stream))
+                                               c_void_p(_native.stream()))
             _native.check(rc, "mesh_adamw_step")
             _native.count_launch()
             return

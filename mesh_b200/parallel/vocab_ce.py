@@ -27,7 +27,8 @@ def _all_reduce(x: torch.Tensor, group, op: str) -> None:
 
 def _s():
     from ctypes import c_void_p
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    from .. import _native
+    return c_void_p(_native.stream())
 
 
 class _VocabParallelCEKernel(torch.autograd.Function):
