@@ -19,6 +19,7 @@
 // (rdma/mesh_compile.py:1571-1579): counts are exchanged, blocks travel at their own sizes, never padded to the largest.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <math_constants.h>
 #include "moe_api.h"
 #include "../device/check.cuh"
 #include "../device/ptx.cuh"
@@ -103,11 +104,16 @@ moe_count_kernel(const int* __restrict__ idx, int n_entries, int* __restrict__ s
   __threadfence();
   if ((int)threadIdx.x < experts) {
     int run = 0;
-    for (int c = 0; c < chunks; ++c) {
-      int* h = hist + (long long)c * experts + threadIdx.x;
-      const int n = __ldcg(h);
-      *h = run;
-      run += n;
+    int* h = hist + threadIdx.x;
+    for (int c0 = 0; c0 < chunks; c0 += 8) {                                 // eight loads in flight, not one
+      int n[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) n[u] = c0 + u < chunks ? __ldcg(h + (long long)(c0 + u) * experts) : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (c0 + u < chunks) h[(long long)(c0 + u) * experts] = run;
+        run += n[u];
+      }
     }
     if (world > 0) {
       uint2* peers[8] = {c0, c1, c2, c3, c4, c5, c6, c7};
@@ -137,6 +143,10 @@ struct PlanArgs {
   Status* status;
 };
 
+// Every CTA works out the same layout (a few microseconds of a 60 us kernel when one CTA wrote all tables, some fifteen
+// thousand 32-byte records at 64 experts); the first one stores it, and the experts' records are shared out.
+constexpr int PLAN_CTAS = 16;
+
 __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
   __shared__ int C[R][MAX_E];
   __shared__ int n_loc[MAX_E], base_loc[MAX_E], pad_loc[MAX_E];
@@ -150,8 +160,9 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
     C[i / E][i % E] = (int)v;
   }
   __syncthreads();
+  const bool first = blockIdx.x == 0;
   if (!ok_s) {
-    if (threadIdx.x < 6) a.n_tiles[threadIdx.x] = 0;
+    if (first && threadIdx.x < 6) a.n_tiles[threadIdx.x] = 0;
     return;
   }
   // every destination's layout is the same function of the matrix; this rank needs all of them as a sender
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
     }
     int before = 0;
     for (int s = 0; s < a.rank; ++s) before += C[s][e];
-    a.send_base[e] = base + before;
+    if (first) a.send_base[e] = base + before;
     if (d == a.rank) {
       int n = 0;
       for (int s = 0; s < P; ++s) n += C[s][e];
@@ -185,15 +196,19 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
         pad_loc[el] = min(pad_loc[el], room);
         n_loc[el] = min(n_loc[el], pad_loc[el]);
       }
-      a.layout[el] = n_loc[el];
-      a.layout[El + el] = base_loc[el];
-      a.layout[2 * El + el] = pad_loc[el];
       total = max(total, base_loc[el] + pad_loc[el]);
     }
-    a.layout[3 * El] = total;
-    a.layout[3 * El + 1] = dropped;
+    if (first) {
+      a.layout[3 * El] = total;
+      a.layout[3 * El + 1] = dropped;
+    }
   }
   __syncthreads();
+  if (first && (int)threadIdx.x < El) {
+    a.layout[threadIdx.x] = n_loc[threadIdx.x];
+    a.layout[El + threadIdx.x] = base_loc[threadIdx.x];
+    a.layout[2 * El + threadIdx.x] = pad_loc[threadIdx.x];
+  }
   // ---- tile tables (pair tiles: 256 output rows each).  Table t of expert el holds cnt[t][el] descriptors starting at
   // off[t][el]; thread 0 lays the offsets out (6 x local experts additions), then every warp writes the descriptors of
   // its experts, a lane per tile: the tables are thousands of 32-byte records, far too many for one thread.
@@ -210,12 +225,12 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
       n += t < 4 ? (rows / 256) * ntn[t] : (rows >= 64 ? dw_mt[t - 4] * ntn[t] : 0);
     }
     off[t][El] = n;
-    a.n_tiles[t] = min(n, a.max_tiles);
+    if (first) a.n_tiles[t] = min(n, a.max_tiles);
   }
   __syncthreads();
   MeshTileDesc* const tab[6] = {a.t_glu, a.t_down, a.t_dh, a.t_dx, a.t_dw2, a.t_dw1};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  for (int el = warp; el < El; el += nwarps) {
+  for (int el = blockIdx.x + gridDim.x * warp; el < El; el += gridDim.x * nwarps) {
     const int base = base_loc[el], kb = pad_loc[el] / 64;
 #pragma unroll
     for (int t = 0; t < 6; ++t) {
@@ -263,34 +278,54 @@ struct DispatchArgs {
 
 __global__ void __launch_bounds__(256) moe_dispatch_kernel(const DispatchArgs a) {
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_entries = a.tokens * a.k;
   const int vec = a.d_model / 8;
-  for (int i = blockIdx.x * warps + warp; i < n_entries; i += gridDim.x * warps) {
-    const int e = a.idx[i];
-    if (!MESH_CHECK_INDEX(e, a.local_experts * a.world, a.status)) continue;      // an expert id from the router
-    const int dest = e / a.local_experts;
-    const int row = a.send_base[e] + a.slot[i];
-    if (!MESH_CHECK_INDEX(row, 1ll << 30, a.status)) continue;                    // negative: a broken plan
-    if (row >= a.cap_rows) {
-      if (lane == 0) a.meta[i] = -1;
-      continue;
-    }
-    if (lane == 0) a.meta[i] = row;
-    const uint4* src = reinterpret_cast<const uint4*>(a.x + (long long)(i / a.k) * a.d_model);
-    uint4* dst = reinterpret_cast<uint4*>(a.recv[dest] + (long long)row * a.d_model);
-    if (a.scale == nullptr) {
-      for (int v = lane; v < vec; v += 32) dst[v] = __ldg(src + v);
-    } else {
-      const float s = a.scale[i];
-      for (int v = lane; v < vec; v += 32) {
-        uint4 q = __ldg(src + v);
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float2 f = __bfloat1622float2(h[c]);
-          h[c] = __floats2bfloat162_rn(f.x * s, f.y * s);
+  // A warp owns a token: its row is read once and stored to the k rows that were assigned to it (a warp per stored row
+  // read it k times): 8192 tokens of 2048, six choices, 49 us now, 61 before.
+  for (int t = blockIdx.x * warps + warp; t < a.tokens; t += gridDim.x * warps) {
+    const uint4* src = reinterpret_cast<const uint4*>(a.x + (long long)t * a.d_model);
+    for (int j0 = 0; j0 < a.k; j0 += 32) {
+      // lane j: where choice j0 + j of this token goes
+      unsigned long long dst = 0;
+      float s = 1.f;
+      const int i = t * a.k + j0 + lane;
+      if (j0 + lane < a.k) {
+        const int e = a.idx[i];
+        if (MESH_CHECK_INDEX(e, a.local_experts * a.world, a.status)) {           // an expert id from the router
+          const int row = a.send_base[e] + a.slot[i];
+          if (MESH_CHECK_INDEX(row, 1ll << 30, a.status)) {                       // negative: a broken plan
+            const bool fits = row < a.cap_rows;
+            a.meta[i] = fits ? row : -1;
+            if (fits) dst = reinterpret_cast<unsigned long long>(a.recv[e / a.local_experts] + (long long)row * a.d_model);
+          }
         }
-        dst[v] = q;
+        if (a.scale) s = a.scale[i];
+      }
+      const int n = min(32, a.k - j0);
+      for (int base = 0; base < vec; base += 4 * 32) {
+        const int v0 = base + lane;
+        uint4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (v0 + u * 32 < vec) q[u] = __ldg(src + v0 + u * 32);
+        for (int j = 0; j < n; ++j) {
+          uint4* d = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, dst, j));
+          const float sj = __shfl_sync(0xffffffffu, s, j);
+          if (d == nullptr) continue;                                             // the same for the whole warp
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (v0 + u * 32 >= vec) break;
+            uint4 o = q[u];
+            if (a.scale) {
+              __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const float2 f = __bfloat1622float2(h[c]);
+                h[c] = __floats2bfloat162_rn(f.x * sj, f.y * sj);
+              }
+            }
+            d[v0 + u * 32] = o;
+          }
+        }
       }
     }
   }
@@ -315,10 +350,15 @@ struct CombineArgs {
   const uint32_t* ready; uint32_t ready_expect;               // this rank's counter: all peers finished their experts
   __nv_bfloat16* out;                          // [tokens, d_model]
   const __nv_bfloat16* dot_with; float* dots;  // optional: dots[t, j] = <row, dot_with[t]>
+  const __nv_bfloat16* addend;                 // optional [tokens, d_model]: added to the sum before it is rounded
   Status* status;
 };
 
-__global__ void __launch_bounds__(256) moe_combine_kernel(const CombineArgs a) {
+// J rows of a token are read together (one after the other, each behind its index loads, the pass ran at 3 TB/s).  J and the
+// kind of result are template parameters because the rows in flight live in registers: 8192 tokens of 2048 with six rows
+// each take 55 us (sum) and 52 us (dots), 73 and 99 before.
+template <int J, bool DOTS>
+__global__ void __launch_bounds__(256, 3) moe_combine_kernel(const CombineArgs a) {
   __shared__ int ok_s;
   if (threadIdx.x == 0) ok_s = wait_flag_ge(a.ready, a.ready_expect, a.status, SITE_PEER_FLAG) ? 1 : 0;
   __syncthreads();
@@ -326,53 +366,169 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const CombineArgs a) {
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int vec = a.d_model / 8;       // 16-byte vectors per row; a lane owns vectors lane, lane+32, ...
   for (int t = blockIdx.x * warps + warp; t < a.tokens; t += gridDim.x * warps) {
-    for (int v = lane; v < vec; v += 32) {
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int j = 0; j < a.k; ++j) {
-        const int row = a.meta[t * a.k + j];
-        if (row < 0) continue;
-        const int dest = a.idx[t * a.k + j] / a.local_experts;
-        if (!MESH_CHECK_INDEX(dest, a.world, a.status) || !MESH_CHECK_INDEX(row, a.cap_rows, a.status)) continue;
-        const float w = a.weight ? a.weight[t * a.k + j] : 1.f;
-        const uint4 q = __ldcg(reinterpret_cast<const uint4*>(a.src[dest] + (long long)row * a.d_model) + v);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float2 f = __bfloat1622float2(h[c]);
-          acc[2 * c] += w * f.x;
-          acc[2 * c + 1] += w * f.y;
-        }
+    // lane j: the row of choice j (k <= 32), null when it was dropped
+    unsigned long long mine = 0;
+    float mw = 1.f;
+    if (lane < a.k) {
+      const int i = t * a.k + lane, row = a.meta[i];
+      if (row >= 0) {
+        const int dest = a.idx[i] / a.local_experts;
+        if (MESH_CHECK_INDEX(dest, a.world, a.status) && MESH_CHECK_INDEX(row, a.cap_rows, a.status))
+          mine = reinterpret_cast<unsigned long long>(a.src[dest] + (long long)row * a.d_model);
       }
-      if (a.out) {
+      if (a.weight) mw = a.weight[i];
+    }
+    const uint4* src[J];
+    float w[J];
+    auto pick = [&](int j0) {
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const unsigned long long p = __shfl_sync(0xffffffffu, mine, (j0 + j) & 31);
+        w[j] = __shfl_sync(0xffffffffu, mw, (j0 + j) & 31);
+        src[j] = j0 + j < a.k ? reinterpret_cast<const uint4*>(p) : nullptr;
+      }
+    };
+    pick(0);
+    if constexpr (!DOTS) {
+      for (int base = 0; base < vec; base += 32) {
+        const int v = base + lane;
+        const bool in = v < vec;
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint4 extra = make_uint4(0, 0, 0, 0);
+        if (a.addend && in) extra = __ldg(reinterpret_cast<const uint4*>(a.addend + (long long)t * a.d_model) + v);
+        for (int j0 = 0; j0 < a.k; j0 += J) {
+          if (a.k > J) pick(j0);
+          uint4 q[J];
+#pragma unroll
+          for (int j = 0; j < J; ++j)
+            if (src[j] != nullptr && in) q[j] = __ldcg(src[j] + v);
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            if (src[j] == nullptr || !in) continue;
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q[j]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float2 f = __bfloat1622float2(h[c]);
+              acc[2 * c] += w[j] * f.x;
+              acc[2 * c + 1] += w[j] * f.y;
+            }
+          }
+        }
+        if (!in) continue;
+        const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&extra);
         uint4 o;
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) h[c] = __floats2bfloat162_rn(acc[2 * c], acc[2 * c + 1]);
+        for (int c = 0; c < 4; ++c) {
+          const float2 f = __bfloat1622float2(e[c]);
+          h[c] = __floats2bfloat162_rn(acc[2 * c] + f.x, acc[2 * c + 1] + f.y);
+        }
         reinterpret_cast<uint4*>(a.out + (long long)t * a.d_model)[v] = o;
       }
     }
-    if (a.dots) {
-      for (int j = 0; j < a.k; ++j) {
-        const int row = a.meta[t * a.k + j];
-        float d = 0.f;
-        if (row >= 0) {
-          const int dest = a.idx[t * a.k + j] / a.local_experts;
-          for (int v = lane; v < vec; v += 32) {
-            const uint4 q = __ldcg(reinterpret_cast<const uint4*>(a.src[dest] + (long long)row * a.d_model) + v);
-            const uint4 g = __ldg(reinterpret_cast<const uint4*>(a.dot_with + (long long)t * a.d_model) + v);
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-            const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g);
+    if constexpr (DOTS) {
+      for (int j0 = 0; j0 < a.k; j0 += J) {
+        if (a.k > J) pick(j0);
+        float dot[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) dot[j] = 0.f;
+        for (int v = lane; v < vec; v += 32) {
+          const uint4 g = __ldg(reinterpret_cast<const uint4*>(a.dot_with + (long long)t * a.d_model) + v);
+          uint4 q[J];
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            q[j] = make_uint4(0, 0, 0, 0);
+            if (src[j] != nullptr) q[j] = __ldcg(src[j] + v);
+          }
+          const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g);
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q[j]);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              float2 f = __bfloat1622float2(h[c]), gg = __bfloat1622float2(gh[c]);
-              d += f.x * gg.x + f.y * gg.y;
+              const float2 f = __bfloat1622float2(h[c]), gg = __bfloat1622float2(gh[c]);
+              dot[j] += f.x * gg.x + f.y * gg.y;
             }
           }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (lane == 0) a.dots[t * a.k + j] = d;
+        for (int j = 0; j < J; ++j) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+          if (lane == j && j0 + j < a.k) a.dots[t * a.k + j0 + j] = src[j] != nullptr ? dot[j] : 0.f;
+        }
       }
+    }
+  }
+}
+
+// Weight gradients of the experts that got no rows: their tables hold no tiles, so nothing else writes them.
+__global__ void __launch_bounds__(256) moe_zero_unused_kernel(uint4* __restrict__ dw1, long long vec1, uint4* __restrict__ dw2,
+                                                              long long vec2, const int* __restrict__ layout, int local_experts,
+                                                              const int* __restrict__ n_tiles) {
+  const int el = blockIdx.y;
+  if (layout[2 * local_experts + el] >= 64 && n_tiles[4] > 0) return;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < vec1; i += gridDim.x * 256ll) dw1[el * vec1 + i] = make_uint4(0, 0, 0, 0);
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < vec2; i += gridDim.x * 256ll) dw2[el * vec2 + i] = make_uint4(0, 0, 0, 0);
+}
+
+// Gradient of the routing weights w = top-k of softmax(logits + bias), renormalised over the k, through to the logits; a warp
+// per token.  dots[t, j]: gradient of w_j (0 counts for a dropped choice).  With p the softmax and S the sum of the chosen
+// p, d p_j = (g_j - sum_i w_i g_i) / S on the chosen experts and 0 elsewhere; sum_e p_e d p_e vanishes, so the softmax's
+// backward is d logits = p d p.
+__global__ void __launch_bounds__(256) moe_router_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ bias,
+                                                             const int* __restrict__ idx, const int* __restrict__ meta,
+                                                             const float* __restrict__ dots, __nv_bfloat16* __restrict__ dlogits,
+                                                             int tokens, int experts, int k) {
+  constexpr int PER = MAX_E / 32;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int t = blockIdx.x * warps + warp; t < tokens; t += gridDim.x * warps) {
+    float v[PER];
+    float mx = -CUDART_INF_F;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int e = lane + 32 * i;
+      v[i] = e < experts ? __bfloat162float(logits[(long long)t * experts + e]) + (bias ? bias[e] : 0.f) : -CUDART_INF_F;
+      mx = fmaxf(mx, v[i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      v[i] = lane + 32 * i < experts ? expf(v[i] - mx) : 0.f;
+      sum += v[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    // lane j: the j-th choice
+    const int i = t * k + lane;
+    const int e = lane < k ? idx[i] : 0;
+    const float g = lane < k && meta[i] >= 0 ? dots[i] : 0.f;
+    float pe = 0.f;
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+      const float got = __shfl_sync(0xffffffffu, v[r], e & 31);
+      if ((e >> 5) == r) pe = got;
+    }
+    pe = lane < k ? pe / sum : 0.f;
+    float S = pe, wg = pe * g;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      S += __shfl_xor_sync(0xffffffffu, S, o);
+      wg += __shfl_xor_sync(0xffffffffu, wg, o);
+    }
+    const float d = pe * (g - wg / S) / S;
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+      const int at = lane + 32 * r;
+      float out = 0.f;
+      for (int j = 0; j < k; ++j) {
+        const int ej = __shfl_sync(0xffffffffu, e, j);
+        const float dj = __shfl_sync(0xffffffffu, d, j);
+        if (ej == at) out = dj;
+      }
+      if (at < experts) dlogits[(long long)t * experts + at] = __float2bfloat16_rn(out);
     }
   }
 }
@@ -409,7 +565,7 @@ extern "C" int mesh_moe_plan(const MeshMoePlan* m, void* stream) {
   a.t_glu = (MeshTileDesc*)m->tables[0]; a.t_down = (MeshTileDesc*)m->tables[1]; a.t_dh = (MeshTileDesc*)m->tables[2];
   a.t_dx = (MeshTileDesc*)m->tables[3]; a.t_dw2 = (MeshTileDesc*)m->tables[4]; a.t_dw1 = (MeshTileDesc*)m->tables[5];
   a.n_tiles = m->n_tiles; a.max_tiles = m->max_tiles; a.status = (Status*)m->status;
-  moe_plan_kernel<<<1, 512, 0, (cudaStream_t)stream>>>(a);
+  moe_plan_kernel<<<PLAN_CTAS, 512, 0, (cudaStream_t)stream>>>(a);
   MESH_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -443,6 +599,7 @@ extern "C" int mesh_moe_signal(int world, void* const* ready_ptrs, void* stream)
 }
 
 extern "C" int mesh_moe_combine(const MeshMoeCombine* m, void* stream) {
+  if (m->k > 32) return set_error(-2, "moe_combine: at most 32 choices per token");
   CombineArgs a;
   a.tokens = m->tokens; a.k = m->k; a.d_model = m->d_model; a.local_experts = m->local_experts; a.world = m->world;
   a.idx = m->idx; a.meta = m->meta; a.weight = m->weight;
@@ -451,9 +608,41 @@ extern "C" int mesh_moe_combine(const MeshMoeCombine* m, void* stream) {
   a.out = (__nv_bfloat16*)m->out; a.dot_with = (const __nv_bfloat16*)m->dot_with; a.dots = m->dots;
   a.status = (Status*)m->status;
   a.cap_rows = m->cap_rows > 0 ? m->cap_rows : (1 << 30);
+  a.addend = (const __nv_bfloat16*)m->addend;
   int grid = (m->tokens + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
-  moe_combine_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+#define MESH_COMBINE(DOTS)                                                                          \
+  do {                                                                                              \
+    if (a.k <= 2) moe_combine_kernel<2, DOTS><<<grid, 256, 0, (cudaStream_t)stream>>>(a);           \
+    else if (a.k <= 4) moe_combine_kernel<4, DOTS><<<grid, 256, 0, (cudaStream_t)stream>>>(a);      \
+    else if (a.k <= 6) moe_combine_kernel<6, DOTS><<<grid, 256, 0, (cudaStream_t)stream>>>(a);      \
+    else moe_combine_kernel<8, DOTS><<<grid, 256, 0, (cudaStream_t)stream>>>(a);                    \
+  } while (0)
+  if (a.out) MESH_COMBINE(false);
+  if (a.dots) MESH_COMBINE(true);
+#undef MESH_COMBINE
+  MESH_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+extern "C" int mesh_moe_zero_unused(void* dw1, long long elems1, void* dw2, long long elems2, const int* layout, int local_experts,
+                                    const int* n_tiles, void* stream) {
+  if (elems1 % 8 || elems2 % 8) return set_error(-2, "moe_zero_unused: expert matrices must be multiples of 8 elements");
+  dim3 grid(16, local_experts);
+  moe_zero_unused_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((uint4*)dw1, elems1 / 8, (uint4*)dw2, elems2 / 8, layout, local_experts,
+                                                                n_tiles);
+  MESH_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+extern "C" int mesh_moe_router_bwd(const void* logits, const float* bias, const int* idx, const int* meta, const float* dots,
+                                   void* dlogits, int tokens, int experts, int k, void* stream) {
+  if (experts > MAX_E || k < 1 || k > 32) return set_error(-2, "moe_router_bwd: experts <= %d, k <= 32", MAX_E);
+  int grid = (tokens + 7) / 8;
+  if (grid > 148 * 8) grid = 148 * 8;
+  if (grid < 1) return 0;
+  moe_router_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, bias, idx, meta, dots,
+                                                               (__nv_bfloat16*)dlogits, tokens, experts, k);
   MESH_CUDA_OK(cudaGetLastError());
   return 0;
 }

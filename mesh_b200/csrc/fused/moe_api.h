@@ -49,8 +49,17 @@ typedef struct MeshMoeCombine {
   void* out; const void* dot_with; float* dots;
   void* status;
   int cap_rows;                 // rows of every source buffer (bounds of the rows named by `meta`)
+  const void* addend;           // optional bf16 [tokens, d_model], added to `out` before it is rounded
 } MeshMoeCombine;
 int mesh_moe_combine(const MeshMoeCombine* m, void* stream);
+
+// Clears the weight gradients (elems1 / elems2 bf16 elements per expert) of the local experts that got no rows.
+int mesh_moe_zero_unused(void* dw1, long long elems1, void* dw2, long long elems2, const int* layout, int local_experts,
+                         const int* n_tiles, void* stream);
+// d logits (bf16 [tokens, experts]) from the gradients `dots` [tokens, k] of the renormalised top-k routing weights; choices
+// with a negative `meta` were dropped and count nothing.
+int mesh_moe_router_bwd(const void* logits, const float* bias, const int* idx, const int* meta, const float* dots, void* dlogits,
+                        int tokens, int experts, int k, void* stream);
 
 #ifdef __cplusplus
 }

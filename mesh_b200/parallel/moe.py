@@ -8,12 +8,12 @@ matmuls are descriptor-driven tcgen05 launches over compact per-expert row regio
 
 Forward:  router GEMM -> top-k -> count/slot -> plan -> dispatch(x) -> GLU GEMM -> down GEMM -> ready -> combine.
 Backward: dispatch(w*dOut) + dots(<y, dOut>) -> dH GEMM (GLU backward epilogue) -> dW2 -> dX GEMM -> dW1 ->
-          ready -> combine(dX) ; router gradient through softmax/top-k in PyTorch on the [tokens, experts] logits.
+          ready -> combine(dX + the router's part) ; router gradient through top-k and softmax in one kernel.
 """
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_int, c_uint32, c_void_p
+from ctypes import c_int, c_longlong, c_uint32, c_void_p
 
 import torch
 
@@ -43,7 +43,7 @@ class _Combine(ctypes.Structure):
     _fields_ = [("tokens", c_int), ("k", c_int), ("d_model", c_int), ("local_experts", c_int), ("world", c_int),
                 ("idx", c_void_p), ("meta", c_void_p), ("weight", c_void_p), ("src", c_void_p * MAX_RANKS),
                 ("ready", c_void_p), ("ready_expect", c_uint32), ("out", c_void_p), ("dot_with", c_void_p),
-                ("dots", c_void_p), ("status", c_void_p), ("cap_rows", c_int)]
+                ("dots", c_void_p), ("status", c_void_p), ("cap_rows", c_int), ("addend", c_void_p)]
 
 
 def _s():
@@ -130,23 +130,26 @@ class EPMoE:
         _native.count_launch()
 
     def _signal(self, sig_index):
+        if self.world == 1:                   # nobody else reads these rows, and the stream orders this rank's kernels
+            return
         arr = (c_void_p * MAX_RANKS)(*[c_void_p(self.sig.ptr(r) + 4 * sig_index) if r < self.world else c_void_p(0) for r in range(MAX_RANKS)])
         _native.check(self.L.mesh_moe_signal(c_int(self.world), arr, _s()), "mesh_moe_signal")
         _native.count_launch()
 
-    def _combine(self, src, sig_index, weight, out, dot_with=None, dots=None):
+    def _combine(self, src, sig_index, weight, out, dot_with=None, dots=None, addend=None):
         c = _Combine()
         c.tokens, c.k, c.d_model, c.local_experts, c.world = self.T, self.k, self.D, self.El, self.world
         c.idx, c.meta = self.idx.data_ptr(), self.meta.data_ptr()
         c.weight = 0 if weight is None else weight.data_ptr()
         for r in range(self.world):
             c.src[r] = src.ptr(r)
-        c.ready, c.ready_expect = self.sig.ptr() + 4 * sig_index, self.world * self.steps
+        c.ready, c.ready_expect = self.sig.ptr() + 4 * sig_index, self.world * self.steps if self.world > 1 else 0
         c.out = 0 if out is None else out.data_ptr()
         c.dot_with = 0 if dot_with is None else dot_with.data_ptr()
         c.dots = 0 if dots is None else dots.data_ptr()
         c.status = status_block(self.dev).data_ptr()
         c.cap_rows = self.cap
+        c.addend = 0 if addend is None else addend.data_ptr()
         _native.check(self.L.mesh_moe_combine(ctypes.byref(c), _s()), "mesh_moe_combine")
         _native.count_launch()
 
@@ -228,13 +231,13 @@ class EPMoE:
             self._combine(self.y, 2, None, None, dot_with=dout, dots=dots.view(-1))
             self._mark("bwd weight dots")
             # router: weights = renormalised top-k of softmax(logits + bias)
-            lg = logits.float().detach().requires_grad_(True)
-            p = torch.softmax(lg + (bias.float() if bias is not None else 0.0), dim=-1)
-            sel = torch.gather(p, 1, self.idx.view(T, k).long())
-            wn = sel / sel.sum(-1, keepdim=True)
-            kept = (self.meta.view(T, k) >= 0).float()
-            (wn * dots * kept).sum().backward()
-            dlogits = lg.grad.to(torch.bfloat16)
+            dlogits = torch.empty_like(logits)
+            b32 = None if bias is None else bias.float().contiguous()
+            _native.check(self.L.mesh_moe_router_bwd(c_void_p(logits.data_ptr()), c_void_p(0 if b32 is None else b32.data_ptr()),
+                                                     c_void_p(self.idx.data_ptr()), c_void_p(self.meta.data_ptr()),
+                                                     c_void_p(dots.data_ptr()), c_void_p(dlogits.data_ptr()), c_int(T), c_int(self.E),
+                                                     c_int(k), _s()), "mesh_moe_router_bwd")
+            _native.count_launch()
             dxr = G.gemm(dlogits, w_router, b_mn=True)
             dwr = G.gemm(dlogits, x, a_mn=True, b_mn=True) if (dlogits.shape[1] % 64 == 0 and x.shape[1] % 64 == 0) else \
                 (dlogits.float().T @ x.float()).to(torch.bfloat16)
@@ -256,23 +259,25 @@ class EPMoE:
         self._grouped(2, rdy, w2, self.dgu, M=self.cap, N=F, K=D, b_mn=True, epi=G.EPI_GLU_BWD, aux=self.gu, d_up_cols=F,
                       a_ready=self.sig.ptr() + 4, a_ready_value=expect, d_cols=2 * F)
         self._mark("bwd dH glu")
-        dw2 = torch.zeros_like(w2)
+        dw1, dw2 = torch.empty_like(w1), torch.empty_like(w2)
+        _native.check(self.L.mesh_moe_zero_unused(c_void_p(dw1.data_ptr()), c_longlong(2 * F * D), c_void_p(dw2.data_ptr()),
+                                                  c_longlong(F * D), c_void_p(self.layout.data_ptr()), c_int(self.El),
+                                                  c_void_p(self.n_tiles.data_ptr()), _s()), "mesh_moe_zero_unused")
+        _native.count_launch()
         self._grouped(4, rdy, self.h, dw2, M=D, N=F, K=self.cap, a_mn=True, b_mn=True)
         self._mark("bwd dW2")
         self._grouped(3, self.dgu, w1, self.dx.local, M=self.cap, N=D, K=2 * F, b_mn=True)
         self._mark("bwd dX")
-        dw1 = torch.zeros_like(w1)
         self._grouped(5, self.dgu, rx, dw1, M=2 * F, N=D, K=self.cap, a_mn=True, b_mn=True)
         self._mark("bwd dW1")
         self._signal(3)
-        dx = torch.empty((T, D), dtype=torch.bfloat16, device=self.dev)
-        self._combine(self.dx, 3, None, dx)
-        self._mark("bwd combine")
         if overlap:
             main.wait_stream(side)
             for t in (dx_router, dw_router, dots):
                 t.record_stream(main)
-        dx = dx + dx_router
+        dx = torch.empty((T, D), dtype=torch.bfloat16, device=self.dev)
+        self._combine(self.dx, 3, None, dx, addend=dx_router)
+        self._mark("bwd combine")
         return dx, dw_router, dw1, dw2
 
 

@@ -66,3 +66,42 @@ def test_moe_expert_parallel(world):
         pytest.skip(f"needs {world} GPUs")
     from mesh_b200.utils.launch import spawn_ranks
     spawn_ranks(_run, world, 256, 256, 128, 8 * world // 2 if world > 2 else 8, 2, 2, use_cuda=True, timeout=300.0)
+
+
+@pytest.mark.parametrize("T,D,F,E,k,spread", [(64, 256, 128, 8, 8, 0.0), (192, 512, 256, 16, 12, 6.0), (320, 256, 384, 64, 1, 4.0)])
+def test_moe_unused_experts_and_many_choices(T, D, F, E, k, spread):
+    """More choices than are read together, experts that no token chose (their weight gradients are zero, in memory that
+    held something else), and the router's gradient, against the dense statement's autograd."""
+    import torch.distributed as dist
+    from mesh_b200.config import MeshConfig, set_config
+    from mesh_b200.distributed.context import MeshContext
+    from mesh_b200.parallel.moe import EPMoE, moe_reference
+    from mesh_b200.runtime.rendezvous import Rendezvous
+    from mesh_b200.utils.status import check_status
+    dev = torch.device("cuda", 0)
+    set_config(MeshConfig.from_env(heap_bytes=512 << 20))
+    ctx = MeshContext(0, 1, dev, Rendezvous(dist.HashStore(), 0, 1), None)
+    g = torch.Generator(device=dev).manual_seed(5)
+    rand = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=dev) * std).bfloat16()
+    x, dy, wr, w1, w2 = rand(T, D), rand(T, D), rand(E, D, std=0.02), rand(E, 2 * F, D, std=0.05), rand(E, D, F, std=0.05)
+    bias = torch.linspace(spread, -spread, E, device=dev)                # the last experts are chosen by nobody
+    moe = EPMoE(ctx, T, D, F, E, k, capacity_factor=2.0)
+    torch.full((E * 3 * F * D * 2,), float("nan"), dtype=torch.bfloat16, device=dev)       # what freed memory may hold
+    out = moe.forward(x, wr, w1.view(-1, D), w2.view(-1, F), bias)
+    dx, dwr, dw1, dw2 = moe.backward(dy)
+    check_status()
+    X, W1, W2, WR = (t.float().requires_grad_(True) for t in (x, w1, w2, wr))
+    want = moe_reference(X, WR, W1, W2, k, bias)
+    # the statement routes on rounded logits, whose rounding autograd passes straight through
+    gx, g1, g2, gr = torch.autograd.grad((want * dy.float()).sum(), (X, W1, W2, WR), allow_unused=True)
+    unused = (moe.layout[:E] == 0)
+    if spread:
+        assert bool(unused.any())
+    assert float(dw1.view(E, 2 * F, D)[unused].abs().sum()) == 0 and float(dw2.view(E, D, F)[unused].abs().sum()) == 0
+    for got, ref in ((out, want), (dx, gx), (dw1.view_as(g1), g1), (dw2.view_as(g2), g2)):
+        _close(got.float(), ref.detach(), 4e-2)
+    if k > 1:
+        _close(dwr, gr, 4e-2)
+    else:                                             # one renormalised weight is the constant 1
+        assert float(dwr.abs().max()) < 1e-4
+    ctx.heap.close()
