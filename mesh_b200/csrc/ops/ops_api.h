@@ -24,6 +24,14 @@ int mesh_rmsnorm_bwd_blocks(int rows);
 int mesh_rope(void* x, const int* positions, const float* cos_t, const float* sin_t, int tokens, int heads,
               int head_dim, long long ld, int inverse, void* stream);
 
+// A fused projection src [tokens, (q_heads + 2 kv_heads) * head_dim] (row stride ld) copied to the dense dst with its query
+// and key heads rotated; and the gradient: the query columns of dqkv (dense) from the fp32 dq [tokens, q_heads * head_dim], its
+// key columns rotated back in place, its value columns left as they are.
+int mesh_rope_qkv(const void* src, long long ld, void* dst, const int* positions, const float* cos_t, const float* sin_t,
+                  int tokens, int q_heads, int kv_heads, int head_dim, void* stream);
+int mesh_rope_qkv_bwd(const float* dq, void* dqkv, const int* positions, const float* cos_t, const float* sin_t, int tokens,
+                      int q_heads, int kv_heads, int head_dim, void* stream);
+
 // out[0] = sum(a[i] * b[i]) for bf16 a, b of n elements (fp32 accumulation, one launch, result independent of block
 // timing).  Scratch: `partials` fp32[mesh_dot_sum_blocks()] and a zero-initialised `ticket` word, left at zero; calls
 // that share scratch must be ordered on one stream.

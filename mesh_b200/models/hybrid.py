@@ -147,6 +147,12 @@ class Attention(nn.Module):
             xg = all_gather_seq(x, tp) if tp.world > 1 else x
             qkv = _linear(xg, self.w_qkv)
         Tc = qkv.shape[0] // B
+        if _fast(x) and cp.world == 1 and self.hd in (64, 128, 256) and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0:
+            from ..ops.attention import rotary_attention
+            cos, sin = self._tables(x.device)
+            o = rotary_attention(qkv, pos.to(torch.int32).repeat(B), cos, sin, batch=B, q_heads=self.Hq, kv_heads=self.Hkv,
+                                 head_dim=self.hd)
+            return self._project(o, fused, B * Tc)
         qkv = qkv.view(B, Tc, self.Hq + 2 * self.Hkv, self.hd)
         q, k, v = qkv[:, :, : self.Hq], qkv[:, :, self.Hq: self.Hq + self.Hkv], qkv[:, :, self.Hq + self.Hkv:]
         if _fast(x):
@@ -173,10 +179,14 @@ class Attention(nn.Module):
             s = torch.einsum("bthd,bshd->bhts", q, kf) * self.hd ** -0.5
             s = s.masked_fill((kpos[None, :] > pos[:, None])[None, None], float("-inf"))
             o = torch.einsum("bhts,bshd->bthd", torch.softmax(s.float(), -1).to(q.dtype), vf)
+        return self._project(o, fused, B * Tc)
+
+    def _project(self, o, fused, rows: int):
+        tp = self.par.tp
         if fused is not None:
             from ..parallel.fused_linear import row_linear
-            return row_linear(o.reshape(B * Tc, self.Hq * self.hd), self.w_o, fused[1])   # GEMM -> reduce-scatter
-        y = _linear(o.reshape(B * Tc, self.Hq * self.hd), self.w_o)
+            return row_linear(o.reshape(rows, self.Hq * self.hd), self.w_o, fused[1])     # GEMM -> reduce-scatter
+        y = _linear(o.reshape(rows, self.Hq * self.hd), self.w_o)
         return reduce_scatter_seq(y, tp) if tp.world > 1 else y
 
 

@@ -172,8 +172,9 @@ def _delta(dout, out, clear=None):
 
 
 def flash_attention_backward(q, k, v, out, lse, dout, *, causal=True, window=0, scale=None, q_off=0, q_stride=1,
-                             k_off=0, k_stride=1, delta=None, dq=None, dkv_acc=None, dropout=None):
-    """Gradients of :func:`flash_attention`.  Returns ``(dq fp32 [B,Tq,H,hd], dk, dv)``.
+                             k_off=0, k_stride=1, delta=None, dq=None, dkv_acc=None, dropout=None, dkv_out=None):
+    """Gradients of :func:`flash_attention`.  Returns ``(dq fp32 [B,Tq,H,hd], dk, dv)``.  ``dkv_out``: two bf16
+    ``[B, Tk, Hkv, hd]`` (dense heads and one row stride for both, e.g. columns of a fused gradient) that take dk and dv.
 
     ``dq`` (fp32) is added to when given.  With ``dkv_acc`` (fp32 ``[2, B, Tk, Hkv, hd]``) the key/value gradients
     are added to it and ``dk, dv`` are returned as its two halves; otherwise they are fresh bf16 tensors.
@@ -190,6 +191,10 @@ def flash_attention_backward(q, k, v, out, lse, dout, *, causal=True, window=0, 
     if dq is None:
         dq = torch.zeros((B, Tq, H, hd), dtype=torch.float32, device=q.device)
     if hd not in (64, 128):
+        if dkv_out is not None:
+            dq, dk, dv = _backward_by_blocks(q, k, v, lse, dout, delta, dq, None, causal, window, scale, q_off, q_stride, k_off,
+                                             k_stride, dropout)
+            return dq, dkv_out[0].copy_(dk), dkv_out[1].copy_(dv)
         # the backward kernel keeps dK and dV of a key block in tensor memory, which holds them up to 128 columns wide
         return _backward_by_blocks(q, k, v, lse, dout, delta, dq, dkv_acc, causal, window, scale, q_off, q_stride, k_off,
                                    k_stride, dropout)
@@ -209,8 +214,12 @@ def flash_attention_backward(q, k, v, out, lse, dout, *, causal=True, window=0, 
     a.delta = delta.data_ptr()
     a.dq, a.ld_dq = dq.data_ptr(), dq.stride(1)
     if dkv_acc is None:
-        dk = torch.empty((B, Tk, Hkv, hd), dtype=torch.bfloat16, device=q.device)
-        dv = torch.empty_like(dk)
+        if dkv_out is not None:
+            dk, dv = dkv_out
+            assert dk.dtype == dv.dtype == torch.bfloat16 and dk.stride() == dv.stride() and _view2d(dk) and _view2d(dv)
+        else:
+            dk = torch.empty((B, Tk, Hkv, hd), dtype=torch.bfloat16, device=q.device)
+            dv = torch.empty_like(dk)
         a.dk, a.dv, a.ld_dkv = dk.data_ptr(), dv.data_ptr(), dk.stride(1)
     else:
         assert dkv_acc.dtype == torch.float32 and dkv_acc.is_contiguous()
@@ -280,6 +289,60 @@ def attention(q, k, v, *, causal=True, window=0, scale=None, dropout=None):
     """Differentiable attention on the flash kernels (``q [B, T, H, hd]``, ``k, v [B, T, Hkv, hd]``, bf16).
     ``dropout``: ``dict(p=..., seed=..., site=0, execution=0)``; the backward pass redraws the same mask."""
     return _Attention.apply(q, k, v, causal, window, scale, dropout)
+
+
+class _RotaryAttention(torch.autograd.Function):
+    """Self-attention of a fused projection with rotary positions.  Queries, keys and values stay columns of one matrix
+    in both directions: one kernel rotates on the way in, the attention kernels read and write columns, one kernel rotates
+    the gradients back (taken apart, the three cost copies, a clone per rotation, and a cleared full-size gradient and an
+    addition per slice)."""
+
+    @staticmethod
+    def forward(ctx, qkv, positions, cos, sin, B, Hq, Hkv, hd, causal, window):
+        n = qkv.shape[0]
+        rot = torch.empty((n, (Hq + 2 * Hkv) * hd), dtype=torch.bfloat16, device=qkv.device)
+        rc = _native.lib().mesh_rope_qkv(c_void_p(qkv.data_ptr()), c_longlong(qkv.stride(0)), c_void_p(rot.data_ptr()),
+                                         c_void_p(positions.data_ptr()), c_void_p(cos.data_ptr()), c_void_p(sin.data_ptr()),
+                                         c_int(n), c_int(Hq), c_int(Hkv), c_int(hd), c_void_p(_native.stream()))
+        _native.check(rc, "mesh_rope_qkv")
+        _native.count_launch()
+        q, k, v = _RotaryAttention.parts(rot, B, Hq, Hkv, hd)
+        out, lse = flash_attention(q, k, v, causal=causal, window=window, need_lse=True)
+        ctx.save_for_backward(rot, out, lse, positions, cos, sin)
+        ctx.cfg = (B, Hq, Hkv, hd, causal, window)
+        return out
+
+    @staticmethod
+    def parts(m, B, Hq, Hkv, hd):
+        m = m.view(B, -1, Hq + 2 * Hkv, hd)
+        return m[:, :, :Hq], m[:, :, Hq:Hq + Hkv], m[:, :, Hq + Hkv:]
+
+    @staticmethod
+    def backward(ctx, dout):
+        rot, out, lse, positions, cos, sin = ctx.saved_tensors
+        B, Hq, Hkv, hd, causal, window = ctx.cfg
+        q, k, v = _RotaryAttention.parts(rot, B, Hq, Hkv, hd)
+        d = torch.empty_like(rot)
+        _, dk, dv = _RotaryAttention.parts(d, B, Hq, Hkv, hd)
+        dq, _, _ = flash_attention_backward(q, k, v, out, lse, dout, causal=causal, window=window, dkv_out=(dk, dv))
+        rc = _native.lib().mesh_rope_qkv_bwd(c_void_p(dq.data_ptr()), c_void_p(d.data_ptr()), c_void_p(positions.data_ptr()),
+                                             c_void_p(cos.data_ptr()), c_void_p(sin.data_ptr()), c_int(rot.shape[0]), c_int(Hq),
+                                             c_int(Hkv), c_int(hd), c_void_p(_native.stream()))
+        _native.check(rc, "mesh_rope_qkv_bwd")
+        _native.count_launch()
+        return d, None, None, None, None, None, None, None, None, None
+
+
+def rotary_attention(qkv, positions, cos, sin, *, batch, q_heads, kv_heads, head_dim, causal=True, window=0):
+    """``qkv [batch * T, (q_heads + 2 kv_heads) * head_dim]`` (a fused projection, bf16, head_dim 64, 128 or 256) ->
+    ``[batch, T, q_heads, head_dim]``: query and key heads rotated by ``positions`` (int32, one per row) through the
+    tables of :func:`mesh_b200.ops.rope.rope_tables`, then attention.  Differentiable in ``qkv``."""
+    n, width = qkv.shape
+    if qkv.dtype != torch.bfloat16 or not qkv.is_cuda or width != (q_heads + 2 * kv_heads) * head_dim or n % batch or qkv.stride(1) != 1:
+        raise ValueError("rotary_attention: expected bf16 CUDA rows of q, k and v heads, whole samples")
+    if positions.dtype != torch.int32 or positions.numel() != n or not positions.is_contiguous():
+        raise ValueError("rotary_attention: one int32 position per row")
+    return _RotaryAttention.apply(qkv, positions, cos, sin, batch, q_heads, kv_heads, head_dim, causal, window)
 
 
 def _ring_positions(r, src, P, T, striped):

@@ -284,3 +284,31 @@ def test_flash_tiles(hd, B, Tq, Tk, H, Hkv, causal, window, off, stride):
     seen = ~blind
     torch.testing.assert_close(lse[:, :, seen].double(), torch.logsumexp(s, -1)[:, :, seen].detach(), atol=1e-4, rtol=1e-4)
     assert bool(torch.isinf(lse[:, :, blind]).all())
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,hd,window", [(2, 200, 4, 2, 64, 0), (1, 257, 2, 2, 128, 100), (3, 64, 4, 1, 256, 0)])
+def test_rotary_attention_of_a_fused_projection(B, T, Hq, Hkv, hd, window):
+    """Against the separate rotation and attention with the same kernels' oracles; the projection may be a column slice."""
+    from mesh_b200.ops.attention import attention_ref, rotary_attention
+    from mesh_b200.ops.rope import rope_tables
+    from mesh_b200.utils.status import check_status
+    g = torch.Generator(device="cuda").manual_seed(B * T)
+    W = (Hq + 2 * Hkv) * hd
+    wide = torch.randn(B * T, W + 64, device="cuda", generator=g).bfloat16()
+    qkv = wide[:, 32:32 + W].requires_grad_(True)
+    do = torch.randn(B, T, Hq, hd, device="cuda", generator=g).bfloat16()
+    cos, sin = rope_tables(2 * T, hd, 1e4)
+    pos = (torch.arange(B * T, device="cuda", dtype=torch.int32) % T) * 2
+    out = rotary_attention(qkv, pos, cos, sin, batch=B, q_heads=Hq, kv_heads=Hkv, head_dim=hd, window=window)
+    (d,) = torch.autograd.grad(out, qkv, do)
+    check_status()
+    x = qkv.detach().float().requires_grad_(True)
+    m = x.view(B * T, Hq + 2 * Hkv, hd)
+    c, s = cos[pos.long()][:, None], sin[pos.long()][:, None]
+    lo, hi = m[:, :Hq + Hkv, :hd // 2], m[:, :Hq + Hkv, hd // 2:]
+    r = torch.cat([lo * c - hi * s, hi * c + lo * s], -1).view(B, T, Hq + Hkv, hd)
+    ref, _ = attention_ref(r[:, :, :Hq], r[:, :, Hq:], m[:, Hq + Hkv:].view(B, T, Hkv, hd), True, window)
+    (dref,) = torch.autograd.grad(ref, x, do.float())
+    # rotated heads, probabilities, score gradients and results are rounded to bf16: 2^-9 each on average, four of them
+    assert float((out.float() - ref).norm() / ref.norm()) < 8e-3
+    assert float((d.float() - dref).norm() / dref.norm()) < 8e-3
