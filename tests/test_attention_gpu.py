@@ -312,3 +312,23 @@ def test_rotary_attention_of_a_fused_projection(B, T, Hq, Hkv, hd, window):
     # rotated heads, probabilities, score gradients and results are rounded to bf16: 2^-9 each on average, four of them
     assert float((out.float() - ref).norm() / ref.norm()) < 8e-3
     assert float((d.float() - dref).norm() / dref.norm()) < 8e-3
+
+
+@pytest.mark.parametrize("p", [0.0, 0.1])
+@pytest.mark.parametrize("T", [100, 256, 300, 640, 901])
+def test_flash_heads_of_256_alternate_between_groups(T, p):
+    """One to eight key blocks, with and without the (slow) dropout draws in between, several times: the groups of warps
+    meet in every order."""
+    from mesh_b200.ops.attention import attention_ref, flash_attention
+    from mesh_b200.utils.status import check_status
+    B, H, Hkv, hd = 2, 4, 2, 256
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v = (torch.randn(B, T, n, hd, device="cuda", generator=g).bfloat16() for n in (H, Hkv, Hkv))
+    kw = dict(causal=True, window=0 if T < 600 else 300, dropout=dict(p=p, seed=7) if p else None)
+    ref, lse_ref = attention_ref(q, k, v, **kw)
+    for _ in range(4):
+        out, lse = flash_attention(q, k, v, need_lse=True, **kw)
+        # probabilities and results are rounded to bf16
+        assert float((out.float() - ref).norm() / ref.norm()) < 6e-3
+        torch.testing.assert_close(lse, lse_ref, atol=1e-4, rtol=1e-4)
+    check_status()
