@@ -25,6 +25,7 @@ decode_argmax_kernel(const float* __restrict__ logits, long long ldl, int vocab_
                      uint2* const* __restrict__ xchg_unused, uint2* x0, uint2* x1, uint2* x2, uint2* x3, uint2* x4,
                      uint2* x5, uint2* x6, uint2* x7, uint32_t* step, Status* st) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  cluster_arrive_relaxed();             // waited for before the store into the first CTA's shared memory
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int b = blockIdx.x / AM_CTAS, part = blockIdx.x % AM_CTAS;
   const uint32_t seq = (step ? *step : 0u) + 1u;
@@ -60,6 +61,7 @@ decode_argmax_kernel(const float* __restrict__ logits, long long ldl, int vocab_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { sv[warp] = best; si[warp] = bi; }
   __syncthreads();
+  cluster_wait();
   if (warp == 0) {
     best = sv[lane];
     bi = si[lane];
