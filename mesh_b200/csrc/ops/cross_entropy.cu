@@ -42,19 +42,35 @@ __device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
-// Eight values at a time: one comparison with the running maximum, and the exponentials relative to it in one fma and one
-// ex2 each (value by value, with a branch and two exponentials in it, the pass ran at 2.8 TB/s).
+// 2^((f - m) log2(e)), two at a time.  The maximum is subtracted before the scaling: near it the difference is exact, while
+// -m log2(e) as the addend of an fma is rounded in proportion to m (1e-5 of a probability at logits of 1000) and is infinite
+// for a mask of bf16's lowest value.
+__device__ __forceinline__ void exp_off(float f0, float f1, float m, float& e0, float& e1) {
+  unsigned long long v, o;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(f0), "f"(f1));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(o) : "f"(-m));
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(o));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(o) : "f"(LOG2E));
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(o));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(e0), "=f"(e1) : "l"(v));
+  e0 = ex2_approx(e0);
+  e1 = ex2_approx(e1);
+}
+// Eight values at a time: one comparison with the running maximum, and the exponentials relative to it in one ex2 each
+// (value by value, with a branch and two exponentials in it, the pass ran at 2.8 TB/s).
 __device__ __forceinline__ void online8(float& m, float& s, const uint4& q) {
   float f[8];
   unpack8(q, f);
   const float mx = fmaxf(fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])), fmaxf(fmaxf(f[4], f[5]), fmaxf(f[6], f[7])));
   if (mx > m) { s *= __expf(m - mx); m = mx; }
-  const float off = (m == -CUDART_INF_F) ? 0.f : -m * LOG2E;
+  const float ref = (m == -CUDART_INF_F) ? 0.f : m;
   float a = 0.f, b = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; i += 2) {
-    a += ex2_approx(fmaf(f[i], LOG2E, off));
-    b += ex2_approx(fmaf(f[i + 1], LOG2E, off));
+    float e0, e1;
+    exp_off(f[i], f[i + 1], ref, e0, e1);
+    a += e0;
+    b += e1;
   }
   s += a + b;
 }
@@ -107,7 +123,7 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int rows
       const long long t = targets[r], local = t - vocab_start;
       const float tl = (t != ignore_index && local >= 0 && local < cols) ? __bfloat162float(x[local]) : 0.f;
       target_logit[r] = tl;
-      if (loss) loss[r] = t != ignore_index ? logf(S) + M - tl : 0.f;
+      if (loss) loss[r] = t != ignore_index ? logf(S) + (M - tl) : 0.f;
     }
     __syncthreads();
   }
@@ -148,14 +164,17 @@ ce_reduce_kernel(const float* __restrict__ loss, const long long* __restrict__ t
   }
 }
 
-__device__ __forceinline__ uint4 grad8(const uint4& q, float off, float inv) {
+__device__ __forceinline__ uint4 grad8(const uint4& q, float m, float inv) {
   float f[8];
   unpack8(q, f);
   uint4 o;
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    h[i] = __floats2bfloat162_rn(ex2_approx(fmaf(f[2 * i], LOG2E, off)) * inv, ex2_approx(fmaf(f[2 * i + 1], LOG2E, off)) * inv);
+  for (int i = 0; i < 4; ++i) {
+    float e0, e1;
+    exp_off(f[2 * i], f[2 * i + 1], m, e0, e1);
+    h[i] = __floats2bfloat162_rn(e0 * inv, e1 * inv);
+  }
   return o;
 }
 
@@ -174,7 +193,7 @@ ce_grad_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, __nv_bflo
     float g = gscale[(long long)r * g_stride];
     if (divisor) g /= divisor[0];
     if (t == ignore_index) g = 0.f;
-    const float off = -gmax[r] * LOG2E, inv = g / gsum[r];
+    const float mx = gmax[r], inv = g / gsum[r];
     const bool mine = local >= 0 && local < cols;
     // d may be the logits themselves: the target's logit is read before its element is written
     const float tx = (threadIdx.x == 0 && mine) ? __bfloat162float(x[local]) : 0.f;
@@ -190,14 +209,14 @@ ce_grad_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, __nv_bflo
 #pragma unroll
       for (int u = 0; u < 4; ++u) q[u] = xv[v + u * CE_THREADS];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) __stcs(ov + v + u * CE_THREADS, grad8(q[u], off, inv));
+      for (int u = 0; u < 4; ++u) __stcs(ov + v + u * CE_THREADS, grad8(q[u], mx, inv));
     }
-    for (; v < nv; v += CE_THREADS) ov[v] = grad8(xv[v], off, inv);
-    for (int c = threadIdx.x; c < head; c += CE_THREADS) o[c] = __float2bfloat16_rn(ex2_approx(fmaf(__bfloat162float(x[c]), LOG2E, off)) * inv);
+    for (; v < nv; v += CE_THREADS) ov[v] = grad8(xv[v], mx, inv);
+    for (int c = threadIdx.x; c < head; c += CE_THREADS) o[c] = __float2bfloat16_rn(__expf(__bfloat162float(x[c]) - mx) * inv);
     for (int c = head + nv * 8 + threadIdx.x; c < cols; c += CE_THREADS)
-      o[c] = __float2bfloat16_rn(ex2_approx(fmaf(__bfloat162float(x[c]), LOG2E, off)) * inv);
+      o[c] = __float2bfloat16_rn(__expf(__bfloat162float(x[c]) - mx) * inv);
     __syncthreads();
-    if (threadIdx.x == 0 && mine) o[local] = __float2bfloat16_rn(ex2_approx(fmaf(tx, LOG2E, off)) * inv - g);
+    if (threadIdx.x == 0 && mine) o[local] = __float2bfloat16_rn(__expf(tx - mx) * inv - g);
   }
 }
 

@@ -113,3 +113,52 @@ def test_cross_entropy_rows_of_any_alignment(n, v, ld, reduction):
     torch.testing.assert_close(loss.double(), want.detach(), rtol=1e-5, atol=1e-5)
     # p - 1 cancels in the target's column: its error is fp32's of p (1e-6 of the upstream value)
     assert bool(((d.double() - dw).abs() <= 2 ** -8 * dw.abs() + 2e-6 * float(up.max())).all())
+
+
+@pytest.mark.parametrize("v", [4096, 4099])
+@pytest.mark.parametrize("off", [0.0, 100.0, -1000.0, 60000.0])
+def test_cross_entropy_of_logits_far_from_zero(off, v):
+    """The loss depends on the differences of the logits alone.  fp32: exponents below 20 are within 2^-20, the logarithm of a
+    sum within as much; gradients are rounded to bf16, and in the target's column p - 1 cancels."""
+    from mesh_b200.parallel.vocab_ce import vocab_parallel_cross_entropy
+    g = torch.Generator(device="cuda").manual_seed(v)
+    n = 33
+    logits = (torch.randn(n, v, device="cuda", generator=g) * 4 + off).bfloat16().requires_grad_(True)
+    t = torch.randint(0, v, (n,), device="cuda", generator=g)
+    t[0] = logits[0].argmax()
+    loss = vocab_parallel_cross_entropy(logits, t, 0, None, reduction="none")
+    (d,) = torch.autograd.grad(loss.sum(), logits)
+    ref = logits.detach().double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(ref, t, reduction="none")
+    (dw,) = torch.autograd.grad(want.sum(), ref)
+    # the largest difference of two logits here is 512 (a bf16 step at 60000 is 256): the loss is rounded at that size
+    spread = float((ref.amax(-1) - ref.amin(-1)).max().detach())
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=2 ** -22, atol=2 ** -23 * max(20.0, spread))
+    assert bool(((d.double() - dw).abs() <= 2 ** -8 * dw.abs() + 2e-6).all())
+
+
+@pytest.mark.parametrize("masked", ["start", "row", "all but one", "alternating"])
+@pytest.mark.parametrize("v", [40, 8192, 8195])
+def test_cross_entropy_of_logits_masked_with_the_lowest_value(v, masked):
+    """Finite masks (bf16's lowest value) over whole vectors, over what a thread reads first, and over whole rows."""
+    from mesh_b200.parallel.vocab_ce import vocab_parallel_cross_entropy
+    g = torch.Generator(device="cuda").manual_seed(v)
+    low = torch.finfo(torch.bfloat16).min
+    logits = (torch.randn(3, v, device="cuda", generator=g) * 3).bfloat16()
+    if masked == "start":
+        logits[:, :v // 2] = low
+    elif masked == "row":
+        logits[1] = low
+    elif masked == "all but one":
+        logits[:, :-1] = low
+    else:
+        logits.view(-1)[::2] = low
+    logits.requires_grad_(True)
+    t = torch.tensor([v - 1, v - 2, v - 1], device="cuda")
+    loss = vocab_parallel_cross_entropy(logits, t, 0, None, reduction="none")
+    (d,) = torch.autograd.grad(loss.sum(), logits)
+    ref = logits.detach().double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(ref, t, reduction="none")
+    (dw,) = torch.autograd.grad(want.sum(), ref)
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=1e-5, atol=1e-5)
+    assert bool(((d.double() - dw).abs() <= 2 ** -8 * dw.abs() + 2e-6).all())
