@@ -29,7 +29,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 __device__ __forceinline__ void merge(float& m, float& s, float m2, float s2) {
   const float mm = fmaxf(m, m2);
-  if (mm == -CUDART_INF_F) { m = mm; s = 0.f; return; }
+  if (mm == -CUDART_INF_F) { s += s2; return; }       // nothing finite yet: both sums are 0, or NaN from a NaN logit
   s = s * __expf(m - mm) + s2 * __expf(m2 - mm);
   m = mm;
 }
@@ -76,7 +76,7 @@ __device__ __forceinline__ void online8(float& m, float& s, const uint4& q) {
 }
 __device__ __forceinline__ void online(float& m, float& s, float x) {
   if (x > m) { s = s * __expf(m - x) + 1.f; m = x; }
-  else s += m == -CUDART_INF_F ? 0.f : __expf(x - m);
+  else if (x != -CUDART_INF_F) s += __expf(x - m);    // NaN comes here, also as the first value
 }
 
 // Elements of a row before its first 16-byte boundary (rows of an odd width start anywhere).

@@ -162,3 +162,18 @@ def test_cross_entropy_of_logits_masked_with_the_lowest_value(v, masked):
     (dw,) = torch.autograd.grad(want.sum(), ref)
     torch.testing.assert_close(loss.double(), want.detach(), rtol=1e-5, atol=1e-5)
     assert bool(((d.double() - dw).abs() <= 2 ** -8 * dw.abs() + 2e-6).all())
+
+
+@pytest.mark.parametrize("v,at", [(1, 0), (7, 3), (17, 0), (17, 16), (300, 2), (4099, 4098), (4099, 1)])
+@pytest.mark.parametrize("rest", ["finite", "-inf"])
+def test_cross_entropy_keeps_a_nan(v, at, rest):
+    """Wherever the NaN logit lies (before the first 16-byte boundary, in the vectors, after them) and whether or not a thread
+    has seen a finite value before it."""
+    from mesh_b200.parallel.vocab_ce import vocab_parallel_cross_entropy
+    buf = torch.randn(3 * v + 1, device="cuda").bfloat16()[1:].view(3, v)      # rows at odd addresses
+    if rest == "-inf":
+        buf[1] = float("-inf")
+    buf[1, at] = float("nan")
+    t = torch.full((3,), (at + 1) % v, device="cuda")
+    loss = vocab_parallel_cross_entropy(buf, t, 0, None, reduction="none")
+    assert torch.isnan(loss).tolist() == [False, True, False]
