@@ -37,8 +37,8 @@ template <int W4, int U> struct StreamGeom {
 };
 
 
-__host__ __device__ inline size_t stream_fixed_bytes(int K, int B, bool coded) {
-  return lin_smem_bytes(K, B) + xsum_bytes(K, coded);
+__host__ __device__ inline size_t stream_fixed_bytes(int K, int B, int w4) {
+  return lin_smem_bytes(K, B) + xsum_bytes(K, w4);
 }
 
 struct StreamMaps { CUtensorMap w, s; };      // weights [chunk][row][128 B]; scales [row][K / 64]
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
   __shared__ int dead_s;
   volatile int* dead = &dead_s;
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * MAX_STAGES;
-  const uint32_t ring = (smem_u32(smem) + (uint32_t)stream_fixed_bytes(a.K, a.B, W4 != 0) + 1023u) & ~1023u;
+  const uint32_t ring = (smem_u32(smem) + (uint32_t)stream_fixed_bytes(a.K, a.B, W4 == 2 ? 1 : 0) + 1023u) & ~1023u;
   const uint8_t* ring_p = smem + (ring - smem_u32(smem));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Let the next kernel of the stream start its own weight requests now.
@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
   stage_x(a, xs, xstride, ComputeBar{});
   prefetch_next(a, THREADS);
   const uint8_t* xrow = xs + (g8 < a.B ? g8 : a.B - 1) * xstride + (warp * CH + t4 * (W4 == 0 ? 8 : 16)) * 2;
-  float* xsum = red + 2 * RED_FLOATS;                             // [K / 64][NB], quantised weights only
-  if constexpr (W4 != 0) sum_x<W4>(a, xs, xstride, xsum, ComputeBar{});
+  float* xsum = red + 2 * RED_FLOATS;                             // [K / 64][NB], 4-bit codes only
+  if constexpr (W4 == 2) sum_x(a, xs, xstride, xsum, ComputeBar{});
   float c[4] = {0.f, 0.f, 0.f, 0.f};
   int stage = 0, turn = 0;
   uint32_t phase = 0;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
         for (int g = 0; g < GROUPS; ++g) {
           const uint8_t* w = ra + (W4 == 2 ? (((c0 + 2 * g + (t4 >> 1)) ^ row) << 4) + (t4 & 1) * 8 : ((c0 + 4 * g + t4) ^ row) << 4);
           mma_codes<W4>(w, w + G::HALF, __half2float(at<__half>(sc + 2 * g)), __half2float(at<__half>(sc + 8 * G::SROWB + 2 * g)),
-                        *reinterpret_cast<const float2*>(xsum + (g0 + g) * NB + 2 * t4), xp + g * 128, c);
+                        W4 == 2 ? *reinterpret_cast<const float2*>(xsum + (g0 + g) * NB + 2 * t4) : make_float2(0.f, 0.f), xp + g * 128, c);
         }
       }
       __syncwarp();
@@ -213,7 +213,7 @@ static int launch_stream(const MeshDecodeLinear* d, const LinArgs& a, void* stre
     if (!encode_tiled(&maps.s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, d->scales, dims, strides, box, ones, CU_TENSOR_MAP_SWIZZLE_NONE))
       return last_error_code();
   }
-  const size_t fixed = stream_fixed_bytes(d->K, d->B, W4 != 0) + 1024;    // and the alignment of the ring
+  const size_t fixed = stream_fixed_bytes(d->K, d->B, d->w4) + 1024;    // and the alignment of the ring
   const int grid = a.n_groups < sm_count() ? a.n_groups : sm_count();
   const int stages = ring_stages(fixed, G::SLOT, (long long)((a.n_groups + grid - 1) / grid) * (d->K / G::KT));
   if (stages < 1) return set_error(-2, "decode_linear: K too large for shared memory");

@@ -414,7 +414,8 @@ __device__ __forceinline__ void finish_group(const LinArgs& a, int grp, const fl
 
 // Shared memory a layer of width K and batch B needs: the staged rows of x plus the K-split partials.
 constexpr int RED_FLOATS = WARPS * 16 * NB;
-__host__ __device__ inline size_t xsum_bytes(int K, bool coded) { return coded ? (size_t)(K / 64) * NB * sizeof(float) : 0; }
+// bytes of sum_x's table (`w4`: the weight format of MeshDecodeLinear)
+__host__ __device__ inline size_t xsum_bytes(int K, int w4) { return w4 == 1 ? (size_t)(K / 64) * NB * sizeof(float) : 0; }
 __host__ __device__ inline size_t lin_smem_bytes(int K, int B) {
   return (size_t)B * ((size_t)K * 2 + XPAD) + (size_t)2 * RED_FLOATS * sizeof(float);
 }
@@ -493,9 +494,22 @@ __device__ __forceinline__ void nibbles(uint32_t p, uint32_t (&o)[4]) {
   for (int i = 0; i < 4; ++i) o[i] = ((p >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
 }
 
-// Sums of the staged x over every 64 k, times what the offset of a code adds to a product (-136 = -(128 + 8) for 4-bit,
-// -2304 = -(17 * 128 + 128) for 8-bit codes): xsum [K / 64][NB].  The computing threads call it together after stage_x.
-template <int W4, class Sync>
+// four 8-bit codes as bf16 pairs code - 128, which are exact: 128 + the low seven bits, less 128 or 256
+__device__ __forceinline__ void bytes4(uint32_t p, uint32_t& lo, uint32_t& hi) {
+  uint32_t o[2] = {__byte_perm(p, 0, 0x4140), __byte_perm(p, 0, 0x4342)};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t t = (o[i] & 0x007F007Fu) | 0x43004300u, base = (o[i] & 0x00800080u) ^ 0x43804380u;
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&t), *reinterpret_cast<const __nv_bfloat162*>(&base));
+    o[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+  lo = o[0];
+  hi = o[1];
+}
+
+// Sums of the staged x over every 64 k, times what the offset of a 4-bit code adds to a product (-136 = -(128 + 8)): xsum
+// [K / 64][NB].  The computing threads call it together after stage_x.
+template <class Sync>
 __device__ __forceinline__ void sum_x(const LinArgs& a, const uint8_t* xs, int xstride, float* xsum, Sync sync) {
   for (int i = threadIdx.x; i < a.K / 64 * NB; i += THREADS) {
     const int n = i % NB;
@@ -512,15 +526,15 @@ __device__ __forceinline__ void sum_x(const LinArgs& a, const uint8_t* xs, int x
         s += f.x + f.y;
       }
     }
-    xsum[i] = s * (W4 == 2 ? -136.f : -2304.f);
+    xsum[i] = s * -136.f;
   }
   sync();
 }
 
-// 64 k of 16 rows: c += scale * (codes . x).  Codes enter the products as the bf16 numbers 128 + nibble, which are exact;
-// the scale, and what the offsets add (`off`: xsum of this group, batch columns 2 t4 and 2 t4 + 1), are applied to the sum
-// in fp32: half the instructions of scaling every weight, and no weight is rounded.  pA / pB: this
-// lane's 8 (4-bit) or 16 (8-bit) bytes of rows A and B, k = 16 t4 ..; xp: the lane's 16 x.
+// 64 k of 16 rows: c += scale * (codes . x).  4-bit codes enter the products as the bf16 numbers 128 + nibble, 8-bit codes as
+// code - 128; both are exact.  The scale, and what the offset of a 4-bit code adds (`off`: xsum of this group, batch columns
+// 2 t4 and 2 t4 + 1; zero for 8-bit codes), are applied to the sum in fp32: fewer instructions than scaling every weight, and
+// no weight is rounded.  pA / pB: this lane's 8 (4-bit) or 16 (8-bit) bytes of rows A and B, k = 16 t4 ..; xp: the lane's 16 x.
 template <int W4>
 __device__ __forceinline__ void mma_codes(const uint8_t* pA, const uint8_t* pB, float sa, float sb, float2 off, const uint8_t* xp, float (&c)[4]) {
   const uint4 x0 = *reinterpret_cast<const uint4*>(xp), x1 = *reinterpret_cast<const uint4*>(xp + 16);
@@ -540,16 +554,12 @@ __device__ __forceinline__ void mma_codes(const uint8_t* pA, const uint8_t* pB, 
     const uint4 pa = at<uint4>(pA), pb = at<uint4>(pB);
     const uint32_t wpa[4] = {pa.x, pa.y, pa.z, pa.w}, wpb[4] = {pb.x, pb.y, pb.z, pb.w};
     const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-    float hi[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {                          // four codes = low and high nibbles of two pairs
-      nibbles(__byte_perm(wpa[j], 0, 0x3120), wa);
-      nibbles(__byte_perm(wpb[j], 0, 0x3120), wb);
-      mma_bf16(lo, wa[0], wb[0], wa[2], wb[2], xw[2 * j], xw[2 * j + 1]);
-      mma_bf16(hi, wa[1], wb[1], wa[3], wb[3], xw[2 * j], xw[2 * j + 1]);
+    for (int j = 0; j < 4; ++j) {
+      bytes4(wpa[j], wa[0], wa[1]);
+      bytes4(wpb[j], wb[0], wb[1]);
+      mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], xw[2 * j], xw[2 * j + 1]);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) lo[i] = fmaf(16.f, hi[i], lo[i]);
   }
   c[0] = fmaf(sa, lo[0], c[0]);
   c[1] = fmaf(sa, lo[1], c[1]);

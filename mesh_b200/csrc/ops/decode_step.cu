@@ -299,7 +299,7 @@ __device__ __forceinline__ void mma_stage(const uint8_t* slot, int warp, int g8,
     for (int g = 0; g < G::CH / 64; ++g) {
       const uint8_t* w = ra + g * GB + t4 * (GB / 4);
       mma_codes<W4>(w, w + 8 * G::RS, __half2float(at<__half>(sc + 2 * g)), __half2float(at<__half>(sc + 8 * G::SROWB + 2 * g)),
-                    *reinterpret_cast<const float2*>(xsum + (k0 / 64 + g) * NB + 2 * t4), xp + g * 128, c);
+                    W4 == 2 ? *reinterpret_cast<const float2*>(xsum + (k0 / 64 + g) * NB + 2 * t4) : make_float2(0.f, 0.f), xp + g * 128, c);
     }
   }
 }
@@ -322,7 +322,7 @@ __device__ __forceinline__ void linear_stream(const LinArgs& a, uint8_t* work, R
   float* xsum = red + 2 * RED_FLOATS;
   if ((int)blockIdx.x < a.n_groups) {                                    // a CTA with no group of this layer stages nothing
     stage_x(a, xs, xstride, ComputeSync{});
-    if constexpr (W4 != 0) sum_x<W4>(a, xs, xstride, xsum, ComputeSync{});
+    if constexpr (W4 == 2) sum_x(a, xs, xstride, xsum, ComputeSync{});
   }
   const uint8_t* xrow = xs + (g8 < a.B ? g8 : a.B - 1) * xstride + (warp * G::CH + t4 * (W4 == 0 ? 8 : 16)) * 2;
   float c[4] = {0.f, 0.f, 0.f, 0.f};
@@ -512,7 +512,7 @@ extern "C" int mesh_decode_step_prepare(const MeshDecodeOp* ops, int n_ops, void
       if (kt == 0) return set_error(-2, "decode_step: a layer of this width has no streamed form (K must be a multiple of 1024 for 4-bit weights)");
       if (((uintptr_t)o.lin.w & 15) || ((uintptr_t)o.lin.scales & 15))
         return set_error(-2, "decode_step: weights and scales must be 16-byte aligned");
-      work = std::max(work, lin_smem_bytes(o.lin.K, o.lin.B) + xsum_bytes(o.lin.K, o.lin.w4 != 0));
+      work = std::max(work, lin_smem_bytes(o.lin.K, o.lin.B) + xsum_bytes(o.lin.K, o.lin.w4));
       slot = std::max(slot, (size_t)16 * (rowb + ROW_PAD) + (size_t)16 * srowb);
     } else if (o.kind == MESH_DEC_OP_ATTENTION) {
       if (o.B < 1 || o.q_heads % o.kv_heads || o.q_heads / o.kv_heads > 4)

@@ -220,3 +220,19 @@ def test_decode_argmax_of_slices_that_take_no_time(V):
     for i in range(400):
         decode_argmax(logits[i], tok[i], None)
     assert torch.equal(tok.long(), logits.argmax(-1))
+
+
+def test_decode_linear_every_8_bit_code():
+    """All 256 codes at every place of a 64-group: one input of one, so that the result is (code - 128) * scale, rounded once."""
+    from mesh_b200.ops.decode import decode_linear
+    K, N = 1024, 256
+    place = torch.arange(K, device="cuda")
+    codes = ((place[None, :] + torch.arange(N, device="cuda")[:, None]) % 256).to(torch.uint8)
+    scales = torch.linspace(0.01, 2.0, N * (K // 64), device="cuda").half().view(N, K // 64)
+    x = torch.zeros(8, K, device="cuda", dtype=torch.bfloat16)
+    for at in (0, 1, 17, 62, 63, 500, 1023):
+        x.zero_()
+        x[5, at] = 1
+        y = decode_linear(x, codes, scales=scales)
+        want = (codes[:, at].float() - 128) * scales[:, at // 64].float()
+        assert torch.equal(y[5], want.bfloat16()) and float(y[:5].abs().sum()) == 0
