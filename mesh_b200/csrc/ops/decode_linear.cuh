@@ -125,16 +125,41 @@ template <int W4, int U> struct ChunkK { static constexpr int value = (W4 == 0 ?
 // byte offset inside an x row of the first k this lane multiplies in a chunk
 template <int W4> __device__ __forceinline__ int lane_k(int t4) { return W4 == 2 ? t4 * 32 : (W4 == 3 ? t4 * 16 : t4 * 8); }
 
-// four 8-bit codes -> two bf16x2 words (c - 128) * s, exact until the final rounding to bf16
-__device__ __forceinline__ void dequant_b4(uint32_t w, float s, uint32_t& lo, uint32_t& hi) {
-  const float k = 8388736.f;                                      // 2^23 + 128
-  const float f0 = (__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540)) - k) * s;
-  const float f1 = (__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541)) - k) * s;
-  const float f2 = (__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7542)) - k) * s;
-  const float f3 = (__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7543)) - k) * s;
-  __nv_bfloat162 a = __floats2bfloat162_rn(f0, f1), b = __floats2bfloat162_rn(f2, f3);
-  lo = *reinterpret_cast<uint32_t*>(&a);
-  hi = *reinterpret_cast<uint32_t*>(&b);
+// the eight nibbles of a word, i-th of each half in o[i], as the bf16 numbers 128 + nibble
+__device__ __forceinline__ void nibbles(uint32_t p, uint32_t (&o)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = ((p >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
+}
+
+// the same as the bf16 numbers nibble - 8
+__device__ __forceinline__ void nibbles8(uint32_t p, uint32_t (&o)[4]) {
+  const __nv_bfloat162 bias2 = __floats2bfloat162_rn(136.f, 136.f);
+  nibbles(p, o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&o[i]), bias2);
+    o[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+// four 8-bit codes as bf16 pairs code - 128, which are exact: 128 + the low seven bits, less 128 or 256
+__device__ __forceinline__ void bytes4(uint32_t p, uint32_t& lo, uint32_t& hi) {
+  uint32_t o[2] = {__byte_perm(p, 0, 0x4140), __byte_perm(p, 0, 0x4342)};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t t = (o[i] & 0x007F007Fu) | 0x43004300u, base = (o[i] & 0x00800080u) ^ 0x43804380u;
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&t), *reinterpret_cast<const __nv_bfloat162*>(&base));
+    o[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+  lo = o[0];
+  hi = o[1];
+}
+
+// c += scale of the row * sum over the quad's 64 k: codes are integers in the products, so the scale is applied in fp32
+__device__ __forceinline__ void add_scaled(const float (&lo)[4], float sa, float sb, float (&c)[4]) {
+  c[0] = fmaf(sa, lo[0], c[0]);
+  c[1] = fmaf(sa, lo[1], c[1]);
+  c[2] = fmaf(sb, lo[2], c[2]);
+  c[3] = fmaf(sb, lo[3], c[3]);
 }
 
 template <int W4, int U>
@@ -219,32 +244,32 @@ __device__ __forceinline__ void mma_chunk(const Chunk<W4, U>& c, const uint8_t* 
       const uint4 x0 = *reinterpret_cast<const uint4*>(xp + 128 * u);
       const uint4 x1 = *reinterpret_cast<const uint4*>(xp + 128 * u + 16);
       const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+      float lo[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {                       // word j: 4 consecutive k = one MMA
         uint32_t al, ah, bl, bh;
-        dequant_b4(pa[j], c.sa[u], al, ah);
-        dequant_b4(pb[j], c.sb[u], bl, bh);
-        mma_bf16(acc, al, bl, ah, bh, xw[2 * j], xw[2 * j + 1]);
+        bytes4(pa[j], al, ah);
+        bytes4(pb[j], bl, bh);
+        mma_bf16(lo, al, bl, ah, bh, xw[2 * j], xw[2 * j + 1]);
       }
+      add_scaled(lo, c.sa[u], c.sb[u], acc);
     }
   } else {
     const uint32_t* pa = reinterpret_cast<const uint32_t*>(c.a);
     const uint32_t* pb = reinterpret_cast<const uint32_t*>(c.b);
-    const __nv_bfloat162 off = __floats2bfloat162_rn(136.f, 136.f);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const __nv_bfloat162 sa2 = __floats2bfloat162_rn(c.sa[u], c.sa[u]), sb2 = __floats2bfloat162_rn(c.sb[u], c.sb[u]);
-      uint32_t wa[4], wb[4];
-      dequant8(pa[2 * u], sa2, off, wa);
-      dequant8(pb[2 * u], sb2, off, wb);
-      uint4 xv = *reinterpret_cast<const uint4*>(xp + 128 * u);
-      mma_bf16(acc, wa[0], wb[0], wa[1], wb[1], xv.x, xv.y);
-      mma_bf16(acc, wa[2], wb[2], wa[3], wb[3], xv.z, xv.w);
-      dequant8(pa[2 * u + 1], sa2, off, wa);
-      dequant8(pb[2 * u + 1], sb2, off, wb);
-      xv = *reinterpret_cast<const uint4*>(xp + 128 * u + 64);
-      mma_bf16(acc, wa[0], wb[0], wa[1], wb[1], xv.x, xv.y);
-      mma_bf16(acc, wa[2], wb[2], wa[3], wb[3], xv.z, xv.w);
+      float lo[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {                       // word j: 8 consecutive k of 32 = two MMAs
+        uint32_t wa[4], wb[4];
+        nibbles8(pa[2 * u + j], wa);
+        nibbles8(pb[2 * u + j], wb);
+        const uint4 xv = *reinterpret_cast<const uint4*>(xp + 128 * u + 64 * j);
+        mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], xv.x, xv.y);
+        mma_bf16(lo, wa[2], wb[2], wa[3], wb[3], xv.z, xv.w);
+      }
+      add_scaled(lo, c.sa[u], c.sb[u], acc);
     }
   }
 }
@@ -488,25 +513,6 @@ __device__ __forceinline__ void linear_body(const LinArgs& a, uint8_t* smem, Wai
 // ---- codes in shared memory (the streaming kernels)
 template <class T>
 __device__ __forceinline__ T at(const uint8_t* p) { return *reinterpret_cast<const T*>(p); }
-// the eight nibbles of a word, i-th of each half in o[i], as the bf16 numbers 128 + nibble
-__device__ __forceinline__ void nibbles(uint32_t p, uint32_t (&o)[4]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) o[i] = ((p >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-}
-
-// four 8-bit codes as bf16 pairs code - 128, which are exact: 128 + the low seven bits, less 128 or 256
-__device__ __forceinline__ void bytes4(uint32_t p, uint32_t& lo, uint32_t& hi) {
-  uint32_t o[2] = {__byte_perm(p, 0, 0x4140), __byte_perm(p, 0, 0x4342)};
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const uint32_t t = (o[i] & 0x007F007Fu) | 0x43004300u, base = (o[i] & 0x00800080u) ^ 0x43804380u;
-    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&t), *reinterpret_cast<const __nv_bfloat162*>(&base));
-    o[i] = *reinterpret_cast<const uint32_t*>(&v);
-  }
-  lo = o[0];
-  hi = o[1];
-}
-
 // Sums of the staged x over every 64 k, times what the offset of a 4-bit code adds to a product (-136 = -(128 + 8)): xsum
 // [K / 64][NB].  The computing threads call it together after stage_x.
 template <class Sync>
@@ -561,10 +567,7 @@ __device__ __forceinline__ void mma_codes(const uint8_t* pA, const uint8_t* pB, 
       mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], xw[2 * j], xw[2 * j + 1]);
     }
   }
-  c[0] = fmaf(sa, lo[0], c[0]);
-  c[1] = fmaf(sa, lo[1], c[1]);
-  c[2] = fmaf(sb, lo[2], c[2]);
-  c[3] = fmaf(sb, lo[3], c[3]);
+  add_scaled(lo, sa, sb, c);
 }
 
 // Kernel variants (weight format, chunk width), chosen from the layer's shape by `lin_prepare`.

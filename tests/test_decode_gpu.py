@@ -165,9 +165,6 @@ def test_decode_linear_streams(bits, B, K, N):
         odd = torch.empty(scales.numel() + 1, dtype=torch.float16, device="cuda")[1:].view_as(scales).copy_(scales)
         _close(decode_linear(x, codes, scales=odd), y)                    # scales off the 16-byte grid: the other reader
     want = x.double() @ wd.T
-    if bits == 4 and K % 1024:
-        wd = wd.bfloat16().double()                                       # that reader rounds the weights
-        want = x.double() @ wd.T
     assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
 
 
@@ -236,3 +233,21 @@ def test_decode_linear_every_8_bit_code():
         y = decode_linear(x, codes, scales=scales)
         want = (codes[:, at].float() - 128) * scales[:, at // 64].float()
         assert torch.equal(y[5], want.bfloat16()) and float(y[:5].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("bits,K,odd", [(4, 512, False), (4, 1536, False), (4, 2048, False), (8, 512, True), (8, 1536, True), (8, 2048, False)])
+def test_decode_linear_codes_are_not_rounded(bits, K, odd):
+    """fp32 results of both readers.  Products of integers and bf16 are exact; partial sums of 4-bit codes run on code + 128,
+    up to 33 times the result: 33 * 2^-24 a step, a few steps."""
+    from mesh_b200.ops.decode import decode_linear, dequantize_w4, dequantize_w8, quantize_w4, quantize_w8
+    g = torch.Generator(device="cuda").manual_seed(K + bits)
+    B, N = 3, 320
+    x = torch.randn(B, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).bfloat16()
+    codes, scales = (quantize_w4 if bits == 4 else quantize_w8)(w)
+    exact = (dequantize_w4 if bits == 4 else dequantize_w8)(codes, torch.ones_like(scales)).double()
+    if odd:                                                               # off the 16-byte grid: read into registers
+        scales = torch.empty(scales.numel() + 1, dtype=torch.float16, device="cuda")[1:].view_as(scales).copy_(scales)
+    y = decode_linear(x, codes, scales=scales, out_f32=True)
+    want = x.double() @ (exact.view(N, -1, 64) * scales.double()[..., None]).view(N, K).T
+    assert float((y.double() - want).norm() / want.norm()) < 2 ** -16
