@@ -19,7 +19,7 @@ namespace decode {
 // 9.2 -> 7.8, 135 -> 103 us: there a group of 16 rows is one stage, and its barrier and epilogue bound it.
 constexpr int STREAM_THREADS = THREADS + 32;
 constexpr int MAX_STAGES = 16;
-constexpr size_t WHOLE_SMEM = 225 * 1024;
+constexpr size_t WHOLE_SMEM = 226 * 1024;           // of 227 KB: the barriers and a few words are static
 
 struct ComputeBar { __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); } };
 
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
   }
 }
 
-// Weights read into registers: 4-bit rows too short for 16 bytes per lane and warp (K an odd multiple of 512).
+// Weights read into registers: where no ring fits beside x, and rows and scales that the copies do not take.
 template <int W4, int U>
 __global__ void __launch_bounds__(THREADS) decode_linear_kernel(const LinArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -185,13 +185,22 @@ static long long weight_rows(const MeshDecodeLinear* d, const LinArgs& a) {
   return d->mode == MESH_DEC_GLU && a.up_off > 0 ? (long long)a.up_off + d->N : (long long)d->N;
 }
 
+static int grid_of(const LinArgs& a) { return a.n_groups < sm_count() ? a.n_groups : sm_count(); }
+template <int W4, int U>
+static long long stages_read(const MeshDecodeLinear* d, const LinArgs& a) {
+  return (long long)((a.n_groups + grid_of(a) - 1) / grid_of(a)) * (d->K / StreamGeom<W4, U>::KT);
+}
 // Stages of the ring: all that fit beside x, at most what the CTA reads.  A ring of half an SM's shared memory, which would
 // let the next launch fill its own while this one runs, was slower over the whole step (bf16, batch 1, five layers and
 // the head: 376 us against 341 us; 4-bit, batch 8: 288 against 249).
-static int ring_stages(size_t fixed, size_t slot, long long need) {
-  long long n = fixed < WHOLE_SMEM ? (long long)((WHOLE_SMEM - fixed) / slot) : 0;
+template <int W4, int U>
+static int ring_stages(const MeshDecodeLinear* d, const LinArgs& a) {
+  using G = StreamGeom<W4, U>;
+  if (d->K % G::KT) return 0;
+  const size_t fixed = stream_fixed_bytes(d->K, d->B, d->w4) + 1024;      // and the alignment of the ring
+  long long n = fixed < WHOLE_SMEM ? (long long)((WHOLE_SMEM - fixed) / G::SLOT) : 0;
   if (n > MAX_STAGES) n = MAX_STAGES;
-  return (int)(n < need ? n : need);
+  return (int)(n < stages_read<W4, U>(d, a) ? n : stages_read<W4, U>(d, a));
 }
 
 template <int W4, int U>
@@ -213,11 +222,50 @@ static int launch_stream(const MeshDecodeLinear* d, const LinArgs& a, void* stre
     if (!encode_tiled(&maps.s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, d->scales, dims, strides, box, ones, CU_TENSOR_MAP_SWIZZLE_NONE))
       return last_error_code();
   }
-  const size_t fixed = stream_fixed_bytes(d->K, d->B, d->w4) + 1024;    // and the alignment of the ring
-  const int grid = a.n_groups < sm_count() ? a.n_groups : sm_count();
-  const int stages = ring_stages(fixed, G::SLOT, (long long)((a.n_groups + grid - 1) / grid) * (d->K / G::KT));
-  if (stages < 1) return set_error(-2, "decode_linear: K too large for shared memory");
-  return launch(kern, grid, STREAM_THREADS, fixed + stages * G::SLOT, stream, a, maps, stages);
+  const int stages = ring_stages<W4, U>(d, a);
+  const size_t fixed = stream_fixed_bytes(d->K, d->B, d->w4) + 1024;
+  return launch(kern, grid_of(a), STREAM_THREADS, fixed + stages * G::SLOT, stream, a, maps, stages);
+}
+
+template <int W4, int U>
+static int launch_registers(const MeshDecodeLinear* d, const LinArgs& a, void* stream) {
+  auto kern = decode_linear_kernel<W4, U>;
+  static bool configured = false;
+  if (!configured) {
+    MESH_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_SMEM_MOST));
+    configured = true;
+  }
+  const size_t smem = lin_smem_bytes(d->K, d->B);
+  const int cap = sm_count() * (smem > 100 * 1024 ? 1 : 2);
+  return launch(kern, a.n_groups < cap ? a.n_groups : cap, THREADS, smem, stream, a);
+}
+
+// The register reader with the widest steps that a warp's slice of K is a multiple of.
+static int launch_registers(const MeshDecodeLinear* d, LinArgs a, int variant, void* stream) {
+  switch (variant) {
+    case LIN_W4W_U2: return launch_registers<2, 2>(d, a, stream);
+    case LIN_W4W_U1: a.xpad = XPAD; return launch_registers<1, 2>(d, a, stream);
+    case LIN_W4N_U2: return launch_registers<1, 2>(d, a, stream);
+    case LIN_W4N_U1: return launch_registers<1, 1>(d, a, stream);
+    case LIN_W8_U4: return launch_registers<3, 4>(d, a, stream);
+    case LIN_W8_U2: return launch_registers<3, 2>(d, a, stream);
+    case LIN_W8_U1: return launch_registers<3, 1>(d, a, stream);
+    case LIN_BF16_U4: return launch_registers<0, 4>(d, a, stream);
+    default: return launch_registers<0, 1>(d, a, stream);
+  }
+}
+
+// A ring needs two stages, or copies and products take turns: N = 4096, batch 8, bf16, K = 11776 with two stages 33 us, 12288
+// with one 55.  Stages of half the size come next, and registers where those do not fit twice either.  Where the register
+// reader's widest step divides a warp's slice it is the better of the two (bf16, K = 12288: 35 us, half stages 41; 8-bit 28
+// and 31); its narrow step is not (bf16, K = 12800: 83 and 56), and 4-bit codes would be rounded in its widest one.
+template <int W4>
+static int launch_reader(const MeshDecodeLinear* d, const LinArgs& a, int variant, void* stream) {
+  const int wide = ring_stages<W4, 2>(d, a), half = ring_stages<W4, 1>(d, a);
+  const bool quick = variant == LIN_BF16_U4 || variant == LIN_W8_U4;
+  if (wide >= 2 || (wide == 1 && stages_read<W4, 2>(d, a) == 1)) return launch_stream<W4, 2>(d, a, stream);
+  if ((half >= 2 && !quick) || (half == 1 && stages_read<W4, 1>(d, a) == 1)) return launch_stream<W4, 1>(d, a, stream);
+  return launch_registers(d, a, variant, stream);
 }
 
 }  // namespace decode
@@ -231,22 +279,8 @@ extern "C" int mesh_decode_linear(const MeshDecodeLinear* d, void* stream) {
   int variant = 0;
   const int rc = lin_prepare(d, a, variant);
   if (rc) return rc;
-  // read into registers: short 4-bit rows, and scales that a copy engine's 16-byte rule does not take
-  if (variant == LIN_W4N_U2 || variant == LIN_W4N_U1 || (d->w4 && (uintptr_t)d->scales % 16)) {
-    const int v = variant == LIN_W4N_U2 ? 0 : variant == LIN_W4N_U1 ? 1 : d->w4 == 8 ? 2 : 3;
-    void (*const kerns[4])(const LinArgs) = {decode_linear_kernel<1, 2>, decode_linear_kernel<1, 1>, decode_linear_kernel<3, 1>,
-                                             decode_linear_kernel<2, 1>};
-    static bool configured[4] = {};
-    if (!configured[v]) {
-      MESH_CUDA_OK(cudaFuncSetAttribute(kerns[v], cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-      configured[v] = true;
-    }
-    const size_t smem = lin_smem_bytes(d->K, d->B);
-    const int cap = sm_count() * (smem > 100 * 1024 ? 1 : 2);
-    return launch(kerns[v], a.n_groups < cap ? a.n_groups : cap, THREADS, smem, stream, a);
-  }
-  // a stage is eight 128-byte chunks of a row when K is a multiple of that many k, else four (K % 256, 512 for codes)
-  if (d->w4 == 8) return d->K % 1024 ? launch_stream<3, 1>(d, a, stream) : launch_stream<3, 2>(d, a, stream);
-  if (d->w4) return d->K % 2048 ? launch_stream<2, 1>(d, a, stream) : launch_stream<2, 2>(d, a, stream);
-  return d->K % 512 ? launch_stream<0, 1>(d, a, stream) : launch_stream<0, 2>(d, a, stream);
+  // 4-bit rows that are not whole 128-byte chunks, and scales off the 16-byte grid, are not for the copy engine
+  if (variant == LIN_W4N_U2 || variant == LIN_W4N_U1 || (d->w4 && (uintptr_t)d->scales % 16)) return launch_registers(d, a, variant, stream);
+  return d->w4 == 8 ? launch_reader<3>(d, a, variant, stream) : d->w4 ? launch_reader<2>(d, a, variant, stream)
+                                                                      : launch_reader<0>(d, a, variant, stream);
 }

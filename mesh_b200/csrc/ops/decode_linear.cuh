@@ -445,6 +445,9 @@ __host__ __device__ inline size_t lin_smem_bytes(int K, int B) {
   return (size_t)B * ((size_t)K * 2 + XPAD) + (size_t)2 * RED_FLOATS * sizeof(float);
 }
 
+// The most that a layer may ask for; the step kernel and the streaming launches need more beside it and look for themselves.
+constexpr size_t LIN_SMEM_MOST = 224 * 1024;
+
 // The layer that follows streams weights that depend on nothing computed here: ask for them to be brought into L2
 // now, behind this kernel's own loads, so that HBM keeps streaming through this kernel's reduction and epilogue,
 // the kernel boundary and the next kernel's prologue.  Every CTA requests its slice in 16 KiB pieces.
@@ -605,7 +608,7 @@ inline int lin_prepare(const MeshDecodeLinear* d, LinArgs& a, int& variant) {
       return set_error(-2, "decode_linear: qkv rows must equal (q_heads + 2 kv_heads) * head_dim");
   }
   if (d->mode == MESH_DEC_GLU) a.n_groups = d->N / 8;   // N = gate rows; every group pairs 8 gate + 8 up rows
-  if (lin_smem_bytes(d->K, d->B) > 220 * 1024) return set_error(-2, "decode_linear: K too large for shared memory");
+  if (lin_smem_bytes(d->K, d->B) > LIN_SMEM_MOST) return set_error(-2, "decode_linear: K too large for shared memory");
   const int kslice = d->K / WARPS;
   // chunk width: 128 k per step when the slice allows it (4 x 16 B per row in flight, twice), else one block
   const bool wide = kslice % 128 == 0;

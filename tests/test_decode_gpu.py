@@ -251,3 +251,28 @@ def test_decode_linear_codes_are_not_rounded(bits, K, odd):
     y = decode_linear(x, codes, scales=scales, out_f32=True)
     want = x.double() @ (exact.view(N, -1, 64) * scales.double()[..., None]).view(N, K).T
     assert float((y.double() - want).norm() / want.norm()) < 2 ** -16
+
+
+@pytest.mark.parametrize("bits,B,K", [(16, 8, 11776), (16, 8, 12288), (16, 8, 12800), (16, 8, 13312), (16, 8, 13568), (16, 7, 15616), (16, 6, 18176),
+                                      (16, 1, 110080), (8, 8, 11264), (8, 8, 12288), (8, 8, 12800), (8, 8, 13312), (8, 7, 14336), (8, 6, 17408),
+                                      (8, 1, 107520), (4, 8, 11264), (4, 8, 12288), (4, 8, 13312), (4, 7, 14336), (4, 6, 16384), (4, 1, 81920),
+                                      (4, 1, 107520)])
+def test_decode_linear_beside_a_large_input(bits, B, K):
+    """The staged rows leave room for two stages of a ring, for two of half the size, for one, for none: every K up to what x
+    and the partial sums need.  The last reader of 4-bit codes rounds weights to bf16; results are rounded to bf16."""
+    from mesh_b200.ops.decode import decode_linear, dequantize_w4, dequantize_w8, quantize_w4, quantize_w8
+    from mesh_b200.utils.status import check_status
+    g = torch.Generator(device="cuda").manual_seed(K)
+    N = 2400 if K < 20000 else 48
+    x = torch.randn(B, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).bfloat16()
+    if bits == 16:
+        y, wd = decode_linear(x, w), w.double()
+    else:
+        codes, scales = (quantize_w4 if bits == 4 else quantize_w8)(w)
+        y, wd = decode_linear(x, codes, scales=scales), (dequantize_w4 if bits == 4 else dequantize_w8)(codes, scales).double()
+    check_status()
+    want = x.double() @ wd.T
+    assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+    with pytest.raises(RuntimeError):                                     # beyond it the layer is refused
+        decode_linear(torch.zeros(B, 16 * 8192, device="cuda", dtype=torch.bfloat16), torch.zeros(16, 16 * 8192, device="cuda", dtype=torch.bfloat16))
