@@ -55,6 +55,7 @@ struct LinArgs {
   Status* status;
   const uint8_t* next_w; unsigned long long next_bytes;   // weights of the linear layer that follows in the stream
   int xpad;                                           // bytes of padding per x row in shared memory (bank spread)
+  int tight;                                          // step kernel: shared memory for one set of partials and no sums of x
 };
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -544,19 +545,22 @@ __device__ __forceinline__ void sum_x(const LinArgs& a, const uint8_t* xs, int x
 // code - 128; both are exact.  The scale, and what the offset of a 4-bit code adds (`off`: xsum of this group, batch columns
 // 2 t4 and 2 t4 + 1; zero for 8-bit codes), are applied to the sum in fp32: fewer instructions than scaling every weight, and
 // no weight is rounded.  pA / pB: this lane's 8 (4-bit) or 16 (8-bit) bytes of rows A and B, k = 16 t4 ..; xp: the lane's 16 x.
+// `centred`: 4-bit codes as nibble - 8 instead, one more operation per pair, and `off` is zero.
 template <int W4>
-__device__ __forceinline__ void mma_codes(const uint8_t* pA, const uint8_t* pB, float sa, float sb, float2 off, const uint8_t* xp, float (&c)[4]) {
+__device__ __forceinline__ void mma_codes(const uint8_t* pA, const uint8_t* pB, float sa, float sb, float2 off, const uint8_t* xp, float (&c)[4],
+                                          bool centred = false) {
   const uint4 x0 = *reinterpret_cast<const uint4*>(xp), x1 = *reinterpret_cast<const uint4*>(xp + 16);
   float lo[4] = {off.x, off.y, off.x, off.y};
   uint32_t wa[4], wb[4];
   if constexpr (W4 == 2) {
     const uint2 pa = at<uint2>(pA), pb = at<uint2>(pB);
-    nibbles(pa.x, wa);
-    nibbles(pb.x, wb);
+    auto split = [&](uint32_t p, uint32_t (&o)[4]) { if (centred) nibbles8(p, o); else nibbles(p, o); };
+    split(pa.x, wa);
+    split(pb.x, wb);
     mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], x0.x, x0.y);
     mma_bf16(lo, wa[2], wb[2], wa[3], wb[3], x0.z, x0.w);
-    nibbles(pa.y, wa);
-    nibbles(pb.y, wb);
+    split(pa.y, wa);
+    split(pb.y, wb);
     mma_bf16(lo, wa[0], wb[0], wa[1], wb[1], x1.x, x1.y);
     mma_bf16(lo, wa[2], wb[2], wa[3], wb[3], x1.z, x1.w);
   } else {

@@ -279,7 +279,7 @@ __host__ __device__ inline void variant_geom(int variant, int& kt, int& rowb, in
 
 // This warp's chunk of a stage: c += W x.
 template <int W4, int U>
-__device__ __forceinline__ void mma_stage(const uint8_t* slot, int warp, int g8, int t4, int k0, const float* xsum,
+__device__ __forceinline__ void mma_stage(const uint8_t* slot, int warp, int g8, int t4, int k0, const float* xsum, bool tight,
                                           const uint8_t* xp, float (&c)[4]) {
   using G = StageGeom<W4, U>;
   constexpr int WB = W4 == 0 ? G::CH * 2 : (W4 == 3 ? G::CH : G::CH / 2);     // bytes of a warp's k range in a row
@@ -299,7 +299,8 @@ __device__ __forceinline__ void mma_stage(const uint8_t* slot, int warp, int g8,
     for (int g = 0; g < G::CH / 64; ++g) {
       const uint8_t* w = ra + g * GB + t4 * (GB / 4);
       mma_codes<W4>(w, w + 8 * G::RS, __half2float(at<__half>(sc + 2 * g)), __half2float(at<__half>(sc + 8 * G::SROWB + 2 * g)),
-                    W4 == 2 ? *reinterpret_cast<const float2*>(xsum + (k0 / 64 + g) * NB + 2 * t4) : make_float2(0.f, 0.f), xp + g * 128, c);
+                    W4 == 2 && !tight ? *reinterpret_cast<const float2*>(xsum + (k0 / 64 + g) * NB + 2 * t4) : make_float2(0.f, 0.f),
+                    xp + g * 128, c, W4 == 2 && tight);
     }
   }
 }
@@ -322,20 +323,23 @@ __device__ __forceinline__ void linear_stream(const LinArgs& a, uint8_t* work, R
   float* xsum = red + 2 * RED_FLOATS;
   if ((int)blockIdx.x < a.n_groups) {                                    // a CTA with no group of this layer stages nothing
     stage_x(a, xs, xstride, ComputeSync{});
-    if constexpr (W4 == 2) sum_x(a, xs, xstride, xsum, ComputeSync{});
+    if (W4 == 2 && !a.tight) sum_x(a, xs, xstride, xsum, ComputeSync{});
   }
   const uint8_t* xrow = xs + (g8 < a.B ? g8 : a.B - 1) * xstride + (warp * G::CH + t4 * (W4 == 0 ? 8 : 16)) * 2;
   float c[4] = {0.f, 0.f, 0.f, 0.f};
   int turn = 0;
+  const bool tight = a.tight != 0;
   for (int grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x, turn ^= 1) {
     for (int ks = 0; ks < kstages; ++ks) {
       if (!*dead) mbar_wait(ring.full(), ring.phase, dead, a.status, SITE_SMEM_FULL);
-      mma_stage<W4, U>(reinterpret_cast<const uint8_t*>(__cvta_shared_to_generic(ring.slot())), warp, g8, t4, ks * G::KT + warp * G::CH, xsum, xrow + (size_t)ks * G::KT * 2, c);
+      mma_stage<W4, U>(reinterpret_cast<const uint8_t*>(__cvta_shared_to_generic(ring.slot())), warp, g8, t4, ks * G::KT + warp * G::CH, xsum, tight,
+                       xrow + (size_t)ks * G::KT * 2, c);
       __syncwarp();
       if (lane == 0) mbar_arrive(ring.empty());
       ring.advance();
     }
-    finish_group(a, grp, c, g8, red + turn * RED_FLOATS, ComputeSync{});
+    finish_group(a, grp, c, g8, red + (tight ? 0 : turn * RED_FLOATS), ComputeSync{});
+    if (tight) ComputeSync{}();          // the one set of partials has been read
     c[0] = c[1] = c[2] = c[3] = 0.f;
   }
   ComputeSync{}();                       // the next operation reuses the shared memory
@@ -512,7 +516,7 @@ extern "C" int mesh_decode_step_prepare(const MeshDecodeOp* ops, int n_ops, void
       if (kt == 0) return set_error(-2, "decode_step: a layer of this width has no streamed form (K must be a multiple of 1024 for 4-bit weights)");
       if (((uintptr_t)o.lin.w & 15) || ((uintptr_t)o.lin.scales & 15))
         return set_error(-2, "decode_step: weights and scales must be 16-byte aligned");
-      work = std::max(work, lin_smem_bytes(o.lin.K, o.lin.B) + xsum_bytes(o.lin.K, o.lin.w4));
+      work = std::max(work, lin_smem_bytes(o.lin.K, o.lin.B) - RED_FLOATS * sizeof(float));       // at least
       slot = std::max(slot, (size_t)16 * (rowb + ROW_PAD) + (size_t)16 * srowb);
     } else if (o.kind == MESH_DEC_OP_ATTENTION) {
       if (o.B < 1 || o.q_heads % o.kv_heads || o.q_heads / o.kv_heads > 4)
@@ -550,9 +554,19 @@ extern "C" int mesh_decode_step_prepare(const MeshDecodeOp* ops, int n_ops, void
     out.push_back(s);
   }
   if (out.size() * sizeof(StepOp) > dev_bytes) return set_error(-2, "decode_step: operation buffer too small");
-  work = (work + 1023) & ~(size_t)1023;
   slot = (slot + 127) & ~(size_t)127;
   if (slot == 0) slot = 128;
+  // Two sets of partials and the sums of x where they fit beside two stages, else one set and centred codes: a barrier more
+  // per group and an operation more per pair of codes, for the last few widths before none fits (batch 8: 12544 with bf16
+  // weights; batch 5: 19456 with 4-bit ones).
+  const size_t most = (STEP_SMEM - std::min((size_t)STEP_SMEM, 2 * slot)) & ~(size_t)1023;
+  for (StepOp& s : out) {
+    if (s.kind != DOP_LINEAR) continue;
+    const size_t full = lin_smem_bytes(s.lin.K, s.lin.B) + (s.variant == LIN_W4W_U2 || s.variant == LIN_W4W_U1 ? xsum_bytes(s.lin.K, 1) : 0);
+    s.lin.tight = full > most;
+    if (!s.lin.tight) work = std::max(work, full);
+  }
+  work = (work + 1023) & ~(size_t)1023;
   if (work + 2 * slot > (size_t)STEP_SMEM) return set_error(-2, "decode_step: a layer needs more shared memory than a CTA has");
   int n_stages = (int)(((size_t)STEP_SMEM - work) / slot);
   if (n_stages > MAX_STAGES) n_stages = MAX_STAGES;

@@ -276,3 +276,29 @@ def test_decode_linear_beside_a_large_input(bits, B, K):
     assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
     with pytest.raises(RuntimeError):                                     # beyond it the layer is refused
         decode_linear(torch.zeros(B, 16 * 8192, device="cuda", dtype=torch.bfloat16), torch.zeros(16, 16 * 8192, device="cuda", dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("bits,B,K", [(16, 8, 9216), (16, 8, 12544), (16, 6, 16640), (16, 1, 100864), (8, 6, 15360), (8, 4, 25088), (4, 5, 19456),
+                                      (4, 4, 23552), (4, 1, 88064)])
+def test_step_kernel_beside_a_large_input(bits, B, K):
+    """A recorded step whose first layer leaves little shared memory, and a second one that reads what the first stored."""
+    from mesh_b200.ops.decode import decode_linear, dequantize_w4, dequantize_w8, quantize_w4, quantize_w8, record_step
+    from mesh_b200.utils.status import check_status
+    g = torch.Generator(device="cuda").manual_seed(K)
+    N = 3072 if K < 20000 else 1024                                       # more than one group of 16 rows for some CTAs
+    x = torch.randn(B, K, device="cuda", generator=g).bfloat16()
+    w, w2 = ((torch.randn(*s, device="cuda", generator=g) * 0.02).bfloat16() for s in ((N, K), (64, 512)))
+    coded = (w, None) if bits == 16 else (quantize_w4 if bits == 4 else quantize_w8)(w)
+    wd = w if bits == 16 else (dequantize_w4 if bits == 4 else dequantize_w8)(*coded)
+    y, y2 = torch.empty(B, N, device="cuda", dtype=torch.bfloat16), torch.empty(B, 64, device="cuda", dtype=torch.bfloat16)
+    with record_step() as step:
+        decode_linear(x, coded[0], scales=coded[1], out=y)
+        decode_linear(y[:, :512], w2, out=y2)
+    for _ in range(2):
+        y.zero_()
+        step.run()
+        check_status()
+        want = x.double() @ wd.double().T
+        assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
+        want = y[:, :512].double() @ w2.double().T
+        assert float((y2.double() - want).norm() / want.norm()) < 2 ** -8
