@@ -1,6 +1,6 @@
-// Vocabulary-parallel greedy selection: a cluster of CTAs per sequence finds (max logit, lowest index) over
-// this rank's vocabulary shard (a slice each, the pairs meet in the first CTA's shared memory), exchanges that 8-byte pair with every rank, and all ranks pick the
-// same winner (highest value, lowest global index on ties) without ever gathering logits.
+// Vocabulary-parallel greedy selection: a CTA, or a cluster of them, per sequence finds (max logit, lowest index) over this
+// rank's vocabulary shard (a slice each, the pairs meet in the first CTA's shared memory), exchanges that 8-byte pair with
+// every rank, and all ranks pick the same winner (highest value, lowest global index on ties) without ever gathering logits.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include "decode_api.h"
@@ -12,20 +12,23 @@ namespace mesh {
 namespace {
 
 constexpr int AM_THREADS = 1024;
-// One CTA of 1024 threads is a chain of 256 loads per thread over 262144 logits: 9.6 us back to back; eight CTAs: 4.4 us.
-constexpr int AM_CTAS = 8;
+// One CTA of 1024 threads is a chain of loads over a long vocabulary, and a cluster's barriers cost more than a short one.
+// Back to back at batch 1 / 8, one CTA and eight: 4096 logits 1.7 / 1.8 and 2.2 / 2.4 us, 16384 2.0 / 2.2 and 2.2 / 2.6,
+// 32768 2.5 / 2.6 and 2.3 / 2.8, 65536 3.4 / 3.6 and 2.6 / 3.0, 262144 8.7 / 8.9 and 3.2 / 3.9.
+constexpr int MOST_CTAS = 8, ONE_CTA_VOCAB = 16384;
 
 __device__ __forceinline__ void better(float& v, int& i, float ov, int oi) {
   if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
 
+template <int AM_CTAS>
 __global__ void __launch_bounds__(AM_THREADS)
 decode_argmax_kernel(const float* __restrict__ logits, long long ldl, int vocab_local, int vocab_offset,
                      int* __restrict__ tokens_out, int* __restrict__ pos, int rank, int world,
                      uint2* const* __restrict__ xchg_unused, uint2* x0, uint2* x1, uint2* x2, uint2* x3, uint2* x4,
                      uint2* x5, uint2* x6, uint2* x7, uint32_t* step, Status* st) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  cluster_arrive_relaxed();             // waited for before the store into the first CTA's shared memory
+  if (AM_CTAS > 1) cluster_arrive_relaxed();             // waited for before the store into the first CTA's shared memory
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int b = blockIdx.x / AM_CTAS, part = blockIdx.x % AM_CTAS;
   const uint32_t seq = (step ? *step : 0u) + 1u;
@@ -61,7 +64,7 @@ decode_argmax_kernel(const float* __restrict__ logits, long long ldl, int vocab_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { sv[warp] = best; si[warp] = bi; }
   __syncthreads();
-  cluster_wait();
+  if (AM_CTAS > 1) cluster_wait();
   if (warp == 0) {
     best = sv[lane];
     bi = si[lane];
@@ -71,21 +74,23 @@ decode_argmax_kernel(const float* __restrict__ logits, long long ldl, int vocab_
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       better(best, bi, ov, oi);
     }
-    if (lane == 0) {
+    if (AM_CTAS > 1 && lane == 0) {
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_u32(smem_u32(&pv[part]), 0)), "f"(best) : "memory");
       asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(smem_u32(&pi[part]), 0)), "r"(bi) : "memory");
     }
     __syncwarp();
   }
-  cluster_sync_all();
+  if (AM_CTAS > 1) cluster_sync_all();
   if (part != 0 || warp != 0) return;
-  best = lane < AM_CTAS ? pv[lane] : -CUDART_INF_F;
-  bi = lane < AM_CTAS ? pi[lane] : 0x7fffffff;
+  if (AM_CTAS > 1) {
+    best = lane < AM_CTAS ? pv[lane] : -CUDART_INF_F;
+    bi = lane < AM_CTAS ? pi[lane] : 0x7fffffff;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    better(best, bi, ov, oi);
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      better(best, bi, ov, oi);
+    }
   }
   int gidx = bi + vocab_offset;
   if (world > 1) {
@@ -151,22 +156,23 @@ extern "C" int mesh_decode_argmax(const float* logits, long long ldl, int B, int
   if (world < 1 || world > 8) return set_error(-4, "decode_argmax: world out of range");
   uint2* x[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   for (int r = 0; r < world && xchg; ++r) x[r] = (uint2*)xchg[r];
+  const int ctas = vocab_local <= ONE_CTA_VOCAB ? 1 : MOST_CTAS;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)B * AM_CTAS);
+  cfg.gridDim = dim3((unsigned)(B * ctas));
   cfg.blockDim = dim3(AM_THREADS);
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = AM_CTAS;
+  attr[1].val.clusterDim.x = (unsigned)ctas;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = ctas > 1 ? 2 : 1;
   uint2* const* none = nullptr;
-  MESH_CUDA_OK(cudaLaunchKernelEx(&cfg, decode_argmax_kernel, logits, ldl, vocab_local, vocab_offset, tokens_out, pos, rank,
+  MESH_CUDA_OK(cudaLaunchKernelEx(&cfg, ctas > 1 ? decode_argmax_kernel<MOST_CTAS> : decode_argmax_kernel<1>, logits, ldl, vocab_local, vocab_offset, tokens_out, pos, rank,
                                   world, none, x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7], step, (Status*)status));
   return 0;
 }

@@ -192,7 +192,7 @@ def test_decode_attention_clusters_and_splits(hd, qh, kvh, splits, S, window):
         assert float((out[b].double() - want).norm() / want.norm()) < 2 ** -8
 
 
-@pytest.mark.parametrize("V,ld", [(1, 1), (5, 8), (16385, 16385), (262144, 262144)])
+@pytest.mark.parametrize("V,ld", [(1, 1), (5, 8), (16383, 16384), (16384, 16384), (16385, 16385), (262144, 262144)])
 def test_decode_argmax_slices(V, ld):
     from mesh_b200.ops.decode import decode_argmax
     B = 3
@@ -206,10 +206,10 @@ def test_decode_argmax_slices(V, ld):
     assert tok.tolist() == [0, V - 1, V // 2]
 
 
-@pytest.mark.parametrize("V", [1, 3, 9, 33])
+@pytest.mark.parametrize("V", [1, 3, 9, 33, 16388])
 def test_decode_argmax_of_slices_that_take_no_time(V):
-    """A CTA of the cluster with an empty slice, or one of a few logits, has its pair ready as soon as it runs; every launch
-    has other logits, so a pair that got lost or came from the launch before shows in the token."""
+    """Few logits, or a cluster with 2056 logits for a CTA, whose pair is ready soon after it runs; every launch has other
+    logits, so a pair that got lost or came from the launch before shows in the token."""
     from mesh_b200.ops.decode import decode_argmax
     g = torch.Generator(device="cuda").manual_seed(V)
     logits = torch.randn(400, 8, V, device="cuda", generator=g)
