@@ -71,12 +71,15 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
     // ---------------------------------------------------------------- weights
     if (lane != 0) return;
     int stage = 0, n = 0;
-    for (int grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
+    bool ok = true;
+    for (int grp = blockIdx.x; ok && grp < a.n_groups; grp += gridDim.x) {
       int rA, rB;
       group_rows(a, grp, rA, rB);
       for (int ks = 0; ks < kstages; ++ks, ++n) {
         const uint32_t full = full0 + 8 * stage;
-        if (n >= n_stages && !mbar_wait(empty0 + 8 * stage, ((n / n_stages) - 1) & 1, dead, a.status, SITE_SMEM_EMPTY)) return;
+        if (n >= n_stages) ok = mbar_wait(empty0 + 8 * stage, ((n / n_stages) - 1) & 1, dead, a.status, SITE_SMEM_EMPTY);
+        ok = ok && !*dead;                     // after that the computing warps free stages whether or not they were filled
+        if (!ok) break;
         mbar_expect_tx(full, G::TX);
         const uint32_t slot = ring + (uint32_t)stage * G::SLOT;
         tma_load_3d(slot, &maps.w, full, 0, rA, ks * G::KC);
@@ -87,6 +90,12 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
         }
         if (++stage == n_stages) stage = 0;
       }
+    }
+    // The CTA's shared memory has to stay until the last copies have landed in it, also when the computing warps gave up on
+    // them: nobody else waits then.
+    for (int i = max(0, n - n_stages); i < n; ++i) {
+      const unsigned long long t0 = globaltimer_ns();
+      while (!mbar_try_wait(full0 + 8 * (i % n_stages), (i / n_stages) & 1) && globaltimer_ns() - t0 < MESH_WAIT_LIMIT_NS) { __nanosleep(100); }
     }
     return;
   }
