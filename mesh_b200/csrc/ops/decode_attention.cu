@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
   visible(A, b, lo, hi);
   WarpState<HD, MAXG> st;
   // neighbouring keys to different CTAs, so that a short context uses all of them
-  scan_keys<HD, MAXG>(A, kvh, b, lo, hi, warp * ranks + rank, ATT_WARPS * ranks, st);
+  scan_keys<HD, MAXG>(A, kvh, b, lo, hi, warp * ranks + rank, ATT_WARPS * ranks, false, st);
   if (lane < 2 * MAXG && !(lane & 1)) {
     sm_m[warp][lane >> 1] = st.m;
     sm_l[warp][lane >> 1] = st.l;
@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
   cluster_sync_all();                                    // nobody's shared memory goes away while it is read
 }
 
-// Many splits of a long context: partial results in global memory, merged by the CTA that finishes last.
+// Many splits of a long context, and inputs that vector loads do not take: partial results in global memory, merged by the CTA
+// that finishes last.
 // Grid = (splits, kv_heads, batch * tokens): one work item per CTA.
 template <int HD, int MAXG>
 __global__ void __launch_bounds__(ATT_THREADS) decode_attention_kernel(const AttArgs A) {
@@ -155,10 +156,11 @@ extern "C" int mesh_decode_attention(const void* q, const void* k_cache, const v
   A.out = (__nv_bfloat16*)out; A.scratch = scratch; A.counters = counters;
   A.q_heads = q_heads; A.kv_heads = kv_heads; A.max_seq = max_seq; A.window = window; A.scale = scale; A.splits = splits;
   A.T = tokens_per_seq; A.B = B; A.head_dim = head_dim;
+  A.unaligned = unaligned(q, k_cache, v_cache, head_dim);
   // A cluster takes what 64 warps scan in a few steps, or whatever is asked for in no more splits than it has CTAs; more
   // splits of a longer context go to more CTAs than a cluster has.
   const int most = window > 0 && window < max_seq ? window : max_seq;
-  const bool cluster = splits <= MAX_CLUSTER || most <= 4096;
+  const bool cluster = !A.unaligned && (splits <= MAX_CLUSTER || most <= 4096);
   const bool four = q_heads / kv_heads <= 4;
   switch (head_dim) {
     case 256: return four ? launch<256, 4>(A, cluster, stream) : launch<256, 8>(A, cluster, stream);

@@ -26,6 +26,7 @@ struct AttArgs {
   __nv_bfloat16* out; float* scratch; int* counters;
   int q_heads, kv_heads, max_seq, window; float scale; int splits, T;
   int B, head_dim;                                   // used by callers that loop over the work items themselves
+  int unaligned;                                     // q or a cache does not start on a multiple of a lane's bytes
 };
 
 struct AttBlockSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
@@ -46,6 +47,20 @@ __device__ __forceinline__ void widen(const Raw<PER>& r, float (&f)[PER]) {
   }
 }
 
+// `one_by_one`: the address is not a multiple of the vector's size.
+template <int PER>
+__device__ __forceinline__ Raw<PER> load_raw(const __nv_bfloat16* p, bool one_by_one) {
+  Raw<PER> r;
+  if (!one_by_one) return *reinterpret_cast<const Raw<PER>*>(p);
+  __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(&r);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) h[i] = p[i];
+  return r;
+}
+inline bool unaligned(const void* q, const void* kc, const void* vc, int head_dim) {
+  return (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % (uintptr_t)(head_dim / 32 * 2)) != 0;
+}
+
 // Running softmax of one warp over its keys.  A lane owns HD / 32 consecutive dims of K, V and the accumulators; m and l
 // are those of head `lane / 2 % MAXG`, the head whose scores the lane holds after the reduction below.
 template <int HD, int MAXG>
@@ -58,9 +73,10 @@ struct WarpState {
 // Keys of this warp: KEYS consecutive ones starting at lo + gw * KEYS, then every `warps` * KEYS further, up to hi.  All
 // loads of a step are issued together (a key costs a trip to L2 or HBM, not two); the 16 partial dot products are
 // reduced with 16 shuffles instead of 5 each, and every lane then works on one score: one exponential, not 16.
+// `one_by_one`: see load_raw.
 template <int HD, int MAXG>
 __device__ __forceinline__ void scan_keys(const AttArgs& A, int kvh, int b, int lo, int hi, int gw, int warps,
-                                          WarpState<HD, MAXG>& st) {
+                                          bool one_by_one, WarpState<HD, MAXG>& st) {
   constexpr int PER = HD / 32, KEYS = WarpState<HD, MAXG>::KEYS;
   const int lane = threadIdx.x & 31;
   const int group = A.q_heads / A.kv_heads;
@@ -73,7 +89,7 @@ __device__ __forceinline__ void scan_keys(const AttArgs& A, int kvh, int b, int 
 #pragma unroll
   for (int g = 0; g < MAXG; ++g) {
     Raw<PER> r = {};
-    if (g < group) r = *reinterpret_cast<const Raw<PER>*>(A.q + ((long long)b * A.q_heads + kvh * group + g) * HD + lane * PER);
+    if (g < group) r = load_raw<PER>(A.q + ((long long)b * A.q_heads + kvh * group + g) * HD + lane * PER, one_by_one);
     widen<PER>(r, qv[g]);
 #pragma unroll
     for (int i = 0; i < PER; ++i) qv[g][i] *= A.scale;
@@ -91,8 +107,8 @@ __device__ __forceinline__ void scan_keys(const AttArgs& A, int kvh, int b, int 
 #pragma unroll
     for (int k = 0; k < KEYS; ++k) {
       const long long at = (long long)min(j + k, hi - 1) * HD;
-      kr[k] = *reinterpret_cast<const Raw<PER>*>(kbase + at);
-      vr[k] = *reinterpret_cast<const Raw<PER>*>(vbase + at);
+      kr[k] = load_raw<PER>(kbase + at, one_by_one);
+      vr[k] = load_raw<PER>(vbase + at, one_by_one);
     }
     float s[16];
 #pragma unroll
@@ -175,7 +191,7 @@ __device__ __forceinline__ void attention_item(const AttArgs& A, int split, int 
   const int per_split = (hi_all - lo_all + splits - 1) / splits;
   const int lo = lo_all + split * per_split;
   WarpState<HD, MAXG> st;
-  scan_keys<HD, MAXG>(A, kvh, b, lo, min(hi_all, lo + per_split), warp, ATT_WARPS, st);
+  scan_keys<HD, MAXG>(A, kvh, b, lo, min(hi_all, lo + per_split), warp, ATT_WARPS, A.unaligned != 0, st);
   // ---- merge the 8 warps of the CTA through shared memory
   __shared__ float sm_m[ATT_WARPS][MAX_GROUP], sm_l[ATT_WARPS][MAX_GROUP];
   auto sm_acc = [&](int w, int g, int d) -> float& { return sm_acc_raw[((long long)w * group + g) * HD + d]; };

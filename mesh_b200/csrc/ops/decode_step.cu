@@ -530,6 +530,7 @@ extern "C" int mesh_decode_step_prepare(const MeshDecodeOp* ops, int n_ops, void
       A.pos = o.pos; A.out = (__nv_bfloat16*)o.att_out; A.scratch = o.scratch; A.counters = o.counters;
       A.q_heads = o.q_heads; A.kv_heads = o.kv_heads; A.max_seq = o.max_seq; A.window = o.window; A.scale = o.scale;
       A.splits = o.splits; A.T = 1; A.B = o.B; A.head_dim = o.head_dim;
+      A.unaligned = decode_att::unaligned(o.q, o.k_cache, o.v_cache, o.head_dim);
       work = std::max(work, (size_t)decode_att::ATT_WARPS * (o.q_heads / o.kv_heads) * o.head_dim * sizeof(float));
     } else if (o.kind == MESH_DEC_OP_EMBED) {
       if (o.d_model % 8 || o.B < 1) return set_error(-2, "decode_step: embedding rows must be a multiple of 8 wide");

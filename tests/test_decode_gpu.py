@@ -302,3 +302,31 @@ def test_step_kernel_beside_a_large_input(bits, B, K):
         assert float((y.double() - want).norm() / want.norm()) < 2 ** -8
         want = y[:, :512].double() @ w2.double().T
         assert float((y2.double() - want).norm() / want.norm()) < 2 ** -8
+
+
+def _shifted(t, by):
+    """The values of ``t`` in memory that starts ``by`` elements after an aligned address."""
+    return torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)[by:].view_as(t).copy_(t)
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("recorded", [False, True])
+@pytest.mark.parametrize("which,by", [("q", 1), ("k", 1), ("v", 3), ("all", 2)])
+def test_decode_attention_of_inputs_at_any_address(hd, recorded, which, by):
+    from mesh_b200.ops.decode import DecodeAttention, record_step
+    B, qh, kvh, S = 2, 8, 2, 150
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    kc, vc = (torch.randn(B, kvh, S, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(B, qh * hd, device="cuda", generator=g).bfloat16()
+    pos = torch.tensor([S - 1, 70], dtype=torch.int32, device="cuda")
+    att = DecodeAttention(B, qh, kvh, hd, splits=16)
+    want, out = (torch.empty(B, qh * hd, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    att(q, kc, vc, pos, want)
+    moved = [_shifted(t, by) if which in (n, "all") else t for n, t in (("q", q), ("k", kc), ("v", vc))]
+    if recorded:
+        with record_step() as step:
+            att(*moved, pos, out)
+        step.run()
+    else:
+        att(*moved, pos, out)
+    _close(out, want, 1e-2)                                               # the same sums in another order, rounded to bf16
