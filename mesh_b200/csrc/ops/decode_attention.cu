@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
       float a = 0.f, ll = 0.f;
 #pragma unroll
       for (int w = 0; w < ATT_WARPS; ++w) {
-        const float wgt = sm_m[w][g] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][g] - mm);
+        const float wgt = partial_weight(sm_m[w][g], sm_l[w][g], mm);
         a += wgt * sm_acc[(long long)w * MAXG * HD + e];
         ll += wgt * sm_l[w][g];
       }
@@ -83,10 +83,10 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
     float a = 0.f, ll = 0.f;
 #pragma unroll
     for (int r = 0; r < MAX_CLUSTER; ++r) {
-      const float wgt = m[r] == -CUDART_INF_F ? 0.f : __expf(m[r] - mm);
-      if (wgt > 0.f) { a += wgt * v[r]; ll += wgt * l[r]; }
+      const float wgt = r < ranks ? partial_weight(m[r], l[r], mm) : 0.f;
+      if (wgt != 0.f) { a += wgt * v[r]; ll += wgt * l[r]; }
     }
-    A.out[((long long)b * A.q_heads + kvh * group) * HD + e] = __float2bfloat16_rn(ll > 0.f ? a / ll : 0.f);
+    A.out[((long long)b * A.q_heads + kvh * group) * HD + e] = __float2bfloat16_rn(ll == 0.f ? 0.f : a / ll);
   }
   cluster_sync_all();                                    // nobody's shared memory goes away while it is read
 }

@@ -57,6 +57,11 @@ __device__ __forceinline__ Raw<PER> load_raw(const __nv_bfloat16* p, bool one_by
   for (int i = 0; i < PER; ++i) h[i] = p[i];
   return r;
 }
+// Weight of a partial result (m, l) relative to the maximum mm: 0 where nothing was seen, NaN where all that was seen was NaN
+// (a maximum ignores NaN, the sum l does not).
+__device__ __forceinline__ float partial_weight(float m, float l, float mm) {
+  return m == -CUDART_INF_F ? 0.f * l : __expf(m - mm);
+}
 inline bool unaligned(const void* q, const void* kc, const void* vc, int head_dim) {
   return (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % (uintptr_t)(head_dim / 32 * 2)) != 0;
 }
@@ -138,8 +143,9 @@ __device__ __forceinline__ void scan_keys(const AttArgs& A, int kvh, int b, int 
     float mx = sc;                                    // over the keys of this head
 #pragma unroll
     for (int o = 16; o >= 2 * MAXG; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const float mn = fmaxf(st.m, mx);                 // finite: key j exists
-    const float corr = __expf(st.m - mn), w = __expf(sc - mn);
+    const float mn = fmaxf(st.m, mx);
+    const float ref = mn == -CUDART_INF_F ? 0.f : mn;  // nothing but -inf (weight 0) and NaN (which stays) so far
+    const float corr = __expf(st.m - ref), w = __expf(sc - ref);
     float ws = w;
 #pragma unroll
     for (int o = 16; o >= 2 * MAXG; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
@@ -212,13 +218,13 @@ __device__ __forceinline__ void attention_item(const AttArgs& A, int split, int 
     for (int w = 0; w < ATT_WARPS; ++w) mm = fmaxf(mm, sm_m[w][g]);
     float ll = 0.f;
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS; ++w) ll += (sm_m[w][g] == -CUDART_INF_F) ? 0.f : sm_l[w][g] * __expf(sm_m[w][g] - mm);
+    for (int w = 0; w < ATT_WARPS; ++w) ll += sm_l[w][g] * partial_weight(sm_m[w][g], sm_l[w][g], mm);
     float* pg = part + (long long)g * splits * (HD + 2);
     for (int d = threadIdx.x; d < HD; d += ATT_THREADS) {
       float a = 0.f;
 #pragma unroll
       for (int w = 0; w < ATT_WARPS; ++w)
-        a += (sm_m[w][g] == -CUDART_INF_F) ? 0.f : sm_acc(w, g, d) * __expf(sm_m[w][g] - mm);
+        a += sm_acc(w, g, d) * partial_weight(sm_m[w][g], sm_l[w][g], mm);
       pg[d] = a;
     }
     if (threadIdx.x == 0) { pg[HD] = mm; pg[HD + 1] = ll; }
@@ -251,12 +257,12 @@ __device__ __forceinline__ void attention_item(const AttArgs& A, int split, int 
     for (int s = 0; s < splits; ++s) mm = fmaxf(mm, w_s[g][s]);
     float ll = 0.f;
     for (int s = 0; s < splits; ++s) {
-      const float ms = w_s[g][s];
-      const float wgt = (ms == -CUDART_INF_F) ? 0.f : __expf(ms - mm);
-      ll += wgt * __ldcg(pbase + ((long long)g * splits + s) * (HD + 2) + HD + 1);
+      const float ls = __ldcg(pbase + ((long long)g * splits + s) * (HD + 2) + HD + 1);
+      const float wgt = partial_weight(w_s[g][s], ls, mm);
+      ll += wgt * ls;
       w_s[g][s] = wgt;
     }
-    inv_s[g] = ll > 0.f ? 1.f / ll : 0.f;
+    inv_s[g] = ll == 0.f ? 0.f : 1.f / ll;
   }
   sync();
   for (int idx = threadIdx.x; idx < group * HD; idx += ATT_THREADS) {

@@ -330,3 +330,21 @@ def test_decode_attention_of_inputs_at_any_address(hd, recorded, which, by):
     else:
         att(*moved, pos, out)
     _close(out, want, 1e-2)                                               # the same sums in another order, rounded to bf16
+
+
+@pytest.mark.parametrize("at", [0, 17, 199])
+@pytest.mark.parametrize("keys", [1, 200, 5000])
+def test_decode_attention_keeps_a_nan(keys, at):
+    """A NaN key, alone in its warp or among others, by both kernels (clusters, and 64 splits of a cache of 5000): the heads that
+    read it are NaN, the others are not."""
+    from mesh_b200.ops.decode import DecodeAttention
+    qh, kvh, hd = 8, 2, 128
+    at = min(at, keys - 1)
+    g = torch.Generator(device="cuda").manual_seed(keys)
+    kc, vc = (torch.randn(1, kvh, max(keys, 256), hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    kc[0, 1, at, 5] = float("nan")
+    q = torch.randn(1, qh * hd, device="cuda", generator=g).bfloat16()
+    pos = torch.tensor([keys - 1], dtype=torch.int32, device="cuda")
+    out = torch.empty(1, qh * hd, device="cuda", dtype=torch.bfloat16)
+    DecodeAttention(1, qh, kvh, hd, splits=64)(q, kc, vc, pos, out)
+    assert torch.isnan(out.view(qh, hd)).all(-1).tolist() == [False] * 4 + [True] * 4 and not torch.isnan(out.view(qh, hd)[:4]).any()
