@@ -730,29 +730,33 @@ __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restr
                                                     float* __restrict__ zero, int B, int T, int H) {
   constexpr int L = HD / 8;
   const long long total = (long long)B * T * H * L;
-  for (long long idx = blockIdx.x * 256ll + threadIdx.x; idx < total; idx += gridDim.x * 256ll) {   // total is a multiple of L
+  // the turns are the warp's, so that all lanes meet at the shuffles; a row's lanes are in or out together (total % L == 0)
+  for (long long first = blockIdx.x * 256ll + (threadIdx.x & ~31); first < total; first += gridDim.x * 256ll) {
+    const long long idx = first + (threadIdx.x & 31);
+    const bool in = idx < total;
     const int v = (int)(idx % L);
     const long long rh = idx / L;
     const int h = (int)(rh % H);
     const long long row = rh / H;
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(dout + row * ld_do + (long long)h * HD) + v);
-    const uint4 o = __ldg(reinterpret_cast<const uint4*>(out + row * ld_o + (long long)h * HD) + v);
-    const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&o);
     float s = 0.f;
+    if (in) {
+      const uint4 a = __ldg(reinterpret_cast<const uint4*>(dout + row * ld_do + (long long)h * HD) + v);
+      const uint4 o = __ldg(reinterpret_cast<const uint4*>(out + row * ld_o + (long long)h * HD) + v);
+      const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+      const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&o);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(o2[i]);
-      s += x.x * y.x + x.y * y.y;
+      for (int i = 0; i < 4; ++i) {
+        const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(o2[i]);
+        s += x.x * y.x + x.y * y.y;
+      }
     }
-    const unsigned lanes = __activemask();             // whole groups of L lanes are in or out of the last pass together
 #pragma unroll
-    for (int m = L / 2; m > 0; m >>= 1) s += __shfl_xor_sync(lanes, s, m);
-    if (v == 0) {
+    for (int m = L / 2; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if (in && v == 0) {
       const long long b = row / T, t = row % T;
       delta[(b * H + h) * T + t] = s;
     }
-    if (zero) {
+    if (in && zero) {
       float4* z = reinterpret_cast<float4*>(zero + rh * HD) + 2 * v;
       z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }

@@ -332,3 +332,18 @@ def test_flash_heads_of_256_alternate_between_groups(T, p):
         assert float((out.float() - ref).norm() / ref.norm()) < 6e-3
         torch.testing.assert_close(lse, lse_ref, atol=1e-4, rtol=1e-4)
     check_status()
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("B,T,H", [(1, 1, 1), (1, 5, 3), (3, 333, 5), (2, 4097, 7)])
+def test_delta_of_any_number_of_rows(hd, B, T, H):
+    """Row sums of dO o O, from fewer rows than a warp holds to more than the grid takes at once, with the accumulator cleared."""
+    from mesh_b200.ops.attention import _delta
+    g = torch.Generator(device="cuda").manual_seed(T)
+    do, o = (torch.randn(B, T, H, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    clear = torch.full((B, T, H, hd), float("nan"), device="cuda")
+    got = _delta(do, o, clear)
+    want = (do.double() * o.double()).sum(-1).transpose(1, 2)
+    # fp32 sums of hd products of order one
+    assert float((got.double() - want).abs().max()) < hd * 2 ** -20
+    assert float(clear.abs().sum()) == 0
