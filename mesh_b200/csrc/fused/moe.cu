@@ -138,13 +138,15 @@ struct PlanArgs {
   int* send_base;              // [experts]: first row for this sender in the destination's region of expert e
   int* layout;                 // [3 * local experts + 2]: n_e..., base_e..., padded_e..., total_rows, dropped flag
   MeshTileDesc* t_glu; MeshTileDesc* t_down; MeshTileDesc* t_dh; MeshTileDesc* t_dx; MeshTileDesc* t_dw2; MeshTileDesc* t_dw1;
-  int* n_tiles;                // [6]
+  int* n_tiles;                // [8]: lengths of the six tables, then two counters that the launch leaves at zero
   int max_tiles;
   Status* status;
 };
 
 // Every CTA works out the same layout (a few microseconds of a 60 us kernel when one CTA wrote all tables, some fifteen
-// thousand 32-byte records at 64 experts); the first one stores it, and the experts' records are shared out.
+// thousand 32-byte records at 64 experts); the first one stores it, and the experts' records are shared out.  Each waits for
+// the counts by itself, so one may give up where another did not: the last to finish publishes the tables' lengths, and
+// publishes zeros when any of them wrote no records.
 constexpr int PLAN_CTAS = 16;
 
 __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
@@ -161,8 +163,25 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
   }
   __syncthreads();
   const bool first = blockIdx.x == 0;
+  __shared__ int off[6][MAX_E + 1];
+  __shared__ int last_s, failed_s;
+  auto publish = [&](bool ok) {            // all threads of the CTA
+    __threadfence();                       // this thread's records before this CTA's mark
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (!ok) atomicAdd(a.n_tiles + 7, 1);
+      __threadfence();
+      last_s = atomicAdd(a.n_tiles + 6, 1) == (int)gridDim.x - 1;
+      if (last_s) {
+        failed_s = atomicExch(a.n_tiles + 7, 0);
+        a.n_tiles[6] = 0;                  // ready for the next launch
+      }
+    }
+    __syncthreads();
+    if (last_s && threadIdx.x < 6) a.n_tiles[threadIdx.x] = failed_s == 0 ? min(off[threadIdx.x][El], a.max_tiles) : 0;
+  };
   if (!ok_s) {
-    if (first && threadIdx.x < 6) a.n_tiles[threadIdx.x] = 0;
+    publish(false);
     return;
   }
   // every destination's layout is the same function of the matrix; this rank needs all of them as a sender
@@ -212,7 +231,6 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
   // ---- tile tables (pair tiles: 256 output rows each).  Table t of expert el holds cnt[t][el] descriptors starting at
   // off[t][el]; thread 0 lays the offsets out (6 x local experts additions), then every warp writes the descriptors of
   // its experts, a lane per tile: the tables are thousands of 32-byte records, far too many for one thread.
-  __shared__ int off[6][MAX_E + 1];
   const int D = a.d_model, F = a.d_ff;
   const int ntn[6] = {(F + 127) / 128, (D + 255) / 256, (F + 255) / 256, (D + 255) / 256, (F + 255) / 256, (D + 255) / 256};
   const int dw_mt[2] = {(D + 255) / 256, (2 * F + 255) / 256};
@@ -225,7 +243,6 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
       n += t < 4 ? (rows / 256) * ntn[t] : (rows >= 64 ? dw_mt[t - 4] * ntn[t] : 0);
     }
     off[t][El] = n;
-    if (first) a.n_tiles[t] = min(n, a.max_tiles);
   }
   __syncthreads();
   MeshTileDesc* const tab[6] = {a.t_glu, a.t_down, a.t_dh, a.t_dx, a.t_dw2, a.t_dw1};
@@ -251,6 +268,7 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
       }
     }
   }
+  publish(true);
 }
 
 // ------------------------------------------------------------------------------------------- zero padding rows

@@ -23,7 +23,7 @@ typedef struct MeshMoePlan {
   int* send_base;            // int32 [experts]
   int* layout;               // int32 [3 * experts/world + 2]
   void* tables[6];           // MeshTileDesc [max_tiles] each: glu, down, dh, dx, dw2, dw1
-  int* n_tiles;              // int32 [6]
+  int* n_tiles;              // int32 [8]: six table lengths, two counters (zero before the first call)
   int max_tiles;
   void* status;
 } MeshMoePlan;

@@ -84,7 +84,7 @@ class EPMoE:
         self.send_base = torch.zeros(experts, **i32)
         self.layout = torch.zeros(3 * self.El + 2, **i32)
         self.tables = [torch.zeros((self.max_tiles, 8), **i32) for _ in range(6)]
-        self.n_tiles = torch.zeros(6, **i32)
+        self.n_tiles = torch.zeros(8, **i32)             # six table lengths and two counters of the planning kernel
         self.h = torch.empty((self.cap, d_ff), dtype=torch.bfloat16, device=dev)
         self.gu = torch.empty((self.cap, 2 * d_ff), dtype=torch.bfloat16, device=dev)
         self.dgu = torch.empty((self.cap, 2 * d_ff), dtype=torch.bfloat16, device=dev)

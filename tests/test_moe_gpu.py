@@ -105,3 +105,41 @@ def test_moe_unused_experts_and_many_choices(T, D, F, E, k, spread):
     else:                                             # one renormalised weight is the constant 1
         assert float(dwr.abs().max()) < 1e-4
     ctx.heap.close()
+
+
+def test_plan_whose_counts_never_come():
+    """Every CTA of the planning kernel gives up on the counts of a step that nobody counted: the tables are empty, the status
+    says why, and the layer works again afterwards."""
+    import ctypes
+    import torch.distributed as dist
+    from mesh_b200 import _native
+    from mesh_b200.config import MeshConfig, set_config
+    from mesh_b200.distributed.context import MeshContext
+    from mesh_b200.parallel import moe as moe_module
+    from mesh_b200.runtime.rendezvous import Rendezvous
+    from mesh_b200.utils.status import MeshDeviceError, check_status, status_block
+    dev = torch.device("cuda", 0)
+    set_config(MeshConfig.from_env(heap_bytes=256 << 20))
+    ctx = MeshContext(0, 1, dev, Rendezvous(dist.HashStore(), 0, 1), None)
+    T, D, F, E, k = 128, 256, 128, 16, 2
+    g = torch.Generator(device=dev).manual_seed(1)
+    rand = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=dev) * std).bfloat16()
+    x, wr, w1, w2 = rand(T, D), rand(E, D, std=0.1), rand(E * 2 * F, D, std=0.05), rand(E * D, F, std=0.05)
+    moe = moe_module.EPMoE(ctx, T, D, F, E, k)
+    want = moe.forward(x, wr, w1, w2).clone()
+    lengths = moe.n_tiles.tolist()
+    assert all(n > 0 for n in lengths[:6]) and lengths[6:] == [0, 0]
+    p = moe_module._Plan()
+    p.counts, p.seq, p.rank, p.world, p.experts = moe.counts.ptr(), moe.steps + 1, 0, 1, E
+    p.cap_rows, p.d_model, p.d_ff = moe.cap, D, F
+    p.send_base, p.layout = moe.send_base.data_ptr(), moe.layout.data_ptr()
+    for i in range(6):
+        p.tables[i] = moe.tables[i].data_ptr()
+    p.n_tiles, p.max_tiles, p.status = moe.n_tiles.data_ptr(), moe.max_tiles, status_block(dev).data_ptr()
+    _native.check(moe.L.mesh_moe_plan(ctypes.byref(p), moe_module._s()), "mesh_moe_plan")
+    assert moe.n_tiles.tolist() == [0] * 8
+    with pytest.raises(MeshDeviceError):
+        check_status()
+    assert torch.equal(moe.forward(x, wr, w1, w2), want) and moe.n_tiles.tolist() == lengths
+    check_status()
+    ctx.heap.close()
