@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(const PlanArgs a) {
         else if (t == 1) d = MeshTileDesc{row, 0, F / 64, el * D + nt * 256, 0, row, nt * 256, 0};           // y = h W2^T
         else if (t == 2) d = MeshTileDesc{row, 0, D / 64, nt * 256, el * D, row, nt * 256, 0};               // dH = dY W2   (W2 stacked [El*D, F], MN-major)
         else if (t == 3) d = MeshTileDesc{row, 0, (2 * F) / 64, nt * 256, el * 2 * F, row, nt * 256, 0};     // dX = dGU W1  (W1 stacked [El*2F, D], MN-major)
-        else if (t == 4) d = MeshTileDesc{mt * 256, base, kb, nt * 256, 0, el * D + mt * 256, nt * 256, 0};  // dW2[el] = dY^T h   [D, F]
-        else d = MeshTileDesc{mt * 256, base, kb, nt * 256, 0, el * 2 * F + mt * 256, nt * 256, 0};          // dW1[el] = dGU^T x  [2F, D]
+        else if (t == 4) d = MeshTileDesc{mt * 256, base, kb, nt * 256, 0, el * D + mt * 256, nt * 256, D - mt * 256};  // dW2[el] = dY^T h   [D, F]
+        else d = MeshTileDesc{mt * 256, base, kb, nt * 256, 0, el * 2 * F + mt * 256, nt * 256, 2 * F - mt * 256};          // dW1[el] = dGU^T x  [2F, D]
         tab[t][at] = d;
       }
     }

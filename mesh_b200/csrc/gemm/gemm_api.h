@@ -11,8 +11,9 @@ extern "C" {
 // All leading dimensions are in elements (bf16).  Pointers are device pointers; peer
 // pointers (ag_dst, ag_flags, rs_recv, rs_count) come from the symmetric heap.
 // One tile of a descriptor-driven GEMM (same layout as mesh::gemm::TileDesc).  In pair mode a descriptor
-// covers 256 output rows: the second CTA of the pair adds 128 to a_mn0 and d_row0.
-typedef struct MeshTileDesc { int a_mn0, k0, k_blocks, b_mn0, b_k0, d_row0, d_col0, pad; } MeshTileDesc;
+// covers 256 output rows: the second CTA of the pair adds 128 to a_mn0 and d_row0.  d_rows: rows of D from d_row0 on that the
+// tile may write (a multiple of 32; 0: all), for stacked matrices whose heights are not multiples of a tile.
+typedef struct MeshTileDesc { int a_mn0, k0, k_blocks, b_mn0, b_k0, d_row0, d_col0, d_rows; } MeshTileDesc;
 
 typedef struct MeshGemmArgs {
   const void* A;

@@ -71,7 +71,7 @@ struct TileDesc {
   int b_k0;       // extra K offset of B (MN-major stacked weights: expert * rows)
   int d_row0;     // first output row
   int d_col0;     // first output column
-  int pad;
+  int d_rows;     // rows of D from d_row0 on that the tile may write, a multiple of 32 (0: all)
 };
 
 struct Params {
@@ -239,7 +239,7 @@ __device__ __forceinline__ TileCoord tile_coord(int tile, int m_tiles, int n_til
 // its own 128 rows of A and its own half of the B tile (plain TMA loads, no multicast); the
 // leader CTA issues the MMAs for both, so every SM pulls a third less from L2 per FLOP.
 struct Work {
-  int m0, ka0, kb0, k_blocks, bn0, d_row0, d_col0;
+  int m0, ka0, kb0, k_blocks, bn0, d_row0, d_col0, d_rows;
 };
 // Resolve tile number `tile` for the CTA with rank `cta_rank` in its pair.
 __device__ __forceinline__ Work get_work(const Params& p, int tile, int cta_rank, int ctas, int tile_n) {
@@ -253,6 +253,7 @@ __device__ __forceinline__ Work get_work(const Params& p, int tile, int cta_rank
     w.bn0 = d.b_mn0;
     w.d_row0 = d.d_row0 + cta_rank * BM;
     w.d_col0 = d.d_col0;
+    w.d_rows = d.d_rows ? d.d_rows - cta_rank * BM : BM;
   } else {
     TileCoord tc = tile_coord(tile, p.m_units, p.n_tiles, p.m_rotate);
     w.m0 = (tc.m_idx * ctas + cta_rank) * BM;
@@ -261,6 +262,7 @@ __device__ __forceinline__ Work get_work(const Params& p, int tile, int cta_rank
     w.bn0 = tc.n_idx * tile_n;
     w.d_row0 = w.m0;
     w.d_col0 = w.bn0;
+    w.d_rows = BM;
   }
   return w;
 }
@@ -543,7 +545,7 @@ gemm_kernel(const __grid_constant__ Params p) {
         const int n0 = wk.d_col0;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
-          if (n0 + c * 32 >= p.N) break;
+          if (n0 + c * 32 >= p.N || q * 32 >= wk.d_rows) break;
           uint32_t r[32];
           tmem_ld_32x32(taddr + c * 32, r);
           tmem_ld_wait();

@@ -143,3 +143,38 @@ def test_plan_whose_counts_never_come():
     assert torch.equal(moe.forward(x, wr, w1, w2), want) and moe.n_tiles.tolist() == lengths
     check_status()
     ctx.heap.close()
+
+
+@pytest.mark.parametrize("F,E", [(64, 16), (192, 16), (320, 8)])
+def test_moe_experts_of_any_height(F, E):
+    """2 F is not a multiple of a 256-row tile: the last tile of an expert's gate and up gradient ends inside it, and stays out
+    of the next expert's rows, whatever order the tiles finish in."""
+    import torch.distributed as dist
+    from mesh_b200.config import MeshConfig, set_config
+    from mesh_b200.distributed.context import MeshContext
+    from mesh_b200.parallel.moe import EPMoE, moe_reference
+    from mesh_b200.runtime.rendezvous import Rendezvous
+    from mesh_b200.utils.status import check_status
+    dev = torch.device("cuda", 0)
+    T, D, k = 256, 512, 2
+    set_config(MeshConfig.from_env(heap_bytes=512 << 20))
+    ctx = MeshContext(0, 1, dev, Rendezvous(dist.HashStore(), 0, 1), None)
+    g = torch.Generator(device=dev).manual_seed(F)
+    rand = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=dev) * std).bfloat16()
+    x, dy, wr, w1, w2 = rand(T, D), rand(T, D), rand(E, D, std=0.1), rand(E, 2 * F, D, std=0.05), rand(E, D, F, std=0.05)
+    moe = EPMoE(ctx, T, D, F, E, k)
+    X, W1, W2, WR = (t.float().requires_grad_(True) for t in (x, w1, w2, wr))
+    want = moe_reference(X, WR, W1, W2, k)
+    grads = torch.autograd.grad((want * dy.float()).sum(), (X, W1, W2))
+    for _ in range(5):
+        out = moe.forward(x, wr, w1.view(-1, D), w2.view(-1, F))
+        dx, dwr, dw1, dw2 = moe.backward(dy)
+        check_status()
+        # expert by expert, and the first and last rows of each by themselves
+        for got, ref in ((dw1.view_as(w1), grads[1]), (dw2.view_as(w2), grads[2])):
+            for e in range(E):
+                for part in (slice(None), slice(0, 64), slice(-64, None)):
+                    _close(got[e, part], ref[e, part], 5e-2)
+        _close(dx, grads[0], 5e-2)
+        _close(out, want, 3e-2)
+    ctx.heap.close()
