@@ -250,7 +250,11 @@ extern "C" int mesh_rmsnorm_bwd_blocks(int rows) { return rows < 592 ? rows : 59
 
 static int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw, __nv_bfloat16* dw16,
                        float* dw_partial, int blocks, int rows, int cols, float w_offset, void* stream) {
-  if (rows <= 0) return 0;
+  if (rows <= 0) {                           // no kernel runs: the weight gradient of no rows is zero
+    if (dw && cols > 0) MESH_CUDA_OK(cudaMemsetAsync(dw, 0, (size_t)cols * 4, (cudaStream_t)stream));
+    if (dw16 && cols > 0) MESH_CUDA_OK(cudaMemsetAsync(dw16, 0, (size_t)cols * 2, (cudaStream_t)stream));
+    return 0;
+  }
   if (cols % 8 || cols > NORM_THREADS * MAX_VEC_PER_THREAD * 8)
     return set_error(-2, "rmsnorm: cols must be a multiple of 8 and <= %d", NORM_THREADS * MAX_VEC_PER_THREAD * 8);
   if (blocks <= 0 || blocks > 1024) return set_error(-2, "rmsnorm_bwd: blocks out of range");

@@ -153,7 +153,10 @@ int partials_for_current_device(float** out) {
 extern "C" int mesh_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
                                         float* dw, int rows, int cols, float w_offset, void* stream) {
   using namespace mesh;
-  if (rows <= 0) return 0;
+  if (rows <= 0) {                           // no kernel runs: the weight gradient of no rows is zero
+    if (dw && cols > 0) MESH_CUDA_OK(cudaMemsetAsync(dw, 0, (size_t)cols * 4, (cudaStream_t)stream));
+    return 0;
+  }
   if (cols <= 0 || cols % 8)
     return set_error(-2, "rmsnorm_bwd_noalloc: cols (%d) must be a positive multiple of 8", cols);
   if (cols > MESH_NOALLOC_MAX_COLS)

@@ -177,3 +177,24 @@ def test_cross_entropy_keeps_a_nan(v, at, rest):
     t = torch.full((3,), (at + 1) % v, device="cuda")
     loss = vocab_parallel_cross_entropy(buf, t, 0, None, reduction="none")
     assert torch.isnan(loss).tolist() == [False, True, False]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rmsnorm_backward_of_no_rows(dtype):
+    """The weight gradient of an empty batch is zero, in memory that held something else."""
+    from mesh_b200.ops.norm import rmsnorm_bwd
+    cols = 2048
+    x, w = torch.empty(0, cols, device="cuda", dtype=torch.bfloat16), torch.ones(cols, device="cuda", dtype=torch.bfloat16)
+    rstd = torch.empty(0, device="cuda")
+    for _ in range(4):
+        junk = [torch.full((cols,), float("nan"), dtype=dtype, device="cuda") for _ in range(8)]
+        del junk
+        dx, dw = rmsnorm_bwd(x, x, w, rstd, 0.0, dtype)
+        assert dx.shape == x.shape and dw.dtype == dtype and float(dw.abs().sum()) == 0
+    from ctypes import c_float, c_int, c_void_p
+    from mesh_b200 import _native
+    dw = torch.full((cols,), float("nan"), device="cuda")
+    p = lambda t: c_void_p(t.data_ptr())
+    assert _native.lib().mesh_rmsnorm_bwd_noalloc(p(x), p(x), p(w), p(rstd), p(x), p(dw), c_int(0), c_int(cols), c_float(0.0),
+                                                  c_void_p(_native.stream())) == 0
+    assert float(dw.abs().sum()) == 0
