@@ -29,7 +29,7 @@ namespace fa {
 constexpr int SM_THREADS = 256;       // 8 softmax warps
 
 struct Params {
-  CUtensorMap tmQ, tmK, tmV;          // 2-D maps over [rows, cols] views; boxes {64, 128} / {64, BKV}
+  CUtensorMap tmQ, tmK, tmV;          // [sample][row][column], boxes of 64 columns and 128 rows
   __nv_bfloat16* out; long long ldo;  // [B*Tq, H*hd]
   float* lse;                         // [B, H, Tq]
   int B, H, Hkv, Tq, Tk;
@@ -169,26 +169,24 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
   if (warp == 8) {
     if (lane == 0 && j_hi > j_lo) {
       // ------------------------------------------------------------------ copies
-      const int q_row = b * p.Tq + q0;
       const int tiles = any1 ? 2 : 1;                  // the second tile may lie past the last query
       mbar_expect_tx(bar(Q_FULL), tiles * C::TILE);
       for (int t = 0; t < tiles; ++t)
         for (int kc = 0; kc < KC; ++kc)
-          tma_load_2d(sQ + t * C::TILE + kc * (TT * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, q_row + t * TT);
+          tma_load_3d(sQ + t * C::TILE + kc * (TT * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, q0 + t * TT, b);
       bool ok = true;
       for (int j = j_lo, n = 0; ok && j < j_hi; ++j, ++n) {
         const int s = n & 1;
-        const int k_row = b * p.Tk + j * TT;
         if (n >= 2) ok = mbar_wait(bar(K_EMPTY + s), ((n >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
         if (!ok) break;
         mbar_expect_tx(bar(K_FULL + s), C::TILE);
         for (int kc = 0; kc < KC; ++kc)
-          tma_load_2d(sK + s * C::TILE + kc * (TT * 128), &p.tmK, bar(K_FULL + s), p.k_col0 + hk * HD + kc * 64, k_row);
+          tma_load_3d(sK + s * C::TILE + kc * (TT * 128), &p.tmK, bar(K_FULL + s), p.k_col0 + hk * HD + kc * 64, j * TT, b);
         if (n >= 2) ok = mbar_wait(bar(V_EMPTY + s), ((n >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
         if (!ok) break;
         mbar_expect_tx(bar(V_FULL + s), C::TILE);
         for (int kc = 0; kc < KC; ++kc)
-          tma_load_2d(sV + s * C::TILE + kc * (TT * 128), &p.tmV, bar(V_FULL + s), p.v_col0 + hk * HD + kc * 64, k_row);
+          tma_load_3d(sV + s * C::TILE + kc * (TT * 128), &p.tmV, bar(V_FULL + s), p.v_col0 + hk * HD + kc * 64, j * TT, b);
       }
     }
   } else if (warp == 9) {
@@ -488,9 +486,8 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd256_kernel(const __grid_
   if (warp == 8) {
     if (lane == 0 && n_blocks > 0) {
       // ------------------------------------------------------------------ copies
-      const int q_row = b * p.Tq + q0;
       mbar_expect_tx(bar(Q_FULL), C::Q_BYTES);
-      for (int kc = 0; kc < 4; ++kc) tma_load_2d(sQ + kc * (TT * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, q_row);
+      for (int kc = 0; kc < 4; ++kc) tma_load_3d(sQ + kc * (TT * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, q0, b);
       bool ok = true;
       int slot = 0, n = 0;
       auto load = [&](const void* map, int col0, int j) {              // a tile as two halves of 128 columns
@@ -499,7 +496,7 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd256_kernel(const __grid_
           if (!ok) return;
           mbar_expect_tx(bar(FULL + slot), C::SLOT);
           for (int kc = 0; kc < 2; ++kc)
-            tma_load_2d(ring + slot * C::SLOT + kc * (TT * 128), map, bar(FULL + slot), col0 + c * 128 + kc * 64, b * p.Tk + (j0 + j) * TT);
+            tma_load_3d(ring + slot * C::SLOT + kc * (TT * 128), map, bar(FULL + slot), col0 + c * 128 + kc * 64, (j0 + j) * TT, b);
           if (++slot == C::SLOTS) slot = 0;
         }
       };
@@ -740,21 +737,23 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd256_kernel(const __grid_
   }
 }
 
-static bool map2d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_rows) {
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t es[2] = {1, 1};
-  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+// [sample][row][column]: what a tile reads past the last row of its sample is zero, not the next sample's.  (Hidden keys have
+// P = 0, but 0 * NaN is NaN: a sample with NaN or infinities would reach the one before it.)
+static bool map3d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t samples, uint64_t ld) {
+  cuuint64_t dims[3] = {cols, rows, samples};
+  cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
+  cuuint32_t box[3] = {64, TT, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int HD>
 static int launch(const MeshFlashArgs* a, cudaStream_t stream) {
   Params p;
   memset(&p, 0, sizeof(p));
-  if (!map2d(&p.tmQ, a->q, (uint64_t)a->q_cols, (uint64_t)a->B * a->Tq, (uint64_t)a->ldq, TT)) return last_error_code();
-  if (!map2d(&p.tmK, a->k, (uint64_t)a->k_cols, (uint64_t)a->B * a->Tk, (uint64_t)a->ldk, TT)) return last_error_code();
-  if (!map2d(&p.tmV, a->v, (uint64_t)a->v_cols, (uint64_t)a->B * a->Tk, (uint64_t)a->ldv, TT)) return last_error_code();
+  if (!map3d(&p.tmQ, a->q, (uint64_t)a->q_cols, (uint64_t)a->Tq, (uint64_t)a->B, (uint64_t)a->ldq)) return last_error_code();
+  if (!map3d(&p.tmK, a->k, (uint64_t)a->k_cols, (uint64_t)a->Tk, (uint64_t)a->B, (uint64_t)a->ldk)) return last_error_code();
+  if (!map3d(&p.tmV, a->v, (uint64_t)a->v_cols, (uint64_t)a->Tk, (uint64_t)a->B, (uint64_t)a->ldv)) return last_error_code();
   p.out = (__nv_bfloat16*)a->out; p.ldo = a->ldo; p.lse = a->lse;
   p.B = a->B; p.H = a->H; p.Hkv = a->Hkv; p.Tq = a->Tq; p.Tk = a->Tk;
   p.q_col0 = a->q_col0; p.k_col0 = a->k_col0; p.v_col0 = a->v_col0;

@@ -30,7 +30,7 @@ constexpr int SM_THREADS = 256;       // 8 softmax warps: threads r and r + 128 
 constexpr int THREADS = 288;          // + 1 copy/MMA warp
 
 struct Params {
-  CUtensorMap tmQ, tmK, tmV, tmdO;           // boxes {64, 128}
+  CUtensorMap tmQ, tmK, tmV, tmdO;           // [sample][row][column], boxes of 64 columns and 128 rows
   CUtensorMap tmdQ;                          // fp32 [B][Tq][H*hd], box {32, 32, 1}
   const float* lse; const float* delta;      // [B, H, Tq]
   float* dq;                                 // fp32 [B*Tq, H*hd], zeroed by the caller
@@ -180,11 +180,10 @@ __global__ void __launch_bounds__(THREADS, 1) flash_bwd_kernel(const __grid_cons
 
   if (warp == 8) {
     if (lane == 0 && n_iter > 0) {
-      const int k_row = b * p.Tk + k0;
       mbar_expect_tx(bar(KV_FULL), 2 * TILE);
       for (int kc = 0; kc < KC; ++kc) {
-        tma_load_2d(sK + kc * (128 * 128), &p.tmK, bar(KV_FULL), p.k_col0 + hk * HD + kc * 64, k_row);
-        tma_load_2d(sV + kc * (128 * 128), &p.tmV, bar(KV_FULL), p.v_col0 + hk * HD + kc * 64, k_row);
+        tma_load_3d(sK + kc * (128 * 128), &p.tmK, bar(KV_FULL), p.k_col0 + hk * HD + kc * 64, k0, b);
+        tma_load_3d(sV + kc * (128 * 128), &p.tmV, bar(KV_FULL), p.v_col0 + hk * HD + kc * 64, k0, b);
       }
       constexpr uint32_t id_s = umma_idesc_bf16(128, 128, 0, 0);        // Q K^T and dO V^T: both K-major over head_dim
       constexpr uint32_t id_t = umma_idesc_bf16(128, HD, 1, 1);         // P^T dO and dS^T Q: A and B MN-major, K = queries
@@ -198,11 +197,10 @@ __global__ void __launch_bounds__(THREADS, 1) flash_bwd_kernel(const __grid_cons
           ok = mbar_wait(bar(MMA2_DONE), (it - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
           if (!ok) break;
         }
-        const int q_row = b * p.Tq + i * BQ;
         mbar_expect_tx(bar(Q_FULL), 2 * TILE);
         for (int kc = 0; kc < KC; ++kc) {
-          tma_load_2d(sQ + kc * (128 * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, q_row);
-          tma_load_2d(sdO + kc * (128 * 128), &p.tmdO, bar(Q_FULL), p.do_col0 + h * HD + kc * 64, q_row);
+          tma_load_3d(sQ + kc * (128 * 128), &p.tmQ, bar(Q_FULL), p.q_col0 + h * HD + kc * 64, i * BQ, b);
+          tma_load_3d(sdO + kc * (128 * 128), &p.tmdO, bar(Q_FULL), p.do_col0 + h * HD + kc * 64, i * BQ, b);
         }
         ok = mbar_wait(bar(Q_FULL), it & 1, abort_smem, p.status, SITE_SMEM_FULL);
         if (!ok) break;
@@ -456,11 +454,10 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_bwd2_kernel(const __grid_co
     // -------------------------------------------------------------------- copies
     if (n_iter > 0) {
       if (lane == 0) {
-        const int k_row = b * p.Tk + k0;
         mbar_expect_tx(bar(B_::KV_FULL), 2 * TILE);
         for (int kc = 0; kc < KC; ++kc) {
-          tma_load_2d(sK + kc * (128 * 128), &p.tmK, bar(B_::KV_FULL), p.k_col0 + hk * HD + kc * 64, k_row);
-          tma_load_2d(sV + kc * (128 * 128), &p.tmV, bar(B_::KV_FULL), p.v_col0 + hk * HD + kc * 64, k_row);
+          tma_load_3d(sK + kc * (128 * 128), &p.tmK, bar(B_::KV_FULL), p.k_col0 + hk * HD + kc * 64, k0, b);
+          tma_load_3d(sV + kc * (128 * 128), &p.tmV, bar(B_::KV_FULL), p.v_col0 + hk * HD + kc * 64, k0, b);
         }
       }
       bool ok = true;
@@ -468,14 +465,13 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_bwd2_kernel(const __grid_co
         const int s = it & 1;
         const int g = it / n_q, i = i_lo + it % n_q;
         const int h = hk * group + g;
-        const int q_row = b * p.Tq + i * BQ;
         if (it >= 2) ok = mbar_wait(bar(B_::Q_EMPTY + s), ((it >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (lane == 0) {
           mbar_expect_tx(bar(B_::Q_FULL + s), TILE);
           for (int kc = 0; kc < KC; ++kc)
-            tma_load_2d(sQ + s * TILE + kc * (128 * 128), &p.tmQ, bar(B_::Q_FULL + s), p.q_col0 + h * HD + kc * 64, q_row);
+            tma_load_3d(sQ + s * TILE + kc * (128 * 128), &p.tmQ, bar(B_::Q_FULL + s), p.q_col0 + h * HD + kc * 64, i * BQ, b);
         }
         if (it >= 1) ok = mbar_wait(bar(B_::DO_EMPTY), (it - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
         ok = __all_sync(0xffffffffu, ok);
@@ -483,7 +479,7 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_bwd2_kernel(const __grid_co
         if (lane == 0) {
           mbar_expect_tx(bar(B_::DO_FULL), TILE);
           for (int kc = 0; kc < KC; ++kc)
-            tma_load_2d(sdO + kc * (128 * 128), &p.tmdO, bar(B_::DO_FULL), p.do_col0 + h * HD + kc * 64, q_row);
+            tma_load_3d(sdO + kc * (128 * 128), &p.tmdO, bar(B_::DO_FULL), p.do_col0 + h * HD + kc * 64, i * BQ, b);
         }
         // rows with no visible key at all (L = -inf) and rows past the end get P = 0 through an infinite offset
         const long long row0 = ((long long)b * p.H + h) * p.Tq + i * BQ;
@@ -763,12 +759,13 @@ __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restr
   }
 }
 
-static bool map2d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t ld) {
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {64, 128};
-  cuuint32_t es[2] = {1, 1};
-  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+// [sample][row][column]: what a tile reads past the last row of its sample is zero, not the next sample's
+static bool map3d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t samples, uint64_t ld) {
+  cuuint64_t dims[3] = {cols, rows, samples};
+  cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
+  cuuint32_t box[3] = {64, 128, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 static bool map_dq(CUtensorMap* tm, const float* dq, const MeshFlashArgs& f, long long ld, int hd) {
@@ -785,10 +782,10 @@ static int launch(const MeshFlashBwdArgs* a, cudaStream_t stream) {
   Params p;
   memset(&p, 0, sizeof(p));
   const MeshFlashArgs& f = a->fwd;
-  if (!map2d(&p.tmQ, f.q, (uint64_t)f.q_cols, (uint64_t)f.B * f.Tq, (uint64_t)f.ldq)) return last_error_code();
-  if (!map2d(&p.tmK, f.k, (uint64_t)f.k_cols, (uint64_t)f.B * f.Tk, (uint64_t)f.ldk)) return last_error_code();
-  if (!map2d(&p.tmV, f.v, (uint64_t)f.v_cols, (uint64_t)f.B * f.Tk, (uint64_t)f.ldv)) return last_error_code();
-  if (!map2d(&p.tmdO, a->dout, (uint64_t)a->do_cols, (uint64_t)f.B * f.Tq, (uint64_t)a->ld_do)) return last_error_code();
+  if (!map3d(&p.tmQ, f.q, (uint64_t)f.q_cols, (uint64_t)f.Tq, (uint64_t)f.B, (uint64_t)f.ldq)) return last_error_code();
+  if (!map3d(&p.tmK, f.k, (uint64_t)f.k_cols, (uint64_t)f.Tk, (uint64_t)f.B, (uint64_t)f.ldk)) return last_error_code();
+  if (!map3d(&p.tmV, f.v, (uint64_t)f.v_cols, (uint64_t)f.Tk, (uint64_t)f.B, (uint64_t)f.ldv)) return last_error_code();
+  if (!map3d(&p.tmdO, a->dout, (uint64_t)a->do_cols, (uint64_t)f.Tq, (uint64_t)f.B, (uint64_t)a->ld_do)) return last_error_code();
   if (!map_dq(&p.tmdQ, a->dq, f, a->ld_dq, HD)) return last_error_code();
   p.lse = f.lse; p.delta = a->delta; p.dq = a->dq; p.dk = (__nv_bfloat16*)a->dk; p.dv = (__nv_bfloat16*)a->dv;
   p.dk_acc = a->dk_acc; p.dv_acc = a->dv_acc;

@@ -347,3 +347,33 @@ def test_delta_of_any_number_of_rows(hd, B, T, H):
     # fp32 sums of hd products of order one
     assert float((got.double() - want).abs().max()) < hd * 2 ** -20
     assert float(clear.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("T", [40, 100, 200, 256])
+@pytest.mark.parametrize("p", [0.0, 0.1])
+def test_a_sample_does_not_reach_the_one_before_it(hd, T, p):
+    """The last tile of a sample ends in rows of the next one.  A sample of NaN or infinities changes nothing in the others."""
+    from mesh_b200.ops.attention import flash_attention, flash_attention_backward
+    from mesh_b200.utils.status import check_status
+    g = torch.Generator(device="cuda").manual_seed(T)
+    clean = dict(zip("qkvd", (torch.randn(3, T, 2, hd, device="cuda", generator=g).bfloat16() for _ in range(4))))
+    kw = dict(causal=False, dropout=dict(p=p, seed=5) if p else None)
+
+    def run(t):
+        out, lse = flash_attention(t["q"], t["k"], t["v"], need_lse=True, **kw)
+        grads = flash_attention_backward(t["q"], t["k"], t["v"], *fixed, t["d"], **kw) if hd < 256 else ()
+        return out, lse, *grads
+
+    fixed = flash_attention(clean["q"], clean["k"], clean["v"], need_lse=True, **kw)
+    want = run(clean)
+    for name in "qkvd":
+        for value in (float("nan"), float("inf")):
+            bad = dict(clean, **{name: clean[name].clone()})
+            bad[name][1] = value
+            for got, ref in zip(run(bad), want):
+                for b in (0, 2):
+                    assert bool(torch.isfinite(got[b]).all()), (name, value, b)
+                    # the same products; only the order in which blocks of dq are added may differ
+                    torch.testing.assert_close(got[b], ref[b], atol=1e-4, rtol=1e-4)
+    check_status()
