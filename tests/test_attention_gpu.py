@@ -253,9 +253,11 @@ def test_flash_backward_with_dropout(hd, H, Hkv):
     (1, 300, 512, 2, 2, True, 0, (0, 150), 1),       # queries that see no key
 ])
 def test_flash_tiles(hd, B, Tq, Tk, H, Hkv, causal, window, off, stride):
-    """Both directions at the edges of the query tiles and key blocks.  Probabilities, score gradients and results are
-    rounded to bf16 (2^-9 each): three of them in quadrature stay below 4e-3; twice that is allowed."""
-    from mesh_b200.ops.attention import attention_ref, flash_attention, flash_attention_backward
+    """Both directions at the edges of the query tiles and key blocks, every row by itself.  A row's probabilities, score
+    gradients and results are rounded to bf16, 2^-9 of their size at most each: three of them stay below 8e-3 of the row.
+    Delta is formed from the rounded output; dP - Delta cancels where few keys are seen, so the rounding that is left of it,
+    three standard deviations of sum(dO o O), is allowed on the rows of dq and dk that it reaches."""
+    from mesh_b200.ops.attention import flash_attention, flash_attention_backward
     from mesh_b200.utils.status import check_status
     g = torch.Generator(device="cuda").manual_seed(3)
     q, do = (torch.randn(B, Tq, H, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
@@ -277,10 +279,15 @@ def test_flash_tiles(hd, B, Tq, Tk, H, Hkv, causal, window, off, stride):
     pr = torch.softmax(s.masked_fill(blind[:, None], 0.0), -1).masked_fill(blind[:, None], 0.0)
     ref = torch.einsum("bhts,bshd->bthd", pr, vf.repeat_interleave(H // Hkv, 2))
     grads = torch.autograd.grad(ref, (qf, kf, vf), do.double())
-    for got, want in zip((out, dq, dk, dv), (ref, *grads)):
-        err = float((got.double() - want).detach().norm())
-        # where the exact value vanishes (one visible key per query) what is left is the rounding of dP - Delta
-        assert err <= 8e-3 * max(float(want.detach().norm()), float(do.double().norm()) * 0.5), (err, float(want.detach().norm()))
+    with torch.no_grad():
+        left = 3 * 2 ** -9 * hd ** -0.5 * (do.double() * ref).square().sum(-1).sqrt()                    # [B, Tq, H]
+        left_q = left * torch.einsum("bhts,bshd->bthd", pr, kf.repeat_interleave(H // Hkv, 2)).norm(dim=-1)
+        left_k = torch.einsum("bhts,bth->bsh", pr.square(), (left * qf.norm(dim=-1)).square())
+        left_k = left_k.view(B, Tk, Hkv, H // Hkv).sum(-1).sqrt()
+        for name, got, want, extra in (("out", out, ref, 0.0), ("dq", dq, grads[0], left_q), ("dk", dk, grads[1], left_k), ("dv", dv, grads[2], 0.0)):
+            err, limit = (got.double() - want).norm(dim=-1), 8e-3 * want.norm(dim=-1) + extra + 1e-6
+            worst = int((err / limit).argmax())
+            assert bool((err <= limit).all()), (name, worst, float(err.view(-1)[worst]), float(limit.view(-1)[worst]))
     seen = ~blind
     torch.testing.assert_close(lse[:, :, seen].double(), torch.logsumexp(s, -1)[:, :, seen].detach(), atol=1e-4, rtol=1e-4)
     assert bool(torch.isinf(lse[:, :, blind]).all())
