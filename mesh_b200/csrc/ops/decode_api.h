@@ -13,7 +13,9 @@ enum MeshDecodeMode { MESH_DEC_STORE = 0, MESH_DEC_GLU = 1, MESH_DEC_QKV = 2, ME
 typedef struct MeshDecodeLinear {
   const void* x; long long ldx; int B, K, N;      // x [B, K] bf16; N = output rows handled (GLU: gate rows)
   const void* norm_w; float eps, norm_off;         // optional RMSNorm prologue
-  const void* w; const void* scales; int w4;       // bf16 [rows, K] or 4-bit codes [rows, K/2] + fp16 scales [rows, K/64]
+  // bf16 [rows, K] (w4 0), 4-bit codes [rows, K/2] (1) or 8-bit codes [rows, K] (8) with fp16 scales [rows, K/64].  Read before
+  // the kernel waits for the one before it in the stream: neither may be what that kernel writes.
+  const void* w; const void* scales; int w4;
   int mode, act, up_off;
   void* out; long long ldo; int out_f32;
   int q_heads, kv_heads, head_dim;

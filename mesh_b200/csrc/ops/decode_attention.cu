@@ -157,8 +157,11 @@ extern "C" int mesh_decode_attention(const void* q, const void* k_cache, const v
   A.q_heads = q_heads; A.kv_heads = kv_heads; A.max_seq = max_seq; A.window = window; A.scale = scale; A.splits = splits;
   A.T = tokens_per_seq; A.B = B; A.head_dim = head_dim;
   A.unaligned = unaligned(q, k_cache, v_cache, head_dim);
-  // A cluster takes what 64 warps scan in a few steps, or whatever is asked for in no more splits than it has CTAs; more
-  // splits of a longer context go to more CTAs than a cluster has.
+  // A cluster, or splits merged through memory.  The host knows the size of the cache and not the context, so the line lies where
+  // a full cache takes as long either way.  Back to back, 8 query heads of 256 over 2 KV heads, batch 1 / 8, a cluster of eight
+  // and 16 splits: at 4096 keys 18.5 / 29.0 and 19.1 / 26.2 us, at 8192 32.1 / 56.3 and 25.5 / 40.3, at 200 keys of a cache of
+  // 8192 5.1 / 6.6 and 11.4 / 12.4; 32 heads of 128 over 8, 4096 keys 15.1 / 47.5 and 19.0 / 54.4, 8192 25.5 / 85.0 and
+  // 26.6 / 80.3.  Whoever asks for no more splits than a cluster has CTAs gets the cluster.
   const int most = window > 0 && window < max_seq ? window : max_seq;
   const bool cluster = !A.unaligned && (splits <= MAX_CLUSTER || most <= 4096);
   const bool four = q_heads / kv_heads <= 4;

@@ -1,16 +1,17 @@
 // Skinny (batch <= 8) linear layers for token-by-token decoding: y[b, n] = sum_k x[b, k] W[n, k].
 //
-// Decoding is bound by the bytes of W, so the kernel is organised around streaming W once at full
-// HBM rate: a CTA owns 16 rows of W (two groups of 8), its 8 warps split K, each lane pulls 16-byte
-// pieces of two rows straight from global memory into mma.sync A fragments (the k order inside a
-// 32-wide block is permuted identically for W and x, which a dot product does not notice), the
-// batch is the 8-wide N side of m16n8k16, and partial sums meet in shared memory.  Around that
-// core sit the fusions that remove the launches between the layers of a decoder block:
+// Decoding is bound by the bytes of W, so the kernels are organised around reading W once at full HBM rate.  A CTA works on
+// groups of 16 rows of W (two groups of 8), its 8 warps split K, the batch is the 8-wide N side of mma.sync m16n8k16 (the k
+// order inside a block is permuted identically for W and x, which a dot product does not notice), and partial sums meet in
+// shared memory.  W reaches the warps in two ways: as tiles that a ninth warp copies into a ring of shared-memory stages
+// (decode_linear.cu, and across layers decode_step.cu: the rule), or as 16-byte pieces that each lane pulls straight from
+// global memory into fragments (`linear_body`: where no ring fits beside x, and for rows or scales that the copies do not
+// take).  Around that core sit the fusions that remove the launches between the layers of a decoder block:
 //   prologue   RMSNorm of x (recomputed by every CTA: duplicated cheap compute is free,
 //              design/collective-goals.md:27-29)
-//   weights    bf16, or 4-bit codes with one fp16 scale per 64 k (dequantised in registers with a
-//              mask, subtract and multiply per pair; reference: `mesh::fragment` coded weights,
-//              rdma/mesh_code.py:9-16, compiler/mesh_compiler/operations.py:6996-7040)
+//   weights    bf16, or 4- or 8-bit codes with one fp16 scale per 64 k: codes are exact bf16 integers in the products and the
+//              scale multiplies the fp32 sum of each 64 (the register reader's widest 4-bit form alone rounds weights;
+//              reference: `mesh::fragment` coded weights, rdma/mesh_code.py:9-16, compiler/mesh_compiler/operations.py:6996-7040)
 //   epilogue   store | GLU (gate and up rows in one CTA) | QKV + RoPE + KV-cache append |
 //              one-shot all-reduce across GPUs + residual add (row-parallel projections of a
 //              tensor-parallel block: 8-byte {value, sequence} words stored into every peer and

@@ -205,7 +205,7 @@ def dequantize_w4(codes: torch.Tensor, scales: torch.Tensor) -> torch.Tensor:
 
 def quantize_w8(w: torch.Tensor, group: int = 64):
     """``w [N, K]`` -> ``(codes uint8 [N, K], scales fp16 [N, K/group])``: ``w ~ (code - 128) * scale[row, k // 64]``,
-    codes in the natural order of k (the north star's 8-bit group-quantised variant)."""
+    codes in the natural order of k."""
     assert group == 64 and w.dim() == 2 and w.shape[1] % 64 == 0
     N, K = w.shape
     wf = w.float().view(N, K // group, group)
@@ -241,6 +241,10 @@ def decode_linear(x: torch.Tensor, w: torch.Tensor, *, scales: torch.Tensor | No
     outputs, adds ``residual``).  ``next_weights``: the weight matrix of the linear layer that follows in the step; this
     kernel asks for its first ``MESH_DECODE_PREFETCH_MB`` (default 8) megabytes to be brought into L2 while it streams its
     own, so that HBM does not sit idle across the kernel boundary.
+
+    Weights and scales are taken as constants of the model: the kernel starts to read them (a ring of stages, up to 200 KB
+    per SM) before it waits for the kernel before it in the stream, so they must not be what that kernel writes.  ``x``,
+    ``residual`` and the caches are waited for.
     """
     B, K = x.shape
     w4 = 0                                   # weight format: 0 bf16, 1 4-bit codes, 8 8-bit codes
