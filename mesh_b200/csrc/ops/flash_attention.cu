@@ -30,6 +30,7 @@ constexpr int SM_THREADS = 256;       // 8 softmax warps
 
 struct Params {
   CUtensorMap tmQ, tmK, tmV;          // [sample][row][column], boxes of 64 columns and 128 rows
+  CUtensorMap tmK2, tmV2;             // [row][column] over all samples: key blocks that end inside their sample
   __nv_bfloat16* out; long long ldo;  // [B*Tq, H*hd]
   float* lse;                         // [B, H, Tq]
   int B, H, Hkv, Tq, Tk;
@@ -177,16 +178,21 @@ __global__ void __launch_bounds__(THREADS2, 1) flash_fwd2_kernel(const __grid_co
       bool ok = true;
       for (int j = j_lo, n = 0; ok && j < j_hi; ++j, ++n) {
         const int s = n & 1;
+        // a copy with three coordinates takes longer: 2.5 % of the kernel with heads of 64 when every block used it
+        const bool whole = (j + 1) * TT <= p.Tk;
+        const int k_row = b * p.Tk + j * TT;
         if (n >= 2) ok = mbar_wait(bar(K_EMPTY + s), ((n >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
         if (!ok) break;
         mbar_expect_tx(bar(K_FULL + s), C::TILE);
         for (int kc = 0; kc < KC; ++kc)
-          tma_load_3d(sK + s * C::TILE + kc * (TT * 128), &p.tmK, bar(K_FULL + s), p.k_col0 + hk * HD + kc * 64, j * TT, b);
+          if (whole) tma_load_2d(sK + s * C::TILE + kc * (TT * 128), &p.tmK2, bar(K_FULL + s), p.k_col0 + hk * HD + kc * 64, k_row);
+          else tma_load_3d(sK + s * C::TILE + kc * (TT * 128), &p.tmK, bar(K_FULL + s), p.k_col0 + hk * HD + kc * 64, j * TT, b);
         if (n >= 2) ok = mbar_wait(bar(V_EMPTY + s), ((n >> 1) - 1) & 1, abort_smem, p.status, SITE_SMEM_EMPTY);
         if (!ok) break;
         mbar_expect_tx(bar(V_FULL + s), C::TILE);
         for (int kc = 0; kc < KC; ++kc)
-          tma_load_3d(sV + s * C::TILE + kc * (TT * 128), &p.tmV, bar(V_FULL + s), p.v_col0 + hk * HD + kc * 64, j * TT, b);
+          if (whole) tma_load_2d(sV + s * C::TILE + kc * (TT * 128), &p.tmV2, bar(V_FULL + s), p.v_col0 + hk * HD + kc * 64, k_row);
+          else tma_load_3d(sV + s * C::TILE + kc * (TT * 128), &p.tmV, bar(V_FULL + s), p.v_col0 + hk * HD + kc * 64, j * TT, b);
       }
     }
   } else if (warp == 9) {
@@ -747,6 +753,14 @@ static bool map3d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t row
   return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+static bool map2d(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint64_t ld) {
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * 2};
+  cuuint32_t box[2] = {64, TT};
+  cuuint32_t es[2] = {1, 1};
+  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
 template <int HD>
 static int launch(const MeshFlashArgs* a, cudaStream_t stream) {
   Params p;
@@ -754,6 +768,9 @@ static int launch(const MeshFlashArgs* a, cudaStream_t stream) {
   if (!map3d(&p.tmQ, a->q, (uint64_t)a->q_cols, (uint64_t)a->Tq, (uint64_t)a->B, (uint64_t)a->ldq)) return last_error_code();
   if (!map3d(&p.tmK, a->k, (uint64_t)a->k_cols, (uint64_t)a->Tk, (uint64_t)a->B, (uint64_t)a->ldk)) return last_error_code();
   if (!map3d(&p.tmV, a->v, (uint64_t)a->v_cols, (uint64_t)a->Tk, (uint64_t)a->B, (uint64_t)a->ldv)) return last_error_code();
+  if (HD <= 128 && !(map2d(&p.tmK2, a->k, (uint64_t)a->k_cols, (uint64_t)a->B * a->Tk, (uint64_t)a->ldk) &&
+                     map2d(&p.tmV2, a->v, (uint64_t)a->v_cols, (uint64_t)a->B * a->Tk, (uint64_t)a->ldv)))
+    return last_error_code();
   p.out = (__nv_bfloat16*)a->out; p.ldo = a->ldo; p.lse = a->lse;
   p.B = a->B; p.H = a->H; p.Hkv = a->Hkv; p.Tq = a->Tq; p.Tk = a->Tk;
   p.q_col0 = a->q_col0; p.k_col0 = a->k_col0; p.v_col0 = a->v_col0;
