@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
   visible(A, b, lo, hi);
   WarpState<HD, MAXG> st;
   // neighbouring keys to different CTAs, so that a short context uses all of them
-  scan_keys<HD, MAXG>(A, kvh, b, lo, hi, warp * ranks + rank, ATT_WARPS * ranks, false, st);
+  scan_keys<HD, MAXG, false>(A, kvh, b, lo, hi, warp * ranks + rank, ATT_WARPS * ranks, st);
   if (lane < 2 * MAXG && !(lane & 1)) {
     sm_m[warp][lane >> 1] = st.m;
     sm_l[warp][lane >> 1] = st.l;
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
       float a = 0.f, ll = 0.f;
 #pragma unroll
       for (int w = 0; w < ATT_WARPS; ++w) {
-        const float wgt = partial_weight(sm_m[w][g], sm_l[w][g], mm);
+        const float wgt = sm_m[w][g] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][g] - mm);
         a += wgt * sm_acc[(long long)w * MAXG * HD + e];
         ll += wgt * sm_l[w][g];
       }
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(ATT_THREADS, MAXG * HD <= 1024 ? 2 : 1) decode
     float a = 0.f, ll = 0.f;
 #pragma unroll
     for (int r = 0; r < MAX_CLUSTER; ++r) {
-      const float wgt = r < ranks ? partial_weight(m[r], l[r], mm) : 0.f;
+      const float wgt = m[r] == -CUDART_INF_F ? 0.f : __expf(m[r] - mm);
       if (wgt != 0.f) { a += wgt * v[r]; ll += wgt * l[r]; }
     }
     A.out[((long long)b * A.q_heads + kvh * group) * HD + e] = __float2bfloat16_rn(ll == 0.f ? 0.f : a / ll);
