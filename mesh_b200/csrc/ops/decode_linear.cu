@@ -71,15 +71,12 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
     // ---------------------------------------------------------------- weights
     if (lane != 0) return;
     int stage = 0, n = 0;
-    bool ok = true;
-    for (int grp = blockIdx.x; ok && grp < a.n_groups; grp += gridDim.x) {
+    for (int grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
       int rA, rB;
       group_rows(a, grp, rA, rB);
       for (int ks = 0; ks < kstages; ++ks, ++n) {
         const uint32_t full = full0 + 8 * stage;
-        if (n >= n_stages) ok = mbar_wait(empty0 + 8 * stage, ((n / n_stages) - 1) & 1, dead, a.status, SITE_SMEM_EMPTY);
-        ok = ok && !*dead;                     // after that the computing warps free stages whether or not they were filled
-        if (!ok) break;
+        if (n >= n_stages && !mbar_wait(empty0 + 8 * stage, ((n / n_stages) - 1) & 1, dead, a.status, SITE_SMEM_EMPTY)) goto drain;
         mbar_expect_tx(full, G::TX);
         const uint32_t slot = ring + (uint32_t)stage * G::SLOT;
         tma_load_3d(slot, &maps.w, full, 0, rA, ks * G::KC);
@@ -91,12 +88,12 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
         if (++stage == n_stages) stage = 0;
       }
     }
+  drain:
     // The CTA's shared memory has to stay until the last copies have landed in it, also when the computing warps gave up on
-    // them: nobody else waits then.
-    for (int i = max(0, n - n_stages); i < n; ++i) {
-      const unsigned long long t0 = globaltimer_ns();
+    // them: nobody else waits then.  (A flag in the loops instead of the jump made the chain of 4-bit layers 5 % slower.)
+    const unsigned long long t0 = globaltimer_ns();
+    for (int i = max(0, n - n_stages); i < n; ++i)
       while (!mbar_try_wait(full0 + 8 * (i % n_stages), (i / n_stages) & 1) && globaltimer_ns() - t0 < MESH_WAIT_LIMIT_NS) { __nanosleep(100); }
-    }
     return;
   }
   // ------------------------------------------------------------------ products
@@ -123,8 +120,8 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
   for (int grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x, turn ^= 1) {
     for (int ks = 0; ks < kstages; ++ks) {
       // after a wait has run out nobody waits any more (the status block says why the results are garbage), but every
-      // thread still meets every barrier
-      if (!*dead) mbar_wait(full0 + 8 * stage, phase, dead, a.status, SITE_SMEM_FULL);
+      // thread still meets every barrier; a stage whose copy was not seen to land is not given back
+      const bool landed = !*dead && mbar_wait(full0 + 8 * stage, phase, dead, a.status, SITE_SMEM_FULL);
       const uint8_t* slot = ring_p + (uint32_t)stage * G::SLOT;
       const uint8_t* ra = slot + chunk * 1024 + row * 128;
       const uint8_t* xp = xrow + (size_t)ks * G::KT * 2;
@@ -149,7 +146,7 @@ __global__ void __launch_bounds__(STREAM_THREADS) decode_stream_kernel(const Lin
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(empty0 + 8 * stage);
+      if (lane == 0 && landed) mbar_arrive(empty0 + 8 * stage);
       if (++stage == n_stages) { stage = 0; phase ^= 1u; }
     }
     finish_group(a, grp, c, row, red + turn * RED_FLOATS, ComputeBar{});
