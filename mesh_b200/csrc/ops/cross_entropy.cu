@@ -6,9 +6,9 @@
 // tiny all-reduces combine them, and the gradient (softmax - onehot) * g is formed from the logits again, so no fp32
 // copy of the logits or of their exponentials is ever stored.
 //
-// Bound by HBM: 8192 rows of 50304 logits (824 MB) are read in 160 us for the statistics (5.2 TB/s; 290 us before the
-// exponentials were batched) and read and written in 269 us for the gradient (6.1 TB/s).  Where the whole vocabulary is
-// here, losses, their mean and the gradient are these launches and one small one: 640 -> 434 us forward and backward,
+// Bound by HBM: 8192 rows of 50304 logits (824 MB) are read in 156 us for the statistics (5.3 TB/s; 290 us before the
+// exponentials were batched) and read and written in 273 us for the gradient (6.0 TB/s).  Where the whole vocabulary is
+// here, losses, their mean and the gradient are these launches and one small one: 641 -> 454 us a call forward and backward,
 // some twenty tensor operations on the rows among what went.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

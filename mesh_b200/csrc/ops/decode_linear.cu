@@ -12,8 +12,8 @@ namespace decode {
 // copies are tiles of a tensor map, eight rows by 128 bytes by eight chunks: the same stream as one bulk copy per row and
 // stage (1 KB) ran at half the rate.
 //
-// One period of five layers and the head, with the attention and selection kernels of this directory: bf16, batch 1
-// 497 -> 341 us; 4-bit, batch 8, head of 65536: 401 -> 249 us.  Alone (bf16, batch 1, back to back, before -> now; HBM
+// One decode call of five layers and the head, with the attention and selection kernels of this directory: bf16, batch 1,
+// head of 262144 498 -> 366 us; 4-bit, batch 8, head of 65536 419 -> 261 us.  Alone (bf16, batch 1, back to back, before -> now; HBM
 // at the measured copy rate): 2048 -> 3072 5.7 -> 4.7 us (1.9), gate and up 2048 -> 2 x 8192 17.0 -> 12.4 us (10.2),
 // 8192 -> 2048 11.9 -> 6.7 us (5.1), head 2048 -> 262144 193 -> 151 us (164).  4-bit, batch 8: 7.4 -> 5.4, 16.7 -> 10.3,
 // 9.2 -> 7.8, 135 -> 103 us: there a group of 16 rows is one stage, and its barrier and epilogue bound it.
@@ -198,7 +198,7 @@ static long long stages_read(const MeshDecodeLinear* d, const LinArgs& a) {
 }
 // Stages of the ring: all that fit beside x, at most what the CTA reads.  A ring of half an SM's shared memory, which would
 // let the next launch fill its own while this one runs, was slower over the whole step (bf16, batch 1, five layers and
-// the head: 376 us against 341 us; 4-bit, batch 8: 288 against 249).
+// the head, kernel time: 376 us against 341; 4-bit, batch 8: 288 against 249).
 template <int W4, int U>
 static int ring_stages(const MeshDecodeLinear* d, const LinArgs& a) {
   using G = StreamGeom<W4, U>;

@@ -82,7 +82,7 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b) {
 //
 // Bound by the exponentials: a 128 x 128 block takes 1024 cycles of the special-function units beside 1024 (head size
 // 128) or 512 (64) of the tensor pipe.  Measured at one sequence of 8192, 16 heads of 128, causal: 1014 us with one
-// tile per CTA and P in shared memory, 277 us with this one (990 TFLOP/s); heads of 64: 238 us.
+// tile per CTA and P in shared memory, 250 us with this one (1100 TFLOP/s); heads of 64: 201 us.
 constexpr int TT = 128;                               // rows of a tile
 constexpr int THREADS2 = 320;
 
